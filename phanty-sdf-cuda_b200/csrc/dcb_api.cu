@@ -74,7 +74,7 @@ struct dcb_context {
     int cells_per_vertex = 0;         // 1: the vertex -> cell list is `sp_vcell` (two vertices per cell)
     // mesh -> SDF workspace
     DevBuf m_verts, m_faces, m_out, m_tris, m_bin_count, m_bin_start, m_bin_fill, m_bin_scratch, m_bin_tris,
-        m_bin_active, m_active_list, m_axis_start, m_far, m_ext, m_tmp, m_partials, m_counters, m_vox;
+        m_items, m_axis_start, m_far, m_ext, m_tmp, m_partials, m_counters, m_vox;
     void* h_sdf_counters = nullptr;   // pinned SdfCounters
     void* h_counters = nullptr;       // pinned Counters
     void* hV = nullptr; size_t hV_bytes = 0;
@@ -954,7 +954,7 @@ struct SdfCounters {
     int changed;
     unsigned long long total_entries;
     unsigned long long exterior;
-    unsigned int active_bins;
+    unsigned int item_counts[2];
     unsigned int work_next;
 };
 
@@ -983,8 +983,6 @@ int run_mesh_sdf(dcb_context* h, const float* d_verts, int64_t nv, const int32_t
     DCB_TRY(h, ensure(h->m_bin_count, sizeof(uint32_t) * P.nbins), "alloc bins");
     DCB_TRY(h, ensure(h->m_bin_start, sizeof(uint32_t) * P.nbins), "alloc bins");
     DCB_TRY(h, ensure(h->m_bin_fill, sizeof(uint32_t) * P.nbins), "alloc bins");
-    DCB_TRY(h, ensure(h->m_bin_active, P.nbins), "alloc bins");
-    DCB_TRY(h, ensure(h->m_active_list, sizeof(uint32_t) * P.nbins), "alloc bins");
     DCB_TRY(h, ensure(h->m_axis_start, sizeof(int) * (P.gx + P.gy + P.gz + 3)), "alloc bins");
     DCB_TRY(h, ensure(h->m_partials, sizeof(uint32_t) * std::max(1LL, scan_partials_len(P.nbins))), "alloc scan");
     DCB_TRY(h, ensure(h->m_far, sizeof(uint32_t) * rows * P.W), "alloc masks");
@@ -996,10 +994,9 @@ int run_mesh_sdf(dcb_context* h, const float* d_verts, int64_t nv, const int32_t
     SdfCounters* hc = reinterpret_cast<SdfCounters*>(h->h_sdf_counters);
     P.tris = as<float>(h->m_tris);
     P.bin_count = as<uint32_t>(h->m_bin_count); P.bin_start = as<uint32_t>(h->m_bin_start);
-    P.bin_fill = as<uint32_t>(h->m_bin_fill); P.bin_active = as<uint8_t>(h->m_bin_active);
-    P.active_list = as<uint32_t>(h->m_active_list); P.axis_start = as<int>(h->m_axis_start);
+    P.bin_fill = as<uint32_t>(h->m_bin_fill); P.axis_start = as<int>(h->m_axis_start);
     P.far = as<uint32_t>(h->m_far); P.ext = as<uint32_t>(h->m_ext); P.err = &dc->err;
-    P.active_count = &dc->active_bins; P.work_next = &dc->work_next;
+    P.item_counts = dc->item_counts; P.work_next = &dc->work_next;
 
     cudaEvent_t* ev = h->ev;
     DCB_TRY(h, cudaEventRecord(ev[0], s), "event");
@@ -1016,7 +1013,10 @@ int run_mesh_sdf(dcb_context* h, const float* d_verts, int64_t nv, const int32_t
     if (entries >= 0xffffffffULL) return fail(h, DCB_ERR_TOO_LARGE, "more than 2^32-1 bin entries");
     DCB_TRY(h, ensure(h->m_bin_scratch, sizeof(uint32_t) * std::max(1ULL, entries)), "alloc bin entries");
     DCB_TRY(h, ensure(h->m_bin_tris, sizeof(uint32_t) * std::max(1ULL, entries)), "alloc bin entries");
+    P.items_cap = sdf_items_capacity(P.nbins, entries);
+    DCB_TRY(h, ensure(h->m_items, sizeof(uint2) * P.items_cap), "alloc bin items");
     P.bin_scratch = as<uint32_t>(h->m_bin_scratch); P.bin_tris = as<uint32_t>(h->m_bin_tris);
+    P.items = as<uint2>(h->m_items);
     DCB_TRY(h, launch_sdf_bins(P, h->num_sms, s), "launch binning");
     DCB_TRY(h, cudaEventRecord(ev[1], s), "event");
     DCB_TRY(h, launch_sdf_band(P, h->num_sms, s), "launch band");
@@ -1161,7 +1161,7 @@ int dcb_destroy(dcb_handle h) {
                       &h->stage_key, &h->faces, &h->wind_items, &h->v64_index, &h->v64_cells, &h->V64,
                       &h->tris, &h->tri_items, &h->m_verts, &h->m_faces, &h->m_out, &h->m_tris,
                       &h->m_bin_count, &h->m_bin_start, &h->m_bin_fill, &h->m_bin_scratch, &h->m_bin_tris,
-                      &h->m_bin_active, &h->m_active_list, &h->m_axis_start, &h->m_far, &h->m_ext, &h->m_tmp,
+                      &h->m_items, &h->m_axis_start, &h->m_far, &h->m_ext, &h->m_tmp,
                       &h->m_partials, &h->m_counters, &h->m_vox, &h->table, &h->cell_slot, &h->adj_rows, &h->adj_owners, &h->ours_ws, &h->wt,
                       &h->sp_words, &h->sp_brick, &h->sp_vcount, &h->sp_vstart, &h->sp_vtmp, &h->sp_ntmp,
                       &h->sp_N, &h->sp_vcell, &h->sp_fcount, &h->sp_fstart, &h->sp_stage, &h->sp_counters};

@@ -348,10 +348,10 @@ struct SdfParams {
     uint32_t* bin_fill;
     uint32_t* bin_scratch;         // bin entries as scattered
     uint32_t* bin_tris;            // bin entries in ascending triangle order
-    uint8_t* bin_active;
-    uint32_t* active_list;         // active bins (any order)
-    unsigned int* active_count;
-    unsigned int* work_next;       // next active bin for the band kernel
+    uint2* items;                  // band kernel's work: bin, part | parts << 8; split bins from the front
+    long long items_cap;           // (item_counts[0]), whole ones from the end (item_counts[1])
+    unsigned int* item_counts;
+    unsigned int* work_next;       // next item
     int* axis_start;               // first point of every bin per axis: [gx+1][gy+1][gz+1]
     float* out;                    // nx*ny*nz values
     uint32_t* far;                 // [nz*ny][W] bits: value is far
@@ -367,6 +367,7 @@ struct SdfParams {
 };
 void sdf_bin_geometry(SdfParams& P);
 size_t sdf_tri_record_bytes();     // bytes of one triangle record in SdfParams::tris
+long long sdf_items_capacity(long long nbins, unsigned long long entries);
 cudaError_t launch_sdf_prep(const SdfParams& P, int num_sms, cudaStream_t s);
 cudaError_t launch_sdf_bins(const SdfParams& P, int num_sms, cudaStream_t s);
 cudaError_t launch_sdf_band(const SdfParams& P, int num_sms, cudaStream_t s);

@@ -23,18 +23,14 @@
 //   k_tri_bins      scatter into bins (atomics), then k_bin_order ranks each bin's entries
 //                   by triangle index (CTA per bin, shared-memory tiles), so the order is the
 //                   ascending one whatever the atomics did
-//   k_bin_active    active flags + a compact list of the active bins; k_axis_starts the
+//   k_bin_active    the active bins as a list of work items; k_axis_starts the
 //                   first grid point of every bin per axis; k_fill_far sets every value far
-//   k_band          persistent CTAs take active bins from a work counter; the 27-bin
-//                   visiting sequence is the same for every point of a bin, so its triangle
-//                   records stream through shared memory once per 8 cubes of 4x4x4 points
-//                   (a cube per warp, 2 points per thread). A triangle whose bounding sphere
-//                   provably lies beyond a point's running minimum plus the tie tolerance is
-//                   skipped — the reference loop would ignore it at that point of the
-//                   sequence, so skipping it changes no bit. The test runs first for a whole
-//                   warp (lane l takes the l-th of 32 triangles against the warp's point box
-//                   and largest reach), then per point, then with the triangle's plane,
-//                   before the exact distance.
+//   k_band          persistent CTAs take work items (a bin or a part of a long one) from a
+//                   counter; the distinct triangles that may be nearest to the item's points are
+//                   staged once in shared memory, a warp takes 32 points at a time (a brick of up
+//                   to 4x4x2), finds each point's minimum and the triangles that tie with it,
+//                   and decides value and sign on those (the reference's walk over every listed
+//                   triangle, without the ones that cannot change its result)
 //   k_sdf_masks     far / positive bit words (ballots over x rows)
 //   k_flood         exterior flood on bit words: 4x16x16-word tiles iterate to local
 //                   convergence in shared memory; the host repeats until nothing changes
@@ -49,15 +45,19 @@ namespace {
 
 constexpr float kFar = FLT_MAX;
 
-// Triangle record, 5 x 16 bytes.
+// Triangle record, 6 x 16 bytes.
 struct Tri {
-    float4 s;   // bounding sphere: centroid xyz, radius grown by a rounding allowance
-    float4 a;   // v0.xyz, doubled area (0: skipped, as the reference skips area <= 1e-12)
-    float4 b;   // v1.xyz
-    float4 c;   // v2.xyz
-    float4 n;   // unit normal xyz
+    float4 s;       // bounding sphere: centroid xyz, radius grown by a rounding allowance
+    float a2;       // doubled area (0: skipped, as the reference skips area <= 1e-12)
+    uint32_t r[3];  // bins it is listed in, per axis: first | last << 16 (kPackedBins axes and below)
+    float v[9];     // vertices
+    float n[3];     // unit normal
+    float w[4];     // tie weights of its vertices: the angles there
 };
-constexpr int kTriF4 = 5;
+constexpr int kTriF4 = 6;
+constexpr int kTriList = 5;             // of them the distances need
+constexpr int kTriAngles = 5;
+constexpr int kPackedBins = 65536;
 static_assert(sizeof(Tri) == kTriF4 * sizeof(float4), "record = kTriF4 float4s");
 
 __device__ __forceinline__ float3 f3(float x, float y, float z) { return make_float3(x, y, z); }
@@ -160,14 +160,18 @@ __global__ void __launch_bounds__(256) k_tri_prep(SdfParams P) {
         const float3 da = sub(a, cc), db = sub(b, cc), dcv = sub(c, cc);
         const float R = sqrtf(fmaxf(dot(da, da), fmaxf(dot(db, db), dot(dcv, dcv))));
         const float mag = fmaxf(fmaxf(fabsf(cc.x), fabsf(cc.y)), fabsf(cc.z)) + R;
-        Tri* t = reinterpret_cast<Tri*>(P.tris) + f;
-        t->s = make_float4(cc.x, cc.y, cc.z, R * 1.0001f + 1e-5f * mag);
-        t->a = make_float4(a.x, a.y, a.z, ok ? a2 : 0.f);
-        t->b = make_float4(b.x, b.y, b.z, 0.f);
-        t->c = make_float4(c.x, c.y, c.z, 0.f);
-        t->n = make_float4(n.x, n.y, n.z, 0.f);
         int r[6];
         tri_bin_range(P, a, b, c, r);
+        float4* t = reinterpret_cast<float4*>(P.tris) + kTriF4 * (size_t)f;
+        t[0] = make_float4(cc.x, cc.y, cc.z, R * 1.0001f + 1e-5f * mag);
+        t[1] = make_float4(ok ? a2 : 0.f, __uint_as_float((uint32_t)r[0] | (uint32_t)r[1] << 16),
+                           __uint_as_float((uint32_t)r[2] | (uint32_t)r[3] << 16),
+                           __uint_as_float((uint32_t)r[4] | (uint32_t)r[5] << 16));
+        t[2] = make_float4(a.x, a.y, a.z, b.x);
+        t[3] = make_float4(b.y, b.z, c.x, c.y);
+        t[4] = make_float4(c.z, n.x, n.y, n.z);
+        t[kTriAngles] = make_float4(angle_at(sub(b, a), sub(c, a), a2), angle_at(sub(a, b), sub(c, b), a2),
+                                    angle_at(sub(a, c), sub(b, c), a2), 0.f);
         for (int bz = r[4]; bz <= r[5]; ++bz)
             for (int by = r[2]; by <= r[3]; ++by)
                 for (int bx = r[0]; bx <= r[1]; ++bx)
@@ -230,19 +234,29 @@ __global__ void __launch_bounds__(kOrderThreads) k_bin_order(SdfParams P) {
     }
 }
 
+// Work items of the band kernel: at most 1 + entries / kPartEntries a bin. Parts repeat the
+// staging of their bin's triangles (512^3, 163,840 triangles: 13.5 ms with parts of 256 entries,
+// 11.3 with 1024) but spread the few long bins of a dense mesh (100^3, 10,240 triangles: 2.0 ms
+// whole, 1.2 with either).
+constexpr uint32_t kPartEntries = 1024;
 __global__ void __launch_bounds__(256) k_bin_active(SdfParams P) {
     for (long long bin = (long long)blockIdx.x * blockDim.x + threadIdx.x; bin < P.nbins; bin += (long long)gridDim.x * blockDim.x) {
         const int bx = (int)(bin % P.gx), by = (int)((bin / P.gx) % P.gy), bz = (int)(bin / ((long long)P.gx * P.gy));
-        uint8_t act = 0;
+        uint32_t entries = 0;
         for (int dz = -1; dz <= 1; ++dz)
             for (int dy = -1; dy <= 1; ++dy)
                 for (int dx = -1; dx <= 1; ++dx) {
                     const int x = bx + dx, y = by + dy, z = bz + dz;
                     if (x < 0 || x >= P.gx || y < 0 || y >= P.gy || z < 0 || z >= P.gz) continue;
-                    if (P.bin_count[x + (long long)P.gx * (y + (long long)P.gy * z)]) act = 1;
+                    entries += P.bin_count[x + (long long)P.gx * (y + (long long)P.gy * z)];
                 }
-        P.bin_active[bin] = act;
-        if (act) P.active_list[atomicAdd(P.active_count, 1u)] = (uint32_t)bin;   // order is irrelevant
+        if (!entries) continue;
+        // a bin with many entries is worked on in parts by several CTAs (its order in the list is
+        // irrelevant: parts from the front, whole bins from the end)
+        const uint32_t parts = entries <= kPartEntries ? 1u : entries <= 4 * kPartEntries ? 2u : entries <= 8 * kPartEntries ? 4u : 8u;
+        const uint32_t at = atomicAdd(P.item_counts + (parts > 1 ? 0 : 1), parts);
+        for (uint32_t q = 0; q < parts; ++q)
+            P.items[parts > 1 ? at + q : P.items_cap - 1 - at] = make_uint2((uint32_t)bin, q | parts << 8);
     }
 }
 
@@ -272,100 +286,360 @@ __global__ void __launch_bounds__(256) k_fill_far(SdfParams P) {
         P.out[q] = kFar;
 }
 
-constexpr int kBandThreads = 256;
-constexpr int kBandChunk = 256;   // triangle records staged per pass (20 KB)
-constexpr int kBandPts = 2;       // grid points per thread (a 4x4x4 cube per warp)
+constexpr int kBandThreads = 128;
+constexpr int kBandWarps = kBandThreads / 32;
+constexpr int kBandCtasPerSm = 6;
+// Triangle records a CTA holds at a time: what leaves room for six CTAs on an SM (a list of 224
+// sends more bins through several lists: 11.8 ms against 11.3 at 512^3).
+constexpr int kBandList = 336;
+constexpr int kBandTies = 7;       // triangles within the tie window of a point's minimum
 
-// Running closest-triangle state of one grid point.
+// Running closest-triangle state of one grid point: squared distance, closest point, summed normals.
 struct BandPoint {
-    float3 p;
-    float best, reach;            // reach: beyond it a triangle cannot reach the tie window
+    float best;
     float3 bp, bn;
 };
 
+__device__ __forceinline__ float tie_tol(float best) { return 1e-5f * (best + 1e-8f); }
+constexpr float kWindow = 12.f;
+__device__ __forceinline__ float window_top(float best) { return best + kWindow * tie_tol(best); }
+
+// Beyond this distance from a point whose largest coordinate is pm, a triangle's float distance
+// is above best and its tie tolerance.
 __device__ __forceinline__ float reach_of(float best, float pm) {
     if (best == kFar) return kFar;
-    return sqrtf(best + 1e-5f * (best + 1e-8f)) * 1.00001f + 1e-5f * pm;
+    return sqrtf(best + tie_tol(best)) * 1.00001f + 1e-5f * pm;
 }
 
-// One triangle against one point, exactly as evaluate_sdf_grid_kernel's loop body, after two
-// lower bounds of the distance: the bounding sphere, then the plane distance h and the
-// lateral distance beyond the sphere (d^2 >= h^2 + (l - R)^2). A triangle beyond the point's
-// reach has a float distance above best + tolerance, so the reference loop ignores it too.
-// The record is read from shared memory by the caller (s_rec = the record's 5 float4s).
-__device__ __forceinline__ void visit(BandPoint& q, float pm, const float4 (&s_rec)[kTriF4], float veps) {
-    const float4 ts = s_rec[0];
-    if (q.best != kFar) {
-        const float dx = q.p.x - ts.x, dy = q.p.y - ts.y, dz = q.p.z - ts.z;
-        const float d2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmul_rn(dz, dz)));
-        const float lim = q.reach + ts.w;
-        if (d2 > __fmul_rn(__fmul_rn(lim, lim), 1.00002f)) return;
-        const float4 tn = s_rec[4];
-        const float reach2 = __fmul_rn(__fmul_rn(q.reach, q.reach), 1.00002f);
-        const float allow = 2e-5f * (pm + fabsf(ts.x) + fabsf(ts.y) + fabsf(ts.z) + ts.w);
-        const float h = __fmaf_rn(dx, tn.x, __fmaf_rn(dy, tn.y, __fmul_rn(dz, tn.z)));
-        const float hh = fmaxf(0.f, fabsf(h) - allow);
-        const float lat = sqrtf(fmaxf(0.f, d2 - h * h));
-        const float ll = fmaxf(0.f, lat - ts.w - allow);
-        if (__fmaf_rn(hh, hh, __fmul_rn(ll, ll)) > reach2) return;
-    }
-    const float4 ta = s_rec[1];
-    if (!(ta.w > 0.f)) return;                          // area <= 1e-12: skipped
-    const float4 tb = s_rec[2], tc = s_rec[3];
-    const float3 v0 = f3(ta.x, ta.y, ta.z), v1 = f3(tb.x, tb.y, tb.z), v2 = f3(tc.x, tc.y, tc.z);
+__device__ __forceinline__ float3 rec_v0(const float4* rec) { return f3(rec[2].x, rec[2].y, rec[2].z); }
+__device__ __forceinline__ float3 rec_v1(const float4* rec) { return f3(rec[2].w, rec[3].x, rec[3].y); }
+__device__ __forceinline__ float3 rec_v2(const float4* rec) { return f3(rec[3].z, rec[3].w, rec[4].x); }
+__device__ __forceinline__ float3 rec_normal(const float4* rec) { return f3(rec[4].y, rec[4].z, rec[4].w); }
+
+// The closest point of a record's triangle to p (xyz) and its squared distance (w). One copy for
+// all callers: inlined, the band kernel no longer fits the instruction cache (14 of 28 stall
+// cycles an instruction were fetches).
+__device__ __noinline__ float4 closest(float3 p, const float4* rec) {
     float3 cp;
-    const float d = point_triangle(q.p, v0, v1, v2, cp);
-    const float tol = 1e-5f * (q.best + 1e-8f);
-    const bool replace = d < q.best - tol;
-    if (!replace && !(fabsf(d - q.best) <= tol)) return;   // ignored: its weight is never used
-    // weight: the doubled area, or the angle at a vertex the closest point sits on
-    float w = ta.w;
-    const float3 c0v = sub(cp, v0), c1v = sub(cp, v1), c2v = sub(cp, v2);
-    if (dot(c0v, c0v) < veps) w = angle_at(sub(v1, v0), sub(v2, v0), w);
-    else if (dot(c1v, c1v) < veps) w = angle_at(sub(v0, v1), sub(v2, v1), w);
-    else if (dot(c2v, c2v) < veps) w = angle_at(sub(v0, v2), sub(v1, v2), w);
-    const float4 tn = s_rec[4];
-    if (replace) {
-        q.best = d;
-        q.bp = cp;
-        q.bn = f3(w * tn.x, w * tn.y, w * tn.z);
-        q.reach = reach_of(d, pm);
-    } else {
-        q.bn = f3(q.bn.x + w * tn.x, q.bn.y + w * tn.y, q.bn.z + w * tn.z);
-    }
+    const float d = point_triangle(p, rec_v0(rec), rec_v1(rec), rec_v2(rec), cp);
+    return make_float4(cp.x, cp.y, cp.z, d);
 }
 
-__global__ void __launch_bounds__(kBandThreads, 2) k_band(SdfParams P) {
-    __shared__ float4 s_tri[kBandChunk][kTriF4];
-    __shared__ int s_seq_bin[27];
-    __shared__ uint32_t s_seq_start[28];
-    __shared__ uint32_t s_next;
-    const uint32_t nact = *P.active_count;
+// A square root from the hardware's approximation, a little below the true one.
+__device__ __forceinline__ float sqrt_below(float x) {
+    float r;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return __fmul_rn(r, 0.999999f);
+}
+
+// Whether the triangle's float distance from p provably exceeds what `reach` was made from:
+// by its bounding sphere, then by its plane distance h and the lateral distance beyond the
+// sphere (d^2 >= h^2 + (l - R)^2).
+__device__ __forceinline__ bool beyond(const float4* rec, float3 p, float pm, float reach) {
+    const float4 ts = rec[0];
+    const float dx = p.x - ts.x, dy = p.y - ts.y, dz = p.z - ts.z;
+    const float d2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmul_rn(dz, dz)));
+    const float lim = reach + ts.w;
+    if (d2 > __fmul_rn(__fmul_rn(lim, lim), 1.00002f)) return true;
+    const float3 n = rec_normal(rec);
+    const float reach2 = __fmul_rn(__fmul_rn(reach, reach), 1.00002f);
+    const float allow = 2e-5f * (pm + fabsf(ts.x) + fabsf(ts.y) + fabsf(ts.z) + ts.w);
+    const float h = __fmaf_rn(dx, n.x, __fmaf_rn(dy, n.y, __fmul_rn(dz, n.z)));
+    const float hh = fmaxf(0.f, fabsf(h) - allow);
+    const float lat = sqrt_below(fmaxf(0.f, d2 - h * h));
+    const float ll = fmaxf(0.f, lat - ts.w - allow);
+    return __fmaf_rn(hh, hh, __fmul_rn(ll, ll)) > reach2;
+}
+
+// The tie weight of triangle f whose closest point is cp: the doubled area, or the angle at a
+// vertex the closest point sits on (from the record).
+__device__ __forceinline__ float tie_weight(const SdfParams& P, uint32_t f, const float4* rec, float3 cp, float veps) {
+    const float3 c0v = sub(cp, rec_v0(rec)), c1v = sub(cp, rec_v1(rec)), c2v = sub(cp, rec_v2(rec));
+    const float* angle = P.tris + 4 * (kTriF4 * (size_t)f + kTriAngles);
+    if (dot(c0v, c0v) < veps) return angle[0];
+    if (dot(c1v, c1v) < veps) return angle[1];
+    if (dot(c2v, c2v) < veps) return angle[2];
+    return rec[1].x;
+}
+
+// One visit of a triangle at squared distance d: replaces the running minimum, ties with it
+// or is ignored, exactly as evaluate_sdf_grid_kernel's loop body. False: ignored.
+__device__ __forceinline__ bool visit(BandPoint& q, float d, float w, float3 tn) {
+    const float tol = tie_tol(q.best);
+    if (d < q.best - tol) {
+        q.best = d;
+        q.bn = f3(w * tn.x, w * tn.y, w * tn.z);
+        return true;
+    }
+    if (fabsf(d - q.best) <= tol) q.bn = f3(q.bn.x + w * tn.x, q.bn.y + w * tn.y, q.bn.z + w * tn.z);
+    return false;
+}
+
+// Signed distance of a point from its closest-triangle state; kFar without one and beyond 2.5 bins.
+__device__ __forceinline__ float band_value(const SdfParams& P, float3 p, const BandPoint& q) {
+    if (q.best == kFar) return kFar;
+    float dist = sqrtf(q.best);
+    float3 bn = q.bn;
+    const float nl = sqrtf(dot(bn, bn));
+    if (nl > 1e-12f) bn = f3(bn.x / nl, bn.y / nl, bn.z / nl);
+    if (dot(sub(p, q.bp), bn) < 0.0f) dist = -dist;
+    return dist > 2.5f * P.min_box || dist < -2.5f * P.min_box ? kFar : dist;
+}
+
+// Visiting order of the 27 bins around a bin: the centre, then the shell in z, y, x order.
+// Bit t of the result: the t-th of them lies in the triangle's bin range (packed, rec[1].yzw).
+__device__ __forceinline__ uint32_t slot_mask(float4 q, int bx, int by, int bz) {
+    auto three = [](float packed, int b) {
+        const uint32_t u = __float_as_uint(packed);
+        const int lo = (int)(u & 0xffffu), hi = (int)(u >> 16);
+        return (lo <= b - 1 && b - 1 <= hi ? 1u : 0u) | (lo <= b && b <= hi ? 2u : 0u) | (lo <= b + 1 && b + 1 <= hi ? 4u : 0u);
+    };
+    const uint32_t mx = three(q.y, bx), my = three(q.z, by), mz = three(q.w, bz);
+    const uint32_t plane = (my & 1u ? mx : 0u) | (my & 2u ? mx << 3 : 0u) | (my & 4u ? mx << 6 : 0u);
+    const uint32_t m = (mz & 1u ? plane : 0u) | (mz & 2u ? plane << 9 : 0u) | (mz & 4u ? plane << 18 : 0u);
+    return ((m >> 13) & 1u) | ((m & 0x1fffu) << 1) | (m & ~0x3fffu);
+}
+
+struct BandShared {
+    float4 tri[kBandList][kTriList];
+    uint32_t idx[kBandList];
+    // triangles in the window of the lanes' minima: place in the list (with several lists the
+    // triangle) and distance
+    uint32_t tie_e[kBandWarps][kBandTies][32];
+    float tie_d[kBandWarps][kBandTies][32];
+    uint32_t live[kBandWarps][(kBandList + 31) / 32];
+    int seq_bin[27];
+    uint32_t seq_start[28];
+    uint32_t next, n, reach, votes[kBandWarps], brick_next;
+    uint32_t redo[4];              // bricks for the full walk (a bin has at most 15 points an axis: 125)
+    int brick[3];
+};
+
+// Entry sq of the bin's visiting sequence: its slot and triangle.
+__device__ __forceinline__ uint32_t seq_entry(const SdfParams& P, const BandShared& S, uint32_t sq, int& slot) {
+    int b = 0;                                   // last slot with start <= sq
+#pragma unroll
+    for (int step = 16; step > 0; step >>= 1)
+        if (b + step < 27 && S.seq_start[b + step] <= sq) b += step;
+    slot = b;
+    return P.bin_tris[P.bin_start[S.seq_bin[b]] + (sq - S.seq_start[b])];
+}
+
+__device__ __forceinline__ float warp_max(float v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+__device__ __forceinline__ float warp_min(float v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = fminf(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+
+// Whether a bounding sphere lies farther than `reach` from the box [lo, hi].
+__device__ __forceinline__ bool sphere_beyond_box(float4 ts, float3 lo, float3 hi, float reach) {
+    const float ex = fmaxf(fmaxf(lo.x - ts.x, ts.x - hi.x), 0.f);
+    const float ey = fmaxf(fmaxf(lo.y - ts.y, ts.y - hi.y), 0.f);
+    const float ez = fmaxf(fmaxf(lo.z - ts.z, ts.z - hi.z), 0.f);
+    const float dd = __fmaf_rn(ex, ex, __fmaf_rn(ey, ey, __fmul_rn(ez, ez)));
+    const float lim = reach + ts.w;
+    return dd > __fmul_rn(__fmul_rn(lim, lim), 1.00002f);
+}
+
+// Signed distances of the active bins' points.
+//
+// What the reference computes per point is a walk over the triangles of 27 bins, a triangle
+// once per bin that lists it (about five times), with a running minimum and a tie rule. The
+// walk's result depends only on the triangles within a few tolerances of the minimum d*: for a
+// g >= d* with no distance in (g, g + 1.15 tol], the first triangle at or below g replaces
+// whatever the walk holds (it is more than tol below everything visited before), and nothing
+// above the gap can tie with or replace what follows. So a warp takes the distinct triangles in
+// any order, keeps those within kWindow tolerances of each point's minimum, finds the gap
+// and decides on the kept ones alone: the magnitude is the distance of the one visited first (they
+// tie), the sign that of its normal's side where all the kept normals agree clearly; else the
+// walk is repeated on the kept ones (their slots among the 27 bins, from the record's bin
+// range, in visiting order, ascending triangle index inside a slot). Points without a gap
+// in the window or with more than kBandTies triangles in it take the full walk (band_serial);
+// so does a grid with over 65536 bins an axis.
+//
+// Bound: instructions (float distances without contraction; 54% issue at 256^3). At 512^3 points
+// and 163,840 triangles the full walk for every point took 46.1 ms, this takes 11.3 ms; 256^3
+// with the same mesh 19.9 and 6.4 ms, 100^3 with 10,240 triangles 4.2 and 1.2 ms.
+__device__ __noinline__ float band_serial(const SdfParams& P, BandShared& S, float3 pt, float pm, bool mine, float3 wlo,
+                                          float3 whi, bool wanted, float veps) {
+    const uint32_t L = S.seq_start[27];
     const int lane = threadIdx.x & 31;
+    BandPoint q;
+    q.best = kFar;
+    q.bp = f3(0.f, 0.f, 0.f);
+    q.bn = f3(0.f, 1.f, 0.f);
+    float reach = kFar;
+    for (uint32_t c0 = 0; c0 < L; c0 += kBandThreads) {
+        const uint32_t m = min((uint32_t)kBandThreads, L - c0);
+        __syncthreads();
+        if (threadIdx.x < m) {
+            int slot;
+            const uint32_t f = seq_entry(P, S, c0 + threadIdx.x, slot);
+            const float4* rec = reinterpret_cast<const float4*>(P.tris) + kTriF4 * (size_t)f;
+#pragma unroll
+            for (int part = 0; part < kTriList; ++part) S.tri[threadIdx.x][part] = rec[part];
+            S.idx[threadIdx.x] = f;
+        }
+        __syncthreads();
+        if (!wanted) continue;
+        for (uint32_t base = 0; base < m; base += 32) {
+            const float wr = warp_max(mine ? reach : 0.f);
+            const uint32_t e = base + lane;
+            const bool cand = e < m && S.tri[e][1].x > 0.f && (wr == kFar || !sphere_beyond_box(S.tri[e][0], wlo, whi, wr));
+            uint32_t live = __ballot_sync(0xffffffffu, cand);
+            while (live) {
+                const uint32_t c = base + __ffs(live) - 1;
+                live &= live - 1;
+                const float4* rec = S.tri[c];
+                if (mine && (reach == kFar || !beyond(rec, pt, pm, reach))) {
+                    const float4 r = closest(pt, rec);
+                    const float3 cp = f3(r.x, r.y, r.z);
+                    if (visit(q, r.w, tie_weight(P, S.idx[c], rec, cp, veps), rec_normal(rec))) {
+                        q.bp = cp;
+                        reach = reach_of(r.w, pm);
+                    }
+                }
+                __syncwarp();
+            }
+        }
+    }
+    return band_value(P, pt, q);
+}
+
+// A kept triangle's record and index (tie_e is a place in the list, or with several lists the
+// triangle).
+__device__ __forceinline__ const float4* tie_record(const SdfParams& P, const BandShared& S, bool single, uint32_t e) {
+    return single ? S.tri[e] : reinterpret_cast<const float4*>(P.tris) + kTriF4 * (size_t)e;
+}
+__device__ __forceinline__ uint32_t tie_triangle(const BandShared& S, bool single, uint32_t e) { return single ? S.idx[e] : e; }
+
+// The walk on a lane's k kept triangles.
+__device__ __noinline__ float band_walk(const SdfParams& P, BandShared& S, bool single, int k, float3 p, int bx, int by, int bz,
+                                        float veps) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float4 tn[kBandTies];                                    // ascending triangle: weighted normal, slots
+    uint32_t slots = 0;
+    for (int t = 0; t < k; ++t) {
+        const uint32_t e = S.tie_e[warp][t][lane];
+        const float dt = S.tie_d[warp][t][lane];
+        const float4* rec = tie_record(P, S, single, e);
+        const float4 r = closest(p, rec);
+        const uint32_t f = tie_triangle(S, single, e), mask = slot_mask(rec[1], bx, by, bz);
+        const float w = tie_weight(P, f, rec, f3(r.x, r.y, r.z), veps);
+        const float3 n = rec_normal(rec);
+        slots |= mask;
+        int to = t;
+        while (to > 0 && tie_triangle(S, single, S.tie_e[warp][to - 1][lane]) > f) {
+            S.tie_e[warp][to][lane] = S.tie_e[warp][to - 1][lane];
+            S.tie_d[warp][to][lane] = S.tie_d[warp][to - 1][lane];
+            tn[to] = tn[to - 1];
+            --to;
+        }
+        S.tie_e[warp][to][lane] = e;
+        S.tie_d[warp][to][lane] = dt;
+        tn[to] = make_float4(w * n.x, w * n.y, w * n.z, __uint_as_float(mask));
+    }
+    BandPoint q;
+    q.best = kFar;
+    q.bn = f3(0.f, 1.f, 0.f);
+    int setter = 0;
+    while (slots) {
+        const uint32_t bit = slots & (0u - slots);
+        slots ^= bit;
+        for (int t = 0; t < k; ++t)
+            if ((__float_as_uint(tn[t].w) & bit) && visit(q, S.tie_d[warp][t][lane], 1.f, f3(tn[t].x, tn[t].y, tn[t].z)))
+                setter = t;
+    }
+    const float4 r = closest(p, tie_record(P, S, single, S.tie_e[warp][setter][lane]));
+    q.bp = f3(r.x, r.y, r.z);
+    return band_value(P, p, q);
+}
+
+// Fills the shared list with the next distinct triangles of the bin's sequence (from entry e0)
+// that may lie within `reach` of the box [lo, hi]; returns the entry it stopped at (S.n: how
+// many it holds). CTA-wide.
+__device__ uint32_t band_fill(const SdfParams& P, BandShared& S, uint32_t e0, int bx, int by, int bz, float3 lo, float3 hi,
+                              float reach) {
+    const uint32_t L = S.seq_start[27];
+    const int lane = threadIdx.x & 31;
+    __syncthreads();
+    uint32_t have = 0;
+    while (e0 < L) {
+        const uint32_t sq = e0 + threadIdx.x;
+        bool keep = false;
+        uint32_t f = 0, mask = 0;
+        float4 ts = make_float4(0.f, 0.f, 0.f, 0.f), tq = ts;
+        const float4* rec = nullptr;
+        if (sq < L) {
+            int slot;
+            f = seq_entry(P, S, sq, slot);
+            rec = reinterpret_cast<const float4*>(P.tris) + kTriF4 * (size_t)f;
+            ts = rec[0];
+            tq = rec[1];
+            mask = slot_mask(tq, bx, by, bz);
+            keep = tq.x > 0.f && slot == __ffs(mask) - 1 && !sphere_beyond_box(ts, lo, hi, reach);
+        }
+        const uint32_t votes = __ballot_sync(0xffffffffu, keep);
+        if (lane == 0) S.votes[threadIdx.x >> 5] = __popc(votes);
+        __syncthreads();
+        uint32_t at = have + __popc(votes & ((1u << lane) - 1u)), all = 0;
+#pragma unroll
+        for (int w = 0; w < kBandWarps; ++w) {
+            if (w < (int)(threadIdx.x >> 5)) at += S.votes[w];
+            all += S.votes[w];
+        }
+        if (have + all > (uint32_t)kBandList) break;     // this stretch starts the next list
+        if (keep) {
+            S.tri[at][0] = ts;
+            S.tri[at][1] = tq;
+#pragma unroll
+            for (int part = 2; part < kTriList; ++part) S.tri[at][part] = rec[part];
+            S.idx[at] = f;
+        }
+        have += all;
+        e0 += kBandThreads;
+        __syncthreads();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) S.n = have;
+    __syncthreads();
+    return e0;
+}
+
+__global__ void __launch_bounds__(kBandThreads, kBandCtasPerSm) k_band(SdfParams P) {
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    BandShared& S = *reinterpret_cast<BandShared*>(s_raw);
+    const uint32_t nlong = P.item_counts[0], nitems = nlong + P.item_counts[1];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const float veps = 1e-6f * P.min_box * P.min_box;
+    // squared distances beyond far2 make a point far, whatever its ties
+    const float far1 = (2.5f * P.min_box) * (2.5f * P.min_box);
+    const float far2 = far1 > FLT_MIN && far1 < 1e37f ? far1 * 1.001f + 2.f * kWindow * tie_tol(far1) : kFar;
+    const bool packed = P.gx <= kPackedBins && P.gy <= kPackedBins && P.gz <= kPackedBins;
     for (;;) {
-        // next active bin from the shared work counter (bins differ a lot in cost)
+        // next item from the shared work counter (bins differ a lot in cost: the parts of the long
+        // ones come first, the others stand at the end of the list)
         __syncthreads();
-        if (threadIdx.x == 0) s_next = atomicAdd(P.work_next, 1u);
+        if (threadIdx.x == 0) S.next = atomicAdd(P.work_next, 1u);
         __syncthreads();
-        const uint32_t ai = s_next;
-        if (ai >= nact) break;
-        const long long bin = P.active_list[ai];
+        const uint32_t ai = S.next;
+        if (ai >= nitems) break;
+        const uint2 item = P.items[ai < nlong ? ai : P.items_cap - 1 - (ai - nlong)];
+        const long long bin = item.x;
+        const int part = (int)(item.y & 0xffu), parts = (int)(item.y >> 8);
         const int bx = (int)(bin % P.gx), by = (int)((bin / P.gx) % P.gy), bz = (int)(bin / ((long long)P.gx * P.gy));
         const int* ys_ = P.axis_start + P.gx + 1;
         const int* zs_ = ys_ + P.gy + 1;
-        const int x0 = P.axis_start[bx], x1 = P.axis_start[bx + 1];
-        const int y0 = ys_[by], y1 = ys_[by + 1];
-        const int z0 = zs_[bz], z1 = zs_[bz + 1];
-        const int sx = x1 - x0, sy = y1 - y0, sz = z1 - z0;
+        const int x0 = P.axis_start[bx], y0 = ys_[by], z0 = zs_[bz];
+        const int sx = P.axis_start[bx + 1] - x0, sy = ys_[by + 1] - y0, sz = zs_[bz + 1] - z0;
         if (sx <= 0 || sy <= 0 || sz <= 0) continue;
-        // points go to warps in 4x4x4 cubes (lane: 4x4x2, the second point 2 planes up), so
-        // that a warp's point box, used to cull triangles, stays small
-        const int cx4 = (sx + 3) / 4, cy4 = (sy + 3) / 4, cz4 = (sz + 3) / 4;
-        const int ncubes = cx4 * cy4 * cz4;
-        // visiting sequence: centre bin, then the shell of radius 1 in z, y, x order; lane t of
-        // warp 0 takes the t-th of the 27 slots, a warp scan gives the starts
-        __syncthreads();
         if (threadIdx.x < 32) {
+            // visiting sequence: lane t takes the t-th of the 27 slots, a warp scan gives the starts
             const int t = threadIdx.x;
             int nb = -1;
             if (t == 0) {
@@ -383,114 +657,281 @@ __global__ void __launch_bounds__(kBandThreads, 2) k_band(SdfParams P) {
                 const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
                 if (t >= o) incl += v;
             }
-            if (t < 27) { s_seq_bin[t] = nb; s_seq_start[t] = incl - c; }
-            if (t == 26) s_seq_start[27] = incl;
+            if (t < 27) { S.seq_bin[t] = nb; S.seq_start[t] = incl - c; }
+            if (t == 26) S.seq_start[27] = incl;
+            // brick of points per warp, a point a lane: sides of 2 to 4 points that cover the bin
+            // in the fewest bricks (8 points an axis: 4x4x2; 9: 3x3x3)
+            const int kx = (sx + 1 + t % 3) / (2 + t % 3), ky = (sy + 1 + t / 3 % 3) / (2 + t / 3 % 3),
+                      kz = (sz + 1 + t / 9) / (2 + t / 9);
+            const int wx = (sx + kx - 1) / kx, wy = (sy + ky - 1) / ky, wz = (sz + kz - 1) / kz;
+            int cost = t < 27 && wx * wy * wz <= 32 ? 32 * kx * ky * kz + t : 0x7fffffff;
+            const int mine_cost = cost;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) cost = min(cost, __shfl_xor_sync(0xffffffffu, cost, o));
+            if (mine_cost == cost) { S.brick[0] = wx; S.brick[1] = wy; S.brick[2] = wz; }
+            if (t == 0) S.reach = __float_as_uint(kFar);
+            if (t < 4) S.redo[t] = 0;
         }
         __syncthreads();
-        const uint32_t L = s_seq_start[27];
-        const float veps = 1e-6f * P.min_box * P.min_box;
-        for (int cube0 = 0; cube0 < ncubes; cube0 += kBandThreads / 32) {
-            BandPoint q[kBandPts];
-            float pm[kBandPts];
-            bool mine[kBandPts];
-            int pidx[kBandPts][3];
-            const int cube = cube0 + (threadIdx.x >> 5);
-            const int ccx = cube % cx4, ccy = (cube / cx4) % cy4, ccz = cube / (cx4 * cy4);
-#pragma unroll
-            for (int u = 0; u < kBandPts; ++u) {
-                const int lx = 4 * ccx + (lane & 3), ly = 4 * ccy + ((lane >> 2) & 3), lz = 4 * ccz + (lane >> 4) + 2 * u;
-                mine[u] = cube < ncubes && lx < sx && ly < sy && lz < sz;
-                const int ix = x0 + (mine[u] ? lx : 0), iy = y0 + (mine[u] ? ly : 0), iz = z0 + (mine[u] ? lz : 0);
-                pidx[u][0] = ix; pidx[u][1] = iy; pidx[u][2] = iz;
-                q[u].p = f3(P.ox + (float)ix * P.vx, P.oy + (float)iy * P.vy, P.oz + (float)iz * P.vz);
-                pm[u] = fmaxf(fabsf(q[u].p.x), fmaxf(fabsf(q[u].p.y), fabsf(q[u].p.z)));
-                q[u].best = kFar;
-                q[u].reach = kFar;
-                q[u].bp = f3(0.f, 0.f, 0.f);
-                q[u].bn = f3(0.f, 1.f, 0.f);
+        const uint32_t L = S.seq_start[27];
+        const int wx = S.brick[0], wy = S.brick[1], wz = S.brick[2];
+        const int nbx = (sx + wx - 1) / wx, nby = (sy + wy - 1) / wy, nbz = (sz + wz - 1) / wz;
+        const int nbricks = nbx * nby * nbz;
+        const int brick_lo = nbricks * part / parts, brick_hi = nbricks * (part + 1) / parts;
+        if (brick_lo >= brick_hi) continue;
+        if (threadIdx.x == 0) S.brick_next = brick_lo;
+        const int zlo = z0 + wz * (brick_lo / (nbx * nby)), zhi = min(z0 + sz, z0 + wz * ((brick_hi - 1) / (nbx * nby) + 1)) - 1;
+        // the item's points, and a bound of their distances: to the centroid nearest their middle
+        const float3 blo = f3(P.ox + (float)x0 * P.vx, P.oy + (float)y0 * P.vy, P.oz + (float)zlo * P.vz);
+        const float3 bhi = f3(P.ox + (float)(x0 + sx - 1) * P.vx, P.oy + (float)(y0 + sy - 1) * P.vy,
+                              P.oz + (float)zhi * P.vz);
+        const float bpm = fmaxf(fmaxf(fmaxf(fabsf(blo.x), fabsf(bhi.x)), fmaxf(fabsf(blo.y), fabsf(bhi.y))),
+                                fmaxf(fabsf(blo.z), fabsf(bhi.z)));
+        float reach_bin = reach_of(far2, bpm);
+        uint32_t stop = 0;
+        bool single = false;
+        if (packed) {
+            // Only triangles whose float distances are good are asked: not slivers (a2 is 2.6 R^2
+            // for an equilateral one) nor tiny ones (barycentrics lose (distance / side)^2 ulps);
+            // two radii of slack.
+            const float3 mid = f3(0.5f * (blo.x + bhi.x), 0.5f * (blo.y + bhi.y), 0.5f * (blo.z + bhi.z));
+            const float small = 0.004f * reach_bin;
+            float near = kFar;
+#pragma unroll 4
+            for (uint32_t sq = threadIdx.x; sq < L; sq += kBandThreads) {
+                int slot;
+                const uint32_t f = seq_entry(P, S, sq, slot);
+                const float4* rec = reinterpret_cast<const float4*>(P.tris) + kTriF4 * (size_t)f;
+                const float4 ts = rec[0];
+                const float3 e = f3(ts.x - mid.x, ts.y - mid.y, ts.z - mid.z);
+                const float d = sqrtf(dot(e, e)) + 2.f * ts.w;
+                if (ts.w > small && rec[1].x > 0.26f * ts.w * ts.w) near = fminf(near, d);
             }
-            // box of this warp's points (lanes without a point add nothing)
-            float3 wlo = f3(kFar, kFar, kFar), whi = f3(-kFar, -kFar, -kFar);
-#pragma unroll
-            for (int u = 0; u < kBandPts; ++u) {
-                if (!mine[u]) continue;
-                wlo = f3(fminf(wlo.x, q[u].p.x), fminf(wlo.y, q[u].p.y), fminf(wlo.z, q[u].p.z));
-                whi = f3(fmaxf(whi.x, q[u].p.x), fmaxf(whi.y, q[u].p.y), fmaxf(whi.z, q[u].p.z));
+            near = warp_min(near);
+            if (lane == 0) atomicMin(&S.reach, __float_as_uint(near));     // non-negative floats order as integers
+            __syncthreads();
+            near = __uint_as_float(S.reach);
+            if (near < 1e18f) {
+                const float3 hd = sub(bhi, mid);
+                const float ub = (near + sqrtf(dot(hd, hd))) * 1.0001f + 1e-5f * bpm;
+                reach_bin = fminf(reach_bin, reach_of(ub * ub * 1.001f + 2.f * kWindow * tie_tol(ub * ub), bpm));
             }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                wlo.x = fminf(wlo.x, __shfl_xor_sync(0xffffffffu, wlo.x, o));
-                wlo.y = fminf(wlo.y, __shfl_xor_sync(0xffffffffu, wlo.y, o));
-                wlo.z = fminf(wlo.z, __shfl_xor_sync(0xffffffffu, wlo.z, o));
-                whi.x = fmaxf(whi.x, __shfl_xor_sync(0xffffffffu, whi.x, o));
-                whi.y = fmaxf(whi.y, __shfl_xor_sync(0xffffffffu, whi.y, o));
-                whi.z = fmaxf(whi.z, __shfl_xor_sync(0xffffffffu, whi.z, o));
+            stop = band_fill(P, S, 0, bx, by, bz, blo, bhi, reach_bin);
+            single = stop >= L;
+        }
+        float3 pt;
+        float pm, val;
+        bool mine;
+        long long at;
+        float3 wlo, whi;                     // box of this warp's points (lanes without a point add nothing)
+        auto take = [&](int brick) {
+            const int qx = brick % nbx, qy = (brick / nbx) % nby, qz = brick / (nbx * nby);
+            const int lx = wx * qx + lane % wx, ly = wy * qy + (lane / wx) % wy, lz = wz * qz + lane / (wx * wy);
+            mine = brick < brick_hi && lane < wx * wy * wz && lx < sx && ly < sy && lz < sz;
+            const int ix = x0 + (mine ? lx : 0), iy = y0 + (mine ? ly : 0), iz = z0 + (mine ? lz : 0);
+            at = ix + (long long)P.nx * (iy + (long long)P.ny * iz);
+            pt = f3(P.ox + (float)ix * P.vx, P.oy + (float)iy * P.vy, P.oz + (float)iz * P.vz);
+            pm = fmaxf(fabsf(pt.x), fmaxf(fabsf(pt.y), fabsf(pt.z)));
+            val = kFar;
+            wlo = f3(warp_min(mine ? pt.x : kFar), warp_min(mine ? pt.y : kFar), warp_min(mine ? pt.z : kFar));
+            whi = f3(warp_max(mine ? pt.x : -kFar), warp_max(mine ? pt.y : -kFar), warp_max(mine ? pt.z : -kFar));
+        };
+        // Minimum and kept triangles of the warp's points over the list in shared memory.
+        float best = 0.f, reach = 0.f;
+        int m = 0;
+        bool serial = false;
+        auto start = [&]() {
+            serial = false;
+            best = far2;
+            reach = fminf(reach_of(far2, pm), reach_bin);
+            m = 0;
+        };
+        auto gather = [&](uint32_t n) {
+            // a first reach: the triangle whose centroid is nearest the brick's middle
+            const float3 mid = f3(0.5f * (wlo.x + whi.x), 0.5f * (wlo.y + whi.y), 0.5f * (wlo.z + whi.z));
+            float near = kFar;
+            uint32_t seed = 0;
+            for (uint32_t e = lane; e < n; e += 32) {
+                const float4 ts = S.tri[e][0];
+                const float3 v = f3(ts.x - mid.x, ts.y - mid.y, ts.z - mid.z);
+                const float d2 = dot(v, v);
+                if (d2 < near) { near = d2; seed = e; }
             }
-            for (uint32_t c0 = 0; c0 < L; c0 += kBandChunk) {
-                const uint32_t m = min((uint32_t)kBandChunk, L - c0);
-                __syncthreads();
-                for (uint32_t ent = threadIdx.x; ent < m; ent += kBandThreads) {
-                    const uint32_t sq = c0 + ent;
-                    int b = 0;                                   // last slot with start <= sq
-#pragma unroll
-                    for (int step = 16; step > 0; step >>= 1)
-                        if (b + step < 27 && s_seq_start[b + step] <= sq) b += step;
-                    const uint32_t f = P.bin_tris[P.bin_start[s_seq_bin[b]] + (sq - s_seq_start[b])];
-                    const float4* rec = reinterpret_cast<const float4*>(P.tris) + kTriF4 * (size_t)f;
-                    float4 r[kTriF4];
-#pragma unroll
-                    for (int part = 0; part < kTriF4; ++part) r[part] = rec[part];
-#pragma unroll
-                    for (int part = 0; part < kTriF4; ++part) s_tri[ent][part] = r[part];
-                }
-                __syncthreads();
-                // Warp culling: lane l tests entry base+l against the box of the warp's points
-                // and the warp's largest reach; only entries that pass are visited by every
-                // lane (each of which still applies its own exact-preserving tests).
-                for (uint32_t base = 0; base < m; base += 32) {
-                    float wr = 0.f;
-#pragma unroll
-                    for (int u = 0; u < kBandPts; ++u)
-                        if (mine[u]) wr = fmaxf(wr, q[u].reach);
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) wr = fmaxf(wr, __shfl_xor_sync(0xffffffffu, wr, o));
-                    const uint32_t e = base + lane;
-                    bool cand = false;
-                    if (e < m && s_tri[e][1].w > 0.f) {
-                        cand = true;
-                        if (wr != kFar) {
-                            const float4 ts = s_tri[e][0];
-                            const float ex = fmaxf(fmaxf(wlo.x - ts.x, ts.x - whi.x), 0.f);
-                            const float ey = fmaxf(fmaxf(wlo.y - ts.y, ts.y - whi.y), 0.f);
-                            const float ez = fmaxf(fmaxf(wlo.z - ts.z, ts.z - whi.z), 0.f);
-                            const float dd = __fmaf_rn(ex, ex, __fmaf_rn(ey, ey, __fmul_rn(ez, ez)));
-                            const float lim = wr + ts.w;
-                            cand = !(dd > __fmul_rn(__fmul_rn(lim, lim), 1.00002f));
+            const float all = warp_min(near);
+            const uint32_t who = __ballot_sync(0xffffffffu, near == all);
+            seed = __shfl_sync(0xffffffffu, seed, __ffs(who) - 1);
+            // Three stages through one loop (one copy of its code): 0, the seed; 1, of what is left
+            // against the brick's box the triangle with the centroid nearest each point; 2, what may
+            // reach each point, 32 triangles at a time, every lane taking its own, so that
+            // lanes work on different triangles at a time.
+            uint32_t own = seed, bits = mine ? 1u : 0u, base = seed;
+            for (int stage = 0;;) {
+                while (__ballot_sync(0xffffffffu, bits != 0u)) {
+                    if (bits) {
+                        const uint32_t e = base + __ffs(bits) - 1;
+                        bits &= bits - 1;
+                        const float d = closest(pt, S.tri[e]).w;
+                        if (d <= window_top(best)) {
+                            if (d < best) {
+                                const float top = window_top(d);
+                                if (best > top) m = 0;               // all kept ones are out of the window
+                                best = d;
+                                reach = fminf(reach, reach_of(top, pm));
+                            }
+                            if (m == kBandTies) {
+                                const float top = window_top(best);
+                                m = 0;
+                                for (int t = 0; t < kBandTies; ++t) {
+                                    const float dt = S.tie_d[warp][t][lane];
+                                    if (dt > top) continue;
+                                    S.tie_d[warp][m][lane] = dt;
+                                    S.tie_e[warp][m][lane] = S.tie_e[warp][t][lane];
+                                    ++m;
+                                }
+                            }
+                            if (m < kBandTies) {
+                                S.tie_d[warp][m][lane] = d;
+                                S.tie_e[warp][m][lane] = single ? e : S.idx[e];
+                                ++m;
+                            } else {
+                                serial = true;
+                            }
                         }
                     }
-                    uint32_t live = __ballot_sync(0xffffffffu, cand);
+                    __syncwarp();
+                }
+                if (stage == 0) {
+                    const float wr = warp_max(mine ? reach : 0.f);
+                    float cd = kFar;
+                    for (uint32_t b0 = 0; b0 < n; b0 += 32) {
+                        const uint32_t e = b0 + lane;
+                        const bool cand = e < n && e != seed && !sphere_beyond_box(S.tri[e][0], wlo, whi, wr);
+                        uint32_t live = __ballot_sync(0xffffffffu, cand);
+                        if (lane == 0) S.live[warp][b0 >> 5] = live;
+                        while (live) {
+                            const uint32_t c = b0 + __ffs(live) - 1;
+                            live &= live - 1;
+                            const float4 ts = S.tri[c][0];
+                            const float dx = pt.x - ts.x, dy = pt.y - ts.y, dz = pt.z - ts.z;
+                            const float d2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmul_rn(dz, dz)));
+                            if (d2 < cd) { cd = d2; own = c; }
+                        }
+                    }
+                    __syncwarp();
+                    base = own;
+                    bits = mine && own != seed ? 1u : 0u;
+                    stage = 1;
+                } else {
+                    base = stage == 1 ? 0u : base + 32u;
+                    stage = 2;
+                    if (base >= n) break;
+                    bits = 0;
+                    uint32_t live = S.live[warp][base >> 5];
                     while (live) {
                         const int b = __ffs(live) - 1;
                         live &= live - 1;
-#pragma unroll
-                        for (int u = 0; u < kBandPts; ++u)
-                            if (mine[u]) visit(q[u], pm[u], s_tri[base + b], veps);
+                        if (!beyond(S.tri[base + b], pt, pm, reach)) bits |= 1u << b;
                     }
+                    if (!mine) bits = 0;
+                    if (own - base < 32u) bits &= ~(1u << (own - base));
                 }
             }
-#pragma unroll
-            for (int u = 0; u < kBandPts; ++u) {
-                if (!mine[u]) continue;
-                float val = kFar;
-                if (q[u].best != kFar) {
-                    float dist = sqrtf(q[u].best);
-                    float3 bn = q[u].bn;
-                    const float nl = sqrtf(dot(bn, bn));
-                    if (nl > 1e-12f) bn = f3(bn.x / nl, bn.y / nl, bn.z / nl);
-                    if (dot(sub(q[u].p, q[u].bp), bn) < 0.0f) dist = -dist;
-                    if (!(dist > 2.5f * P.min_box || dist < -2.5f * P.min_box)) val = dist;
+            __syncwarp();
+        };
+        // The value from the kept triangles; sets serial where the window does not decide.
+        auto decide = [&]() {
+            if (!mine || !(best < far2) || serial) return;
+            const float top = window_top(best), gap = 1.15f * tie_tol(top);
+            float g = best;
+            for (;;) {
+                float next = kFar;
+                for (int t = 0; t < m; ++t) {
+                    const float dt = S.tie_d[warp][t][lane];
+                    if (dt > g) next = fminf(next, dt);
                 }
-                P.out[pidx[u][0] + (long long)P.nx * (pidx[u][1] + (long long)P.ny * pidx[u][2])] = val;
+                if (next - g > gap) break;
+                g = next;
+            }
+            if (g + gap > top) { serial = true; return; }
+            int k = 0;
+            for (int t = 0; t < m; ++t) {                      // those at or below g
+                const float dt = S.tie_d[warp][t][lane];
+                if (dt > g) continue;
+                S.tie_d[warp][k][lane] = dt;
+                S.tie_e[warp][k][lane] = S.tie_e[warp][t][lane];
+                ++k;
+            }
+            // the first one visited: by slot, then triangle
+            int first = 0;
+            if (k > 1) {
+                uint32_t slot1 = 33, tri1 = 0;
+                for (int t = 0; t < k; ++t) {
+                    const uint32_t e = S.tie_e[warp][t][lane];
+                    const uint32_t slot = __ffs(slot_mask(tie_record(P, S, single, e)[1], bx, by, bz));
+                    const uint32_t tri = tie_triangle(S, single, e);
+                    if (slot < slot1 || (slot == slot1 && tri < tri1)) { slot1 = slot; tri1 = tri; first = t; }
+                }
+            }
+            BandPoint q;
+            q.best = S.tie_d[warp][first][lane];
+            const float4 r = closest(pt, tie_record(P, S, single, S.tie_e[warp][first][lane]));
+            q.bp = f3(r.x, r.y, r.z);
+            // all tie with the first, and all normals on one side by 1e-3 of the distance: every
+            // sum of them lies on that side
+            const float3 v = sub(pt, q.bp);
+            const float vv = dot(v, v), clear = vv > 1e-30f ? 1e-3f * sqrtf(vv) : kFar;
+            bool above = true, below = true;
+            for (int t = 0; t < k; ++t) {
+                const float side = dot(v, rec_normal(tie_record(P, S, single, S.tie_e[warp][t][lane])));
+                above = above && side > clear;
+                below = below && side < -clear;
+            }
+            if ((above || below) && g - best <= 0.99f * tie_tol(best)) {
+                q.bn = above ? v : f3(-v.x, -v.y, -v.z);
+                val = band_value(P, pt, q);
+            } else {
+                val = band_walk(P, S, single, k, pt, bx, by, bz, veps);
+            }
+        };
+        auto finish = [&](int brick) {
+            if (__ballot_sync(0xffffffffu, serial) && lane == 0 && brick < brick_hi)
+                atomicOr(&S.redo[brick >> 5], 1u << (brick & 31));
+            if (mine) P.out[at] = val;
+        };
+        // With one list the warps take bricks as they come; with several they go through the
+        // lists together.
+        for (int brick = brick_lo + warp;;) {
+            if (single) {
+                if (lane == 0) brick = (int)atomicAdd(&S.brick_next, 1u);
+                brick = __shfl_sync(0xffffffffu, brick, 0);
+            }
+            if ((single ? brick : brick - warp) >= brick_hi) break;
+            take(brick);
+            start();
+            if (packed) {
+                for (uint32_t e0 = single ? stop : 0u;;) {
+                    if (!single) e0 = band_fill(P, S, e0, bx, by, bz, blo, bhi, reach_bin);
+                    if (brick < brick_hi && S.n) gather(S.n);
+                    if (e0 >= L) break;
+                }
+                __syncwarp();
+                decide();
+                __syncwarp();
+            } else {
+                serial = true;
+            }
+            finish(brick);
+            if (!single) brick += kBandWarps;
+        }
+        __syncthreads();
+        if (S.redo[0] | S.redo[1] | S.redo[2] | S.redo[3]) {
+            for (int brick0 = 0; brick0 < nbricks; brick0 += kBandWarps) {
+                const uint32_t flags = (S.redo[brick0 >> 5] >> (brick0 & 31)) & ((1u << kBandWarps) - 1u);
+                if (!flags) continue;
+                const bool want = (flags >> warp) & 1u;
+                take(brick0 + warp);
+                val = band_serial(P, S, pt, pm, mine, wlo, whi, want, veps);
+                if (want && mine) P.out[at] = val;
             }
         }
     }
@@ -724,6 +1165,11 @@ unsigned grid_for(long long items, int per_block, int num_sms, int per_sm) {
 
 size_t sdf_tri_record_bytes() { return sizeof(Tri); }
 
+// Bound of the band kernel's work items: the bins' 27-bin entry counts sum to at most 27 * entries.
+long long sdf_items_capacity(long long nbins, unsigned long long entries) {
+    return nbins + (long long)(27 * entries / kPartEntries) + 1;
+}
+
 void sdf_bin_geometry(SdfParams& P) {
     P.gx = std::max(1, P.nx / 8);
     P.gy = std::max(1, P.ny / 8);
@@ -754,7 +1200,10 @@ cudaError_t launch_sdf_bins(const SdfParams& P, int num_sms, cudaStream_t s) {
 }
 
 cudaError_t launch_sdf_band(const SdfParams& P, int num_sms, cudaStream_t s) {
-    k_band<<<grid_for(P.nbins, 1, num_sms, 2), kBandThreads, 0, s>>>(P);   // persistent: 2 CTAs per SM
+    // persistent: every CTA that fits on the GPU at once takes bins from the work counter
+    cudaError_t e = cudaFuncSetAttribute(k_band, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BandShared));
+    if (e != cudaSuccess) return e;
+    k_band<<<grid_for(P.items_cap, 1, num_sms, kBandCtasPerSm), kBandThreads, sizeof(BandShared), s>>>(P);
     return cudaGetLastError();
 }
 
