@@ -271,6 +271,13 @@ struct OursCell {
     int hmask;            // edges with a Hermite sample
     int fmask;            // faces with a point
 };
+// Internal BVH node, one 64-byte line: both children's boxes (lo xyz, hi xyz) and the children
+// (< 0: ~triangle).
+struct __align__(16) BvhNode {
+    float box[2][6];
+    int child[2];
+    int pad[2];
+};
 struct OursParams {
     GridDesc g;
     const uint64_t* list;
@@ -299,19 +306,20 @@ struct OursParams {
     unsigned int* cell_start;
     unsigned int* cell_fill;
     uint32_t* cell_spheres;         // grid points by cell, by radius
+    float4* cell_centres;           // their positions and values
     int* prev_tri;                  // [npts] closest triangle of each grid point last time
-    uint32_t* heavy;                // cells with many spheres (a warp each)
-    unsigned int* heavy_count;
+    uint32_t* team_list[3];         // cells by number of spheres (the inner loop's team sizes)
+    unsigned int* team_count;       // [3] their numbers, [3] next to take
+    uint32_t* long_query;           // selected points whose search exceeded a thread's budget
+    unsigned int* long_count;
     long long nt;                   // triangles
     unsigned long long* mkeys_sorted;
     uint32_t* tcode;                // triangles' 30-bit Morton codes and indices, then sorted
     uint32_t* tidx;
     uint32_t* tcode_sorted;
     uint32_t* tidx_sorted;
-    int2* child;                    // internal nodes: children (< 0: ~leaf)
-    int* parent;                    // [2 nt]: internal nodes, then leaves at nt - 1 + leaf
-    float4* bmin;
-    float4* bmax;
+    BvhNode* nodes;                 // [nt - 1] internal nodes
+    int* parent;                    // [2 nt]: internal nodes, then leaves at nt - 1 + leaf: node << 1 | side
     unsigned int* flags;
     double* tri9;                   // [9 nt] triangle vertices
 };

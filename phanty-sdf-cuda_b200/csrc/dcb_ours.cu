@@ -22,7 +22,8 @@
 //      proximal rows (Cell::minimize_qef, Cell.cpp:364-473), until the vertex moves less
 //      than 1e-6 (contouring.cpp:1288-1309).
 // Everything is FP64 and compiled with --fmad=false, like the CPU restatement it is checked
-// against. One thread per cell (steps 3-5), per quad (1), per grid point (2).
+// against. One thread per cell (steps 3, 4), per quad (1), per grid point (2; a warp for the
+// points with long searches), a team of lanes per cell (5).
 #include <cfloat>
 #include "dcb_f64.cuh"
 #include "dcb_sort.cuh"
@@ -31,16 +32,9 @@ namespace dcb {
 
 namespace {
 
-// Corners of the six faces (vertex_refinement.cpp:12-19), faces 0:+X 1:-X 2:+Y 3:-Y 4:+Z 5:-Z.
-__constant__ int kFaceCorners[6][4] = {{1, 5, 6, 2}, {0, 3, 7, 4}, {2, 6, 7, 3}, {0, 4, 5, 1}, {4, 7, 6, 5}, {0, 1, 2, 3}};
-
-__device__ __forceinline__ int edge_of_corners(int c1, int c2) {
-    for (int e = 0; e < 12; ++e) {
-        const int a = edge_a(e), b = edge_b(e);
-        if ((c1 == a && c2 == b) || (c1 == b && c2 == a)) return e;
-    }
-    return -1;
-}
+// The four edges around each face, faces 0:+X 1:-X 2:+Y 3:-Y 4:+Z 5:-Z (between consecutive
+// corners of vertex_refinement.cpp:12-19).
+__constant__ int kFaceEdges[6][4] = {{9, 5, 10, 1}, {3, 11, 7, 8}, {10, 6, 11, 2}, {8, 4, 9, 0}, {7, 6, 5, 4}, {0, 1, 2, 3}};
 
 __device__ __forceinline__ double dot3(const double* a, const double* b) { return a[0] * b[0] + a[1] * b[1] + a[2] * b[2]; }
 __device__ __forceinline__ double norm3(const double* a) { return sqrt(a[0] * a[0] + a[1] * a[1] + a[2] * a[2]); }
@@ -78,42 +72,7 @@ __device__ void seg_closest(const double* p, const double* a, const double* b, d
     for (int d = 0; d < 3; ++d) out[d] = a[d] + t * ab[d];
 }
 
-__device__ void tri_closest(const double* p, const double* a, const double* b, const double* c, double* out) {
-    double ab[3], ac[3], ap[3], bp[3], cp[3];
-    for (int d = 0; d < 3; ++d) { ab[d] = b[d] - a[d]; ac[d] = c[d] - a[d]; ap[d] = p[d] - a[d]; }
-    const double d1 = dot3(ab, ap), d2 = dot3(ac, ap);
-    if (d1 <= 0.0 && d2 <= 0.0) { for (int d = 0; d < 3; ++d) out[d] = a[d]; return; }
-    for (int d = 0; d < 3; ++d) bp[d] = p[d] - b[d];
-    const double d3 = dot3(ab, bp), d4 = dot3(ac, bp);
-    if (d3 >= 0.0 && d4 <= d3) { for (int d = 0; d < 3; ++d) out[d] = b[d]; return; }
-    const double vc = d1 * d4 - d3 * d2;
-    if (vc <= 0.0 && d1 >= 0.0 && d3 <= 0.0) {
-        const double v = d1 / (d1 - d3);
-        for (int d = 0; d < 3; ++d) out[d] = a[d] + v * ab[d];
-        return;
-    }
-    for (int d = 0; d < 3; ++d) cp[d] = p[d] - c[d];
-    const double d5 = dot3(ab, cp), d6 = dot3(ac, cp);
-    if (d6 >= 0.0 && d5 <= d6) { for (int d = 0; d < 3; ++d) out[d] = c[d]; return; }
-    const double vb = d5 * d2 - d1 * d6;
-    if (vb <= 0.0 && d2 >= 0.0 && d6 <= 0.0) {
-        const double w = d2 / (d2 - d6);
-        for (int d = 0; d < 3; ++d) out[d] = a[d] + w * ac[d];
-        return;
-    }
-    const double va = d3 * d6 - d5 * d4;
-    if (va <= 0.0 && (d4 - d3) >= 0.0 && (d5 - d6) >= 0.0) {
-        const double w = (d4 - d3) / ((d4 - d3) + (d5 - d6));
-        for (int d = 0; d < 3; ++d) out[d] = b[d] + w * (c[d] - b[d]);
-        return;
-    }
-    const double sum = va + vb + vc;
-    if (sum != 0.0 && isfinite(sum)) {
-        const double denom = 1.0 / sum;
-        const double v = vb * denom, w = vc * denom;
-        for (int d = 0; d < 3; ++d) out[d] = a[d] + ab[d] * v + ac[d] * w;
-        if (isfinite(out[0]) && isfinite(out[1]) && isfinite(out[2])) return;
-    }
+__device__ __noinline__ void tri_closest_degenerate(const double* p, const double* a, const double* b, const double* c, double* out) {
     double q[3], best = DBL_MAX;
     const double* E[3][2] = {{a, b}, {b, c}, {c, a}};
     for (int s = 0; s < 3; ++s) {
@@ -122,6 +81,50 @@ __device__ void tri_closest(const double* p, const double* a, const double* b, c
         const double d2q = dot3(dd, dd);
         if (d2q < best) { best = d2q; out[0] = q[0]; out[1] = q[1]; out[2] = q[2]; }
     }
+}
+
+// The regions (vertex a, b, edge ab, vertex c, edges ac, bc, interior, tested in that order)
+// select what one division and one sum are made of, so that lanes in different regions run
+// the same instructions; every lane's operations are its region's own.
+__device__ __forceinline__ void tri_closest(const double* p, const double* a, const double* b, const double* c, double* out) {
+    double ab[3], ac[3], ap[3], bp[3], cp[3];
+    for (int d = 0; d < 3; ++d) {
+        ab[d] = b[d] - a[d]; ac[d] = c[d] - a[d];
+        ap[d] = p[d] - a[d]; bp[d] = p[d] - b[d]; cp[d] = p[d] - c[d];
+    }
+    const double d1 = dot3(ab, ap), d2 = dot3(ac, ap), d3 = dot3(ab, bp), d4 = dot3(ac, bp), d5 = dot3(ab, cp), d6 = dot3(ac, cp);
+    const double vc = d1 * d4 - d3 * d2, vb = d5 * d2 - d1 * d6, va = d3 * d6 - d5 * d4;
+    const bool at_a = d1 <= 0.0 && d2 <= 0.0;
+    const bool at_b = !at_a && d3 >= 0.0 && d4 <= d3;
+    bool rest = !at_a && !at_b;
+    const bool on_ab = rest && vc <= 0.0 && d1 >= 0.0 && d3 <= 0.0;
+    rest = rest && !on_ab;
+    const bool at_c = rest && d6 >= 0.0 && d5 <= d6;
+    rest = rest && !at_c;
+    const bool on_ac = rest && vb <= 0.0 && d2 >= 0.0 && d6 <= 0.0;
+    rest = rest && !on_ac;
+    const double e = d4 - d3, f = d5 - d6;
+    const bool on_bc = rest && va <= 0.0 && e >= 0.0 && f >= 0.0;
+    rest = rest && !on_bc;
+    const double sum = va + vb + vc;
+    double num = 1.0, den = 1.0;
+    if (on_ab) { num = d1; den = d1 - d3; }
+    if (on_ac) { num = d2; den = d2 - d6; }
+    if (on_bc) { num = e; den = e + f; }
+    if (rest) den = sum;
+    const double ratio = num / den;
+    const double first = rest ? vb * ratio : ratio, second = vc * ratio;
+    const bool corner = at_a || at_b || at_c;
+    for (int d = 0; d < 3; ++d) {
+        const double from = at_b || on_bc ? b[d] : at_c ? c[d] : a[d];
+        const double along = on_ac ? ac[d] : on_bc ? c[d] - b[d] : ab[d];
+        double x = from;
+        if (!corner) x = from + first * along;
+        if (rest) x = x + ac[d] * second;
+        out[d] = x;
+    }
+    if (rest && !(sum != 0.0 && isfinite(sum) && isfinite(out[0]) && isfinite(out[1]) && isfinite(out[2])))
+        tri_closest_degenerate(p, a, b, c, out);
 }
 
 // compute_barycentric_coords (vertex_refinement.cpp:36-66).
@@ -192,8 +195,9 @@ __device__ __forceinline__ unsigned long long splitmix64(unsigned long long x) {
 
 }  // namespace
 
-// Cells with at least this many spheres run their inner loop on a warp (a chunk per lane).
-constexpr unsigned int kWarpCellSpheres = 8;
+// Lanes that work on one cell's inner loop, by its number of spheres (below kTeamSpheres[i]).
+constexpr int kTeamLanes[3] = {8, 16, 256};
+constexpr unsigned int kTeamSpheres[2] = {16, 128};
 
 // ---- setup -------------------------------------------------------------------------------
 
@@ -381,7 +385,7 @@ __global__ void k_bvh_keys(OursParams P) {
 }
 
 // Radix tree over the sorted keys (Karras, "Maximizing parallelism in the construction of
-// BVHs, octrees, and k-d trees", HPG 2012). Children < 0 are leaves (~leaf).
+// BVHs, octrees, and k-d trees", HPG 2012).
 __device__ __forceinline__ int key_delta(const unsigned long long* k, long long n, long long a, long long b) {
     if (b < 0 || b >= n) return -1;
     return __clzll(k[a] ^ k[b]);
@@ -408,134 +412,241 @@ __global__ void __launch_bounds__(128) k_bvh_tree(OursParams P) {
         }
         const long long gamma = i + s * d + (d < 0 ? -1 : 0);
         const long long lo = i < j ? i : j, hi = i < j ? j : i;
-        const int left = lo == gamma ? ~(int)gamma : (int)gamma;
-        const int right = hi == gamma + 1 ? ~(int)(gamma + 1) : (int)(gamma + 1);
-        P.child[i] = make_int2(left, right);
-        if (left < 0) P.parent[n - 1 + ~left] = (int)i; else P.parent[left] = (int)i;
-        if (right < 0) P.parent[n - 1 + ~right] = (int)i; else P.parent[right] = (int)i;
+        const bool leaf_l = lo == gamma, leaf_r = hi == gamma + 1;
+        P.nodes[i].child[0] = leaf_l ? ~(int)(K[gamma] & 0xffffffffull) : (int)gamma;
+        P.nodes[i].child[1] = leaf_r ? ~(int)(K[gamma + 1] & 0xffffffffull) : (int)(gamma + 1);
+        P.parent[leaf_l ? n - 1 + gamma : gamma] = (int)i << 1;
+        P.parent[leaf_r ? n + gamma : gamma + 1] = (int)i << 1 | 1;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) P.parent[0] = -1;
 }
 
-// Boxes bottom-up: leaf boxes rounded outward to float; the second child to arrive at a node
-// writes the union.
+// Boxes bottom-up: leaf boxes rounded outward to float, every box stored at its parent; the
+// second child to arrive at a node carries the union on.
 __global__ void __launch_bounds__(128) k_bvh_boxes(OursParams P) {
     const long long n = P.nt;
     for (long long L = (long long)blockIdx.x * blockDim.x + threadIdx.x; L < n; L += (long long)gridDim.x * blockDim.x) {
         const long long t = (long long)(P.mkeys_sorted[L] & 0xffffffffull);
-        float lo[3], hi[3];
+        float box[6];
         for (int d = 0; d < 3; ++d) {
             double a = P.tri9[9 * t + d], b = P.tri9[9 * t + 3 + d], c = P.tri9[9 * t + 6 + d];
-            lo[d] = __double2float_rd(fmin(a, fmin(b, c)));
-            hi[d] = __double2float_ru(fmax(a, fmax(b, c)));
+            box[d] = __double2float_rd(fmin(a, fmin(b, c)));
+            box[3 + d] = __double2float_ru(fmax(a, fmax(b, c)));
         }
-        const long long node_l = n - 1 + L;
-        P.bmin[node_l] = make_float4(lo[0], lo[1], lo[2], 0.f);
-        P.bmax[node_l] = make_float4(hi[0], hi[1], hi[2], 0.f);
-        __threadfence();
-        int node = P.parent[node_l];
-        while (node >= 0) {
+        int up = P.parent[n - 1 + L];
+        while (up >= 0) {
+            const int node = up >> 1;
+            float2* const dst = reinterpret_cast<float2*>(P.nodes[node].box[up & 1]);
+            for (int d = 0; d < 3; ++d) dst[d] = make_float2(box[2 * d], box[2 * d + 1]);
+            __threadfence();
             if (atomicAdd(P.flags + node, 1u) == 0) break;       // the other child is not done yet
             __threadfence();
-            const int2 ch = P.child[node];
-            const long long a = ch.x < 0 ? n - 1 + ~ch.x : ch.x, b = ch.y < 0 ? n - 1 + ~ch.y : ch.y;
-            const float4 amin = __ldcg(P.bmin + a), amax = __ldcg(P.bmax + a);
-            const float4 bmn = __ldcg(P.bmin + b), bmx = __ldcg(P.bmax + b);
-            P.bmin[node] = make_float4(fminf(amin.x, bmn.x), fminf(amin.y, bmn.y), fminf(amin.z, bmn.z), 0.f);
-            P.bmax[node] = make_float4(fmaxf(amax.x, bmx.x), fmaxf(amax.y, bmx.y), fmaxf(amax.z, bmx.z), 0.f);
-            __threadfence();
-            node = P.parent[node];
+            const float2* const other = reinterpret_cast<const float2*>(P.nodes[node].box[1 - (up & 1)]);
+            float2 o[3];
+            for (int d = 0; d < 3; ++d) o[d] = __ldcg(other + d);
+            const float ob[6] = {o[0].x, o[0].y, o[1].x, o[1].y, o[2].x, o[2].y};
+            for (int d = 0; d < 3; ++d) { box[d] = fminf(box[d], ob[d]); box[3 + d] = fmaxf(box[3 + d], ob[3 + d]); }
+            up = P.parent[node];
         }
     }
 }
 
-__device__ __forceinline__ double box_d2(const OursParams& P, long long node, const double* p) {
-    const float4 a = __ldg(P.bmin + node), b = __ldg(P.bmax + node);
-    const double lo[3] = {a.x, a.y, a.z}, hi[3] = {b.x, b.y, b.z};
-    double s = 0.0;
-    for (int d = 0; d < 3; ++d) {
-        const double e = p[d] < lo[d] ? lo[d] - p[d] : (p[d] > hi[d] ? p[d] - hi[d] : 0.0);
-        s += e * e;
-    }
-    return s;
+// A query point in double and, rounded both ways, in float.
+struct QueryPoint {
+    double p[3];
+    float lo[3], hi[3];
+};
+
+// Lower bound of the squared distance to a box, every operation rounded down: searches skip
+// only what is provably farther than the best so far, so the answer is that of exact bounds.
+__device__ __forceinline__ float box_below(const QueryPoint& q, const float* box) {
+    float e[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) e[d] = fmaxf(fmaxf(__fsub_rd(box[d], q.hi[d]), __fsub_rd(q.lo[d], box[3 + d])), 0.f);
+    return __fmaf_rd(e[0], e[0], __fmaf_rd(e[1], e[1], __fmul_rd(e[2], e[2])));
 }
 
-// Closest point of the mesh to p (point_mesh_squared_distance, contouring.cpp:869): among
+// Closest point of the mesh to a query (point_mesh_squared_distance, contouring.cpp:869): among
 // equally close triangles the one of smallest index, so the answer does not depend on the
 // traversal order (nodes as close as the best so far are still visited).
-// seed: a triangle to test first (the previous outer iteration's answer for this point), or -1;
-// the answer does not depend on it, only the number of nodes visited does.
-__device__ double bvh_closest(const OursParams& P, const double* p, double* best_c, long long seed, int& out_t) {
-    const long long n = P.nt;
-    double best = DBL_MAX;
-    long long best_t = 0x7fffffffffffffffLL;
-    auto test = [&](long long t) {
-        const double* T = P.tri9 + 9 * t;
-        double q[3];
-        tri_closest(p, T, T + 3, T + 6, q);
-        double dd[3] = {q[0] - p[0], q[1] - p[1], q[2] - p[2]};
-        const double d2 = dot3(dd, dd);
-        if (d2 < best || (d2 == best && t < best_t)) {
-            best = d2; best_t = t;
-            best_c[0] = q[0]; best_c[1] = q[1]; best_c[2] = q[2];
-        }
-    };
-    auto leaf = [&](long long L) { test((long long)(P.mkeys_sorted[L] & 0xffffffffull)); };
-    if (seed >= 0 && seed < n) test(seed);
-    if (n == 1) { leaf(0); out_t = (int)best_t; return best; }
-    int stack[96];
-    int sp = 0;
-    stack[sp++] = 0;
-    while (sp > 0) {
-        const int node = stack[--sp];
-        const int2 ch = P.child[node];
-        const int c2[2] = {ch.x, ch.y};
-        double dc[2];
-        for (int u = 0; u < 2; ++u) dc[u] = box_d2(P, c2[u] < 0 ? n - 1 + ~c2[u] : c2[u], p);
-        const int first = dc[1] < dc[0] ? 1 : 0;
-        // leaves now, internal nodes onto the stack (the nearer one on top)
-        for (int u = 0; u < 2; ++u) {
-            const int w = u == 0 ? first : 1 - first;
-            if (c2[w] < 0 && dc[w] <= best) leaf(~c2[w]);
-        }
-        for (int u = 1; u >= 0; --u) {
-            const int w = u == 0 ? first : 1 - first;
-            if (c2[w] >= 0 && dc[w] <= best) {
-                if (sp < 96) stack[sp++] = c2[w];
-                else set_error(P.err, kErrOverflow);
-            }
-        }
+struct Closest {
+    double d2 = DBL_MAX;
+    int t = 0x7fffffff;
+    float above = FLT_MAX;              // d2 rounded up
+    double c[3] = {0.0, 0.0, 0.0};
+};
+
+// One copy of the distance for all callers (instruction cache).
+__device__ __noinline__ double tri_distance(const double* p, const double* T, double* c) {
+    tri_closest(p, T, T + 3, T + 6, c);
+    double dd[3] = {c[0] - p[0], c[1] - p[1], c[2] - p[2]};
+    return dot3(dd, dd);
+}
+
+__device__ __forceinline__ void closest_test(const OursParams& P, const QueryPoint& q, int t, Closest& best) {
+    double c[3];
+    const double d2 = tri_distance(q.p, P.tri9 + 9 * (size_t)t, c);
+    if (d2 < best.d2 || (d2 == best.d2 && t < best.t)) {
+        best.d2 = d2;
+        best.t = t;
+        best.above = __double2float_ru(d2);
+        best.c[0] = c[0]; best.c[1] = c[1]; best.c[2] = c[2];
     }
-    out_t = (int)best_t;
-    return best;
+}
+
+__device__ __forceinline__ void load_node(const OursParams& P, int node, float (&box)[2][6], int (&child)[2]) {
+    const float4* const src = reinterpret_cast<const float4*>(P.nodes + node);
+    const float4 a = __ldg(src), b = __ldg(src + 1), c = __ldg(src + 2), d = __ldg(src + 3);
+    box[0][0] = a.x; box[0][1] = a.y; box[0][2] = a.z; box[0][3] = a.w; box[0][4] = b.x; box[0][5] = b.y;
+    box[1][0] = b.z; box[1][1] = b.w; box[1][2] = c.x; box[1][3] = c.y; box[1][4] = c.z; box[1][5] = c.w;
+    child[0] = __float_as_int(d.x);
+    child[1] = __float_as_int(d.y);
 }
 
 // ---- sphere assignment ---------------------------------------------------------------------
 
+// The query of selected point s, without its answer.
+__device__ __forceinline__ QueryPoint query_point(const OursParams& P, long long s) {
+    QueryPoint q;
+    point_of(P.g, P.sel[s], q.p);
+    for (int d = 0; d < 3; ++d) { q.lo[d] = __double2float_rd(q.p[d]); q.hi[d] = __double2float_ru(q.p[d]); }
+    return q;
+}
+
+// The sphere about selected point s to the active cell that holds its closest mesh point.
+__device__ __forceinline__ void assign_sphere(const OursParams& P, long long s, const Closest& best) {
+    const long long gidx = P.sel[s];
+    P.prev_tri[gidx] = best.t;
+    const double radius = fabs((double)__ldg(P.g.v + gidx));
+    int rank = -1;
+    if (best.d2 < DBL_MAX && sqrt(best.d2) - radius < P.cell_diag) {
+        int ci[3];
+        const int cmax[3] = {P.g.nx - 2, P.g.ny - 2, P.g.nz - 2};
+        for (int d = 0; d < 3; ++d) {
+            const double f = floor((best.c[d] - P.gmin[d]) / P.gd[d]);
+            int v = f < -1e9 ? -1000000000 : (f > 1e9 ? 1000000000 : (int)f);
+            ci[d] = max(0, min(v, cmax[d]));
+        }
+        if (active_bit(P, ci[0], ci[1], ci[2])) {
+            rank = (int)cell_rank(P.bits, P.super, P.g, ci[0], ci[1], ci[2]);
+            atomicAdd(P.cell_count + rank, 1u);
+        }
+    }
+    P.sel_cell[s] = rank;
+}
+
+// A thread per query, depth first, the near child first; the search starts with the point's
+// answer of the previous outer iteration. A search of more than kQueryBudget nodes is left to
+// k_ours_query_long (with the best triangle so far): the mean is 80 nodes, but a point far
+// from the mesh visits thousands, and one such thread kept the launch (128^3 perturbed sphere,
+// 200,000 points: 6.9 ms at 4.5% issue, 1.1 with both kernels; with a budget of 96 nodes 1.2,
+// of 320 1.4, of 640 1.9).
+constexpr int kQueryBudget = 160;
 __global__ void __launch_bounds__(128) k_ours_query(OursParams P) {
     for (long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x; s < P.nsel; s += (long long)gridDim.x * blockDim.x) {
-        const long long gidx = P.sel[s];
-        double c[3], C[3];
-        point_of(P.g, gidx, c);
-        int t = -1;
-        const double d2 = bvh_closest(P, c, C, P.prev_tri[gidx], t);
-        P.prev_tri[gidx] = t;
-        const double radius = fabs((double)__ldg(P.g.v + gidx));
-        int rank = -1;
-        if (d2 < DBL_MAX && sqrt(d2) - radius < P.cell_diag) {
-            int ci[3];
-            const int cmax[3] = {P.g.nx - 2, P.g.ny - 2, P.g.nz - 2};
-            for (int d = 0; d < 3; ++d) {
-                const double f = floor((C[d] - P.gmin[d]) / P.gd[d]);
-                int v = f < -1e9 ? -1000000000 : (f > 1e9 ? 1000000000 : (int)f);
-                ci[d] = max(0, min(v, cmax[d]));
+        const QueryPoint q = query_point(P, s);
+        const int seed = P.prev_tri[P.sel[s]];
+        Closest best;
+        if (seed >= 0 && seed < P.nt) closest_test(P, q, seed, best);
+        int stack[96], sp = 0;                   // a tree over unique 62-bit keys is at most 62 deep
+        float bound[96];
+        if (P.nt == 1) closest_test(P, q, 0, best);
+        else { stack[sp] = 0; bound[sp++] = 0.f; }
+        for (int visits = 0; sp > 0 && visits < kQueryBudget;) {
+            --sp;
+            if (bound[sp] > best.above) continue;
+            ++visits;
+            float box[2][6];
+            int child[2];
+            load_node(P, stack[sp], box, child);
+            const float d0 = box_below(q, box[0]), d1 = box_below(q, box[1]);
+            const bool swap = d1 < d0;
+            const int near = swap ? child[1] : child[0], far = swap ? child[0] : child[1];
+            const float dn = swap ? d1 : d0, df = swap ? d0 : d1;
+            // leaves now, internal nodes onto the stack (the nearer one on top)
+            for (int w = 0; w < 2; ++w) {
+                const int c = w == 0 ? near : far;
+                if (c < 0 && (w == 0 ? dn : df) <= best.above) closest_test(P, q, ~c, best);
             }
-            if (active_bit(P, ci[0], ci[1], ci[2])) {
-                rank = (int)cell_rank(P.bits, P.super, P.g, ci[0], ci[1], ci[2]);
-                atomicAdd(P.cell_count + rank, 1u);
+            if (far >= 0 && df <= best.above) { stack[sp] = far; bound[sp++] = df; }
+            if (near >= 0 && dn <= best.above) { stack[sp] = near; bound[sp++] = dn; }
+            if (sp > 94) { set_error(P.err, kErrOverflow); sp = 0; }
+        }
+        if (sp > 0) {
+            P.prev_tri[P.sel[s]] = best.t < P.nt ? best.t : -1;
+            P.long_query[atomicAdd(P.long_count, 1u)] = (uint32_t)s;
+        } else {
+            assign_sphere(P, s, best);
+        }
+    }
+}
+
+// The long searches, a warp each: the lanes take the top nodes of one stack. 32 at a time push
+// at most 64; near the stack's end one node at a time (depth first) adds at most the tree's
+// depth.
+constexpr int kLongStack = 768, kLongWarps = 4;
+__global__ void __launch_bounds__(32 * kLongWarps) k_ours_query_long(OursParams P) {
+    __shared__ int s_node[kLongWarps][kLongStack];
+    __shared__ float s_bound[kLongWarps][kLongStack];
+    const int lane = threadIdx.x & 31;
+    int* const node = s_node[threadIdx.x >> 5];
+    float* const bound = s_bound[threadIdx.x >> 5];
+    const unsigned int n = *P.long_count;
+    for (unsigned int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < n; w += (gridDim.x * blockDim.x) >> 5) {
+        const long long s = P.long_query[w];
+        const QueryPoint q = query_point(P, s);
+        const int seed = P.prev_tri[P.sel[s]];
+        Closest best;
+        if (seed >= 0) closest_test(P, q, seed, best);
+        __syncwarp();
+        if (lane == 0) { node[0] = 0; bound[0] = 0.f; }
+        int sp = 1;
+        while (sp > 0) {
+            __syncwarp();
+            const int take = kLongStack - sp >= 192 ? min(sp, 32) : 1;
+            const int at = sp - 1 - lane;
+            const bool mine = lane < take && bound[at] <= best.above;
+            int child[2] = {-1, -1};
+            float d[2] = {0.f, 0.f};
+            bool push[2] = {false, false};
+            const double had = best.d2;
+            const int had_t = best.t;
+            if (mine) {
+                float box[2][6];
+                load_node(P, node[at], box, child);
+                d[0] = box_below(q, box[0]);
+                d[1] = box_below(q, box[1]);
+                for (int c = 0; c < 2; ++c) {
+                    if (child[c] >= 0) push[c] = true;
+                    else if (d[c] <= best.above) closest_test(P, q, ~child[c], best);
+                }
+            }
+            __syncwarp();
+            // the lanes' best (ties: smallest index)
+            if (__any_sync(0xffffffffu, best.d2 < had || best.t != had_t)) {
+                for (int o = 16; o > 0; o >>= 1) {
+                    const double od = __shfl_xor_sync(0xffffffffu, best.d2, o);
+                    const int ot = __shfl_xor_sync(0xffffffffu, best.t, o);
+                    if (od < best.d2 || (od == best.d2 && ot < best.t)) { best.d2 = od; best.t = ot; }
+                }
+                best.above = best.d2 < DBL_MAX ? __double2float_ru(best.d2) : FLT_MAX;
+            }
+            sp -= take;
+            for (int c = 0; c < 2; ++c) {
+                const bool on = push[c] && d[c] <= best.above;
+                const unsigned int votes = __ballot_sync(0xffffffffu, on);
+                if (on) {
+                    const int to = sp + __popc(votes & ((1u << lane) - 1u));
+                    node[to] = child[c];
+                    bound[to] = d[c];
+                }
+                sp += __popc(votes);
             }
         }
-        P.sel_cell[s] = rank;
+        if (lane == 0) {
+            if (best.t < P.nt) tri_distance(q.p, P.tri9 + 9 * (size_t)best.t, best.c);
+            assign_sphere(P, s, best);
+        }
     }
 }
 
@@ -548,12 +659,15 @@ __global__ void __launch_bounds__(128) k_ours_scatter(OursParams P) {
     }
 }
 
-// Each cell's spheres by radius (then grid index, for a deterministic order among equal radii).
+// Each cell's spheres by radius (then grid index, for a deterministic order among equal radii),
+// and their centres (float grid positions) with the values there.
 __global__ void __launch_bounds__(128) k_ours_sort(OursParams P) {
     for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < P.nv; r += (long long)gridDim.x * blockDim.x) {
         const unsigned int n = P.cell_count[r];
-        if (n >= kWarpCellSpheres) P.heavy[atomicAdd(P.heavy_count, 1u)] = (uint32_t)r;
-        if (n < 2) continue;
+        if (n) {
+            const int team = n < kTeamSpheres[0] ? 0 : n < kTeamSpheres[1] ? 1 : 2;
+            P.team_list[team][atomicAdd(P.team_count + team, 1u)] = (uint32_t)r;
+        }
         uint32_t* a = P.cell_spheres + P.cell_start[r];
         auto less = [&](uint32_t x, uint32_t y) {
             const float rx = fabsf(__ldg(P.g.v + x)), ry = fabsf(__ldg(P.g.v + y));
@@ -569,6 +683,11 @@ __global__ void __launch_bounds__(128) k_ours_sort(OursParams P) {
                 while (y >= gap && less(t, a[y - gap])) { a[y] = a[y - gap]; y -= gap; }
                 a[y] = t;
             }
+        }
+        for (unsigned int x = 0; x < n; ++x) {
+            double c[3];
+            point_of(P.g, a[x], c);
+            P.cell_centres[P.cell_start[r] + x] = make_float4((float)c[0], (float)c[1], (float)c[2], __ldg(P.g.v + a[x]));
         }
     }
 }
@@ -691,28 +810,37 @@ __global__ void __launch_bounds__(128) k_ours_hermite(OursParams P) {
     }
 }
 
+// What the team of one cell works on.
+struct TeamCell {
+    double hp[12][3], fi[6][3];
+    double prev[3];                  // the vertex this iteration starts from
+    double h0[9], cen[3], sums[9];
+    unsigned char fan[24];           // edge | face << 4
+};
+
 // One sphere's row of Cell::minimize_qef (Cell.cpp:400-446) for a cell whose vertex is prev:
 // its closest point on the local fan (first minimum in fan order), the point on the sphere,
 // the barycentric blend of (vertex, Hermite point, face point). False if the row is skipped.
-__device__ bool sphere_row(const OursParams& P, const OursCell& S, const int* fan, int nfan, const double* prev,
-                           uint32_t gidx, double ssw, double row[3], double& rb) {
-    double c[3];
-    point_of(P.g, gidx, c);
-    const double sval = (double)__ldg(P.g.v + gidx);
+// row: three entries and the right-hand side. One copy for all callers (instruction cache).
+__device__ __noinline__ bool sphere_row(const TeamCell& C, int nfan, const float4* sphere, double ssw, double* row) {
+    const double prev[3] = {C.prev[0], C.prev[1], C.prev[2]};
+    const float4 centre = __ldg(sphere);
+    const double c[3] = {(double)centre.x, (double)centre.y, (double)centre.z};
+    const double sval = (double)centre.w;
     const double rs = fabs(sval);
     double best = DBL_MAX, tm[3] = {0, 0, 0};
     int bf = 0;
     for (int f = 0; f < nfan; ++f) {
-        const int e = fan[f] & 15, d = fan[f] >> 4;
+        const int e = C.fan[f] & 15, d = C.fan[f] >> 4;
         double q[3];
-        tri_closest(c, prev, S.hp[e], S.fi[d], q);
+        tri_closest(c, prev, C.hp[e], C.fi[d], q);
         double dd[3] = {q[0] - c[0], q[1] - c[1], q[2] - c[2]};
         const double d2 = dot3(dd, dd);
         if (d2 < best) { best = d2; bf = f; tm[0] = q[0]; tm[1] = q[1]; tm[2] = q[2]; }
     }
-    const int e = fan[bf] & 15, d = fan[bf] >> 4;
-    const double* Hp = S.hp[e];
-    const double* Fp = S.fi[d];
+    const int e = C.fan[bf] & 15, d = C.fan[bf] >> 4;
+    const double* Hp = C.hp[e];
+    const double* Fp = C.fi[d];
     double ct[3];
     for (int a = 0; a < 3; ++a) ct[a] = tm[a] - c[a];
     const double rho0 = norm3(ct);
@@ -736,40 +864,12 @@ __device__ bool sphere_row(const OursParams& P, const OursCell& S, const int* fa
     double dv[3];
     for (int a = 0; a < 3; ++a) dv[a] = q[a] - c[a];
     for (int a = 0; a < 3; ++a) row[a] = alpha * ssw * dv[a];
-    rb = ssw * ((dot3(q, dv) - beta * dot3(Hp, dv)) - gamma * dot3(Fp, dv));
+    row[3] = ssw * ((dot3(q, dv) - beta * dot3(Hp, dv)) - gamma * dot3(Fp, dv));
     return true;
 }
 
-// Sphere rows of one chunk, summed in order from zero: 6 entries of the symmetric A^T A
-// (00 01 02 11 12 22) and 3 of A^T b.
-__device__ void chunk_sums(const OursParams& P, const OursCell& S, const int* fan, int nfan, const double* prev,
-                           const uint32_t* sph, unsigned int lo, unsigned int hi, double ssw, double acc[9]) {
-    for (int q = 0; q < 9; ++q) acc[q] = 0.0;
-    for (unsigned int s = lo; s < hi; ++s) {
-        double row[3], rb;
-        if (!sphere_row(P, S, fan, nfan, prev, sph[s], ssw, row, rb)) continue;
-        acc[0] += row[0] * row[0]; acc[1] += row[0] * row[1]; acc[2] += row[0] * row[2];
-        acc[3] += row[1] * row[1]; acc[4] += row[1] * row[2]; acc[5] += row[2] * row[2];
-        acc[6] += row[0] * rb; acc[7] += row[1] * rb; acc[8] += row[2] * rb;
-    }
-}
-
-// The local fan of a cell: (vertex, Hermite point on edge e, face point d) for each face d
-// with a point and each of its four edges with a Hermite point, in face then edge order.
-__device__ int cell_fan(const OursCell& S, int fan[24]) {
-    int nfan = 0;
-    for (int d = 0; d < 6; ++d) {
-        if (!(S.fmask & (1 << d))) continue;
-        for (int u = 0; u < 4; ++u) {
-            const int e = edge_of_corners(kFaceCorners[d][u], kFaceCorners[d][(u + 1) & 3]);
-            if (e >= 0 && (S.hmask & (1 << e))) fan[nfan++] = e | (d << 4);
-        }
-    }
-    return nfan;
-}
-
 // The Hermite rows dc_weight * n_e in edge order and the Hermite centroid.
-__device__ void hermite_rows(const OursParams& P, const OursCell& S, double H0[9], double cen[3]) {
+__device__ void hermite_rows(const OursParams& P, const OursCell& S, double* H0, double* cen) {
     for (int q = 0; q < 9; ++q) H0[q] = 0.0;
     cen[0] = cen[1] = cen[2] = 0.0;
     int m = 0;
@@ -808,78 +908,201 @@ __device__ void inner_solve(const OursParams& P, const double Acc[9], const doub
     }
 }
 
-// The inner loop of one cell (contouring.cpp:1288-1309): refine_vertex_from_face_intersections
+// The inner loop of the cells (contouring.cpp:1288-1309): refine_vertex_from_face_intersections
 // (vertex_refinement.cpp:201-280) + Cell::minimize_qef (Cell.cpp:364-473) until the vertex
-// moves less than 1e-6. The sphere rows are summed in 32 chunks of consecutive spheres, each
-// from zero, added in chunk order: the same sums whether a thread or a warp computes them.
-__global__ void __launch_bounds__(128) k_ours_inner(OursParams P) {
-    for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < P.nv; r += (long long)gridDim.x * blockDim.x) {
-        OursCell& S = P.cells[r];
-        const unsigned int nsph = P.cell_count[r];
-        if (!S.fmask || !nsph || !S.hmask || nsph >= kWarpCellSpheres) continue;
-        int fan[24];
-        const int nfan = cell_fan(S, fan);
-        if (!nfan) continue;
-        const uint32_t* sph = P.cell_spheres + P.cell_start[r];
-        double H0[9], cen[3];
-        hermite_rows(P, S, H0, cen);
-        const double ssw = sqrt(P.sphere_weight), smu = sqrt(P.mu);
-        const unsigned int cs = (nsph + 31) / 32;
-        double v[3] = {S.v[0], S.v[1], S.v[2]};
-        for (int it = 0; it < P.inner_iters; ++it) {
-            const double prev[3] = {v[0], v[1], v[2]};
-            double Acc[9];
-            for (int q = 0; q < 9; ++q) Acc[q] = H0[q];
-            for (unsigned int l = 0; l < 32; ++l) {
-                const unsigned int lo = l * cs, hi = min(nsph, lo + cs);
-                if (lo >= hi) break;
-                double part[9];
-                chunk_sums(P, S, fan, nfan, prev, sph, lo, hi, ssw, part);
-                for (int q = 0; q < 9; ++q) Acc[q] += part[q];
-            }
-            inner_solve(P, Acc, prev, cen, smu, v);
-            double dm[3] = {v[0] - prev[0], v[1] - prev[1], v[2] - prev[2]};
-            if (norm3(dm) < 1e-6) break;
+// moves less than 1e-6. A sphere's row is skipped or adds to the 6 entries of the symmetric
+// A^T A (00 01 02 11 12 22) and the 3 of A^T b; rows are summed in 32 chunks of consecutive
+// spheres, each from zero, added in chunk order: the same sums for every team size.
+//
+// A team of T lanes per cell, cells from a counter: each lane forms rows of the team's next T
+// spheres (the distances to the local fan, most of the work), then the nine sums are
+// spread over the lanes, then every lane solves. Cells differ a hundredfold in work (1 to
+// 1,600 spheres, 2 to 100 iterations): with a thread per cell below 8 spheres and a warp above,
+// 3 and 18 lanes were active and the longest cells kept the launch. An outer iteration on a
+// 128^3 perturbed sphere: 12.4 ms before, 4.7 now; 72^3 (cells of up to 1,600 spheres) 20.1 and
+// 6.8. Eight lanes for the short cells because their 100 iterations are a chain (4 lanes: 5.3,
+// 16: 4.8). Bound: FP64 instructions (45% of the pipe) and the chain of the solve's divisions.
+// Loads cell r; how many triangles its local fan has: (vertex, Hermite point on edge e, face
+// point d) for each face d with a point and each of its four edges with a Hermite point, in
+// face then edge order. 0: nothing to do. By the T lanes of a team; a team synchronisation has
+// to follow.
+template <int T>
+__device__ int team_load(const OursParams& P, const OursCell& S, TeamCell& C, int tl) {
+    const int hmask = S.hmask, fmask = S.fmask;
+    int nfan = 0;
+    for (int x = 0; x < 24; ++x) {
+        const int d = x >> 2, e = kFaceEdges[d][x & 3];
+        if ((fmask & (1 << d)) && (hmask & (1 << e))) {
+            if (tl == 0) C.fan[nfan] = (unsigned char)(e | d << 4);
+            ++nfan;
         }
-        for (int a = 0; a < 3; ++a) S.v[a] = v[a];
+    }
+    if (!nfan) return 0;
+    for (int x = tl; x < 36; x += T) (&C.hp[0][0])[x] = (&S.hp[0][0])[x];
+    for (int x = tl; x < 18; x += T) (&C.fi[0][0])[x] = (&S.fi[0][0])[x];
+    if (tl == 0) hermite_rows(P, S, C.h0, C.cen);
+    return nfan;
+}
+
+// Factors of the nine sums: row entries 0..2, 3 the right-hand side.
+__device__ __forceinline__ int sum_left(int q) { return q < 3 ? 0 : q < 5 ? 1 : q == 5 ? 2 : q - 6; }
+__device__ __forceinline__ int sum_right(int q) { return q < 3 ? q : q < 5 ? q - 2 : q == 5 ? 2 : 3; }
+
+constexpr int kInnerThreads = 256;
+struct InnerShared {
+    TeamCell cell[kInnerThreads / kTeamLanes[0]];
+    double row[kInnerThreads][4];
+    unsigned char ok[kInnerThreads];
+    double part[32][9];
+    unsigned int next;
+};
+
+template <int T>
+__device__ void inner_teams(const OursParams& P, InnerShared& S, int team) {
+    constexpr int kSums = (9 + T - 1) / T;
+    static_assert(T >= 3 && T <= 16, "three lanes hand on the vertex; a team lies within a warp");
+    const int tl = threadIdx.x % T, tm = threadIdx.x / T;
+    const unsigned int lanes = ((1u << T) - 1u) << (threadIdx.x & 31 & ~(T - 1));
+    TeamCell& C = S.cell[tm];
+    double (*const rows)[4] = S.row + tm * T;
+    const unsigned char* const oks = S.ok + tm * T;
+    const unsigned int ncells = P.team_count[team];
+    const double ssw = sqrt(P.sphere_weight), smu = sqrt(P.mu);
+    bool active = false, more = true;
+    long long r = 0;
+    unsigned int nsph = 0, cs = 1;
+    int nfan = 0, it = 0;
+    const float4* sph = nullptr;
+    double v[3] = {0.0, 0.0, 0.0};
+    for (;;) {
+        if (!active && more) {
+            unsigned int w = 0;
+            if (tl == 0) w = atomicAdd(P.team_count + 3 + team, 1u);
+            w = __shfl_sync(lanes, w, 0, T);
+            more = w < ncells;
+            if (more) {
+                r = P.team_list[team][w];
+                const OursCell& cell = P.cells[r];
+                nfan = team_load<T>(P, cell, C, tl);
+                active = nfan > 0;
+                nsph = P.cell_count[r];
+                cs = (nsph + 31) / 32;
+                sph = P.cell_centres + P.cell_start[r];
+                for (int a = 0; a < 3; ++a) v[a] = cell.v[a];
+                it = 0;
+            }
+        }
+        __syncwarp();
+        if (!__any_sync(0xffffffffu, active || more)) break;
+        const double prev[3] = {v[0], v[1], v[2]};
+        if (tl < 3) C.prev[tl] = tl == 0 ? v[0] : tl == 1 ? v[1] : v[2];
+        __syncwarp();
+        double sum[kSums], part[kSums];
+        for (int q = 0; q < kSums; ++q) { sum[q] = active && tl + q * T < 9 ? C.h0[tl + q * T] : 0.0; part[q] = 0.0; }
+        const unsigned int steps = __reduce_max_sync(0xffffffffu, active ? (nsph + T - 1) / T : 0u);
+        unsigned int edge = cs;                          // first sphere of the next chunk
+        for (unsigned int k = 0; k < steps; ++k) {
+            const unsigned int s0 = k * T;
+            if (active && s0 + tl < nsph)
+                S.ok[threadIdx.x] = sphere_row(C, nfan, sph + s0 + tl, ssw, rows[tl]);
+            __syncwarp();
+            if (active && s0 < nsph) {
+                const unsigned int m = min((unsigned int)T, nsph - s0);
+                for (unsigned int j = 0; j < m; ++j) {
+                    if (s0 + j == edge) {
+                        for (int q = 0; q < kSums; ++q) { sum[q] += part[q]; part[q] = 0.0; }
+                        edge += cs;
+                    }
+                    if (!oks[j]) continue;
+                    for (int q = 0; q < kSums; ++q) {
+                        const int e = min(tl + q * T, 8);
+                        part[q] += rows[j][sum_left(e)] * rows[j][sum_right(e)];
+                    }
+                }
+            }
+            __syncwarp();
+        }
+        for (int q = 0; q < kSums; ++q)
+            if (active && tl + q * T < 9) C.sums[tl + q * T] = sum[q] + part[q];
+        __syncwarp();
+        if (active) {
+            inner_solve(P, C.sums, prev, C.cen, smu, v);
+            double dm[3] = {v[0] - prev[0], v[1] - prev[1], v[2] - prev[2]};
+            if (norm3(dm) < 1e-6 || ++it >= P.inner_iters) {
+                active = false;
+                if (tl == 0) for (int a = 0; a < 3; ++a) P.cells[r].v[a] = v[a];
+            }
+        }
+        __syncwarp();
     }
 }
 
-// The same inner loop for the cells with many spheres, a warp per cell.
-__global__ void __launch_bounds__(128) k_ours_inner_warp(OursParams P) {
-    const int lane = threadIdx.x & 31;
-    const unsigned int nheavy = *P.heavy_count;
-    for (long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < nheavy;
-         w += ((long long)gridDim.x * blockDim.x) >> 5) {
-        const long long r = P.heavy[w];
-        OursCell& S = P.cells[r];
-        const unsigned int nsph = P.cell_count[r];
-        if (!S.fmask || !S.hmask) continue;                  // warp-uniform
-        int fan[24];
-        const int nfan = cell_fan(S, fan);
+// The same with the block as one team: 8 lanes a chunk.
+__device__ void inner_block(const OursParams& P, InnerShared& S, int team) {
+    constexpr int T = kInnerThreads, kLanes = T / 32;
+    TeamCell& C = S.cell[0];
+    const int tid = threadIdx.x, chunk = tid / kLanes, sub = tid % kLanes;
+    const unsigned int ncells = P.team_count[team];
+    const double ssw = sqrt(P.sphere_weight), smu = sqrt(P.mu);
+    for (;;) {
+        __syncthreads();
+        if (tid == 0) S.next = atomicAdd(P.team_count + 3 + team, 1u);
+        __syncthreads();
+        if (S.next >= ncells) break;
+        const long long r = P.team_list[team][S.next];
+        const OursCell& cell = P.cells[r];
+        const int nfan = team_load<T>(P, cell, C, tid);
         if (!nfan) continue;
-        const uint32_t* sph = P.cell_spheres + P.cell_start[r];
-        double H0[9], cen[3];
-        hermite_rows(P, S, H0, cen);
-        const double ssw = sqrt(P.sphere_weight), smu = sqrt(P.mu);
-        const unsigned int cs = (nsph + 31) / 32;
-        const unsigned int lo = min(nsph, lane * cs), hi = min(nsph, lo + cs);
-        double v[3] = {S.v[0], S.v[1], S.v[2]};
+        const unsigned int nsph = P.cell_count[r], cs = (nsph + 31) / 32, nchunks = (nsph + cs - 1) / cs;
+        const float4* const sph = P.cell_centres + P.cell_start[r];
+        if (tid < 3) C.prev[tid] = cell.v[tid];
+        __syncthreads();
         for (int it = 0; it < P.inner_iters; ++it) {
-            const double prev[3] = {v[0], v[1], v[2]};
-            double part[9];
-            chunk_sums(P, S, fan, nfan, prev, sph, lo, hi, ssw, part);
-            double Acc[9];
-            for (int q = 0; q < 9; ++q) Acc[q] = H0[q];
-            const int nchunks = (int)((nsph + cs - 1) / cs);      // warp-uniform
-            for (int l = 0; l < nchunks; ++l)
-                for (int q = 0; q < 9; ++q) Acc[q] += __shfl_sync(0xffffffffu, part[q], l);
-            inner_solve(P, Acc, prev, cen, smu, v);
-            double dm[3] = {v[0] - prev[0], v[1] - prev[1], v[2] - prev[2]};
-            if (norm3(dm) < 1e-6) break;
+            for (int x = tid; x < 32 * 9; x += T) (&S.part[0][0])[x] = 0.0;
+            for (unsigned int k = 0; k < cs; k += kLanes) {
+                const unsigned int s = chunk * cs + k + sub;
+                S.ok[tid] = k + sub < cs && s < nsph && sphere_row(C, nfan, sph + s, ssw, S.row[tid]);
+                __syncthreads();
+                for (int x = tid; x < 32 * 9; x += T) {
+                    const int l = x / 9, e = x % 9;
+                    double part = S.part[l][e];
+                    for (int j = l * kLanes; j < (l + 1) * kLanes; ++j)
+                        if (S.ok[j]) part += S.row[j][sum_left(e)] * S.row[j][sum_right(e)];
+                    S.part[l][e] = part;
+                }
+                __syncthreads();
+            }
+            if (tid < 9) {
+                double sum = C.h0[tid];
+                for (unsigned int l = 0; l < nchunks; ++l) sum += S.part[l][tid];
+                C.sums[tid] = sum;
+            }
+            __syncthreads();
+            bool done = false;
+            if (tid < 32) {
+                const double prev[3] = {C.prev[0], C.prev[1], C.prev[2]};
+                double v[3];
+                inner_solve(P, C.sums, prev, C.cen, smu, v);
+                const double dm[3] = {v[0] - prev[0], v[1] - prev[1], v[2] - prev[2]};
+                done = norm3(dm) < 1e-6;
+                __syncwarp();
+                if (tid < 3) C.prev[tid] = tid == 0 ? v[0] : tid == 1 ? v[1] : v[2];
+            }
+            if (__syncthreads_or(done)) break;
         }
-        if (lane == 0) for (int a = 0; a < 3; ++a) S.v[a] = v[a];
+        if (tid < 3) P.cells[r].v[tid] = C.prev[tid];
     }
+}
+
+// Longest cells first; every block that fits on the GPU takes cells from the counters, so a block
+// with a long cell keeps only itself.
+__global__ void __launch_bounds__(kInnerThreads, 2) k_ours_inner(const __grid_constant__ OursParams P) {
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    InnerShared& S = *reinterpret_cast<InnerShared*>(s_raw);
+    inner_block(P, S, 2);
+    inner_teams<kTeamLanes[1]>(P, S, 1);
+    __syncthreads();
+    inner_teams<kTeamLanes[0]>(P, S, 0);
 }
 
 __global__ void k_ours_mesh(OursParams P) {
@@ -929,12 +1152,14 @@ size_t ours_workspace_bytes(long long nv, long long nq, long long npts, size_t* 
     b += 3 * al(sizeof(uint32_t) * npts) + al(sizeof(int) * npts);           // sel, band/rest, sel_cell
     b += al(sizeof(unsigned long long) * npts) * 2 + al(sizeof(uint32_t) * npts);  // fill keys/values
     b += 3 * al(sizeof(unsigned int) * (nv + 1)) + al(sizeof(uint32_t) * npts);    // count/start/fill, spheres
-    b += al(sizeof(uint32_t) * (nv + 1));                                    // cells with many spheres
+    b += al(sizeof(float4) * npts);                                          // their centres
+    b += 3 * al(sizeof(uint32_t) * (nv + 1));                                // cells by team size
+    b += al(sizeof(uint32_t) * npts);                                        // points with long searches
     b += al(sizeof(uint32_t) * npts);                                        // selected points, sorted
     b += al(sizeof(int) * npts);                                             // last closest triangle per point
-    b += al(sizeof(unsigned long long) * nt) + al(sizeof(int2) * nt) + al(sizeof(int) * 2 * nt);
+    b += al(sizeof(unsigned long long) * nt) + al(sizeof(BvhNode) * nt) + al(sizeof(int) * 2 * nt);
     b += 4 * al(sizeof(uint32_t) * nt);                                      // triangle codes / indices
-    b += 2 * al(sizeof(float4) * 2 * nt) + al(sizeof(unsigned int) * nt) + al(sizeof(double) * 9 * nt);
+    b += al(sizeof(unsigned int) * nt) + al(sizeof(double) * 9 * nt);
     b += al(sizeof(uint32_t) * (scan_partials_len(nv + 1) + 1)) + al(64);    // scan partials, counters
     b += al(*sort_bytes);
     return b + 4096;
@@ -961,16 +1186,16 @@ cudaError_t ours_run(OursRun& R, cudaStream_t s) {
     P.cell_start = (unsigned int*)take(sizeof(unsigned int) * (nv + 1));
     P.cell_fill = (unsigned int*)take(sizeof(unsigned int) * (nv + 1));
     P.cell_spheres = (uint32_t*)take(sizeof(uint32_t) * npts);
-    P.heavy = (uint32_t*)take(sizeof(uint32_t) * (nv + 1));
+    P.cell_centres = (float4*)take(sizeof(float4) * npts);
+    for (int q = 0; q < 3; ++q) P.team_list[q] = (uint32_t*)take(sizeof(uint32_t) * (nv + 1));
+    P.long_query = (uint32_t*)take(sizeof(uint32_t) * npts);
     P.mkeys_sorted = (unsigned long long*)take(sizeof(unsigned long long) * nt);
     P.tcode = (uint32_t*)take(sizeof(uint32_t) * nt);
     P.tidx = (uint32_t*)take(sizeof(uint32_t) * nt);
     P.tcode_sorted = (uint32_t*)take(sizeof(uint32_t) * nt);
     P.tidx_sorted = (uint32_t*)take(sizeof(uint32_t) * nt);
-    P.child = (int2*)take(sizeof(int2) * nt);
+    P.nodes = (BvhNode*)take(sizeof(BvhNode) * nt);
     P.parent = (int*)take(sizeof(int) * 2 * nt);
-    P.bmin = (float4*)take(sizeof(float4) * 2 * nt);
-    P.bmax = (float4*)take(sizeof(float4) * 2 * nt);
     P.flags = (unsigned int*)take(sizeof(unsigned int) * nt);
     P.tri9 = (double*)take(sizeof(double) * 9 * nt);
     uint32_t* partials = (uint32_t*)take(sizeof(uint32_t) * (scan_partials_len(nv + 1) + 1));
@@ -978,7 +1203,8 @@ cudaError_t ours_run(OursRun& R, cudaStream_t s) {
     void* sort_temp = take(R.sort_bytes);
     uint32_t* sel_sorted = (uint32_t*)take(sizeof(uint32_t) * npts);
     P.prev_tri = (int*)take(sizeof(int) * npts);
-    P.heavy_count = counters + 8;
+    P.team_count = counters + 8;
+    P.long_count = counters + 14;
     P.sel = sel_sorted;
     P.nt = nt;
     const int sms = R.num_sms;
@@ -1003,6 +1229,7 @@ cudaError_t ours_run(OursRun& R, cudaStream_t s) {
         k_ours_point_keys<<<grid_for(nband, 256, sms), 256, 0, s>>>(P, band, nband, fk);
         OURS_TRY(radix_sort_pairs(sort_temp, R.sort_bytes, fk, fk2, band, sel_sorted, nband, 0, 63, s));
     }
+    OURS_TRY(cudaFuncSetAttribute(k_ours_inner, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(InnerShared)));
     for (int it = 0; it < R.outer_iters; ++it) {
         if (nq > 0) {
             k_ours_tris<<<grid_for(nq, 128, sms), 128, 0, s>>>(P);
@@ -1020,20 +1247,20 @@ cudaError_t ours_run(OursRun& R, cudaStream_t s) {
             }
             OURS_TRY(cudaMemsetAsync(P.cell_count, 0, sizeof(unsigned int) * (nv + 1), s));
             OURS_TRY(cudaMemsetAsync(P.cell_fill, 0, sizeof(unsigned int) * (nv + 1), s));
-            OURS_TRY(cudaMemsetAsync(P.heavy_count, 0, sizeof(unsigned int), s));
+            OURS_TRY(cudaMemsetAsync(P.team_count, 0, sizeof(unsigned int) * 7, s));
             k_ours_query<<<grid_for(P.nsel, 128, sms), 128, 0, s>>>(P);
+            k_ours_query_long<<<(unsigned)sms * 8, 32 * kLongWarps, 0, s>>>(P);
             OURS_TRY(launch_scan(P.cell_count, nv, partials, P.cell_start,
                                  reinterpret_cast<unsigned long long*>(counters + 4), s));
             k_ours_scatter<<<grid_for(P.nsel, 128, sms), 128, 0, s>>>(P);
             k_ours_sort<<<grid_for(nv, 128, sms), 128, 0, s>>>(P);
         } else {
             OURS_TRY(cudaMemsetAsync(P.cell_count, 0, sizeof(unsigned int) * (nv + 1), s));
-            OURS_TRY(cudaMemsetAsync(P.heavy_count, 0, sizeof(unsigned int), s));
+            OURS_TRY(cudaMemsetAsync(P.team_count, 0, sizeof(unsigned int) * 7, s));
         }
         k_ours_faces<<<grid_for(nv, 128, sms), 128, 0, s>>>(P);
         if (R.hermite_update && it > 0) k_ours_hermite<<<grid_for(12 * nv, 128, sms), 128, 0, s>>>(P);
-        k_ours_inner<<<grid_for(nv, 128, sms), 128, 0, s>>>(P);
-        k_ours_inner_warp<<<grid_for(32 * nv, 128, sms), 128, 0, s>>>(P);
+        if (P.inner_iters > 0) k_ours_inner<<<(unsigned)sms * 2, kInnerThreads, sizeof(InnerShared), s>>>(P);
         k_ours_mesh<<<grid_for(nv, 128, sms), 128, 0, s>>>(P);
         OURS_TRY(cudaGetLastError());
     }
