@@ -987,7 +987,10 @@ int run_mesh_sdf(dcb_context* h, const float* d_verts, int64_t nv, const int32_t
     DCB_TRY(h, ensure(h->m_partials, sizeof(uint32_t) * std::max(1LL, scan_partials_len(P.nbins))), "alloc scan");
     DCB_TRY(h, ensure(h->m_far, sizeof(uint32_t) * rows * P.W), "alloc masks");
     DCB_TRY(h, ensure(h->m_ext, sizeof(uint32_t) * rows * P.W), "alloc masks");
-    DCB_TRY(h, ensure(h->m_tmp, sizeof(float) * (size_t)nx * ny * nz), "alloc relaxation buffer");
+    if (!voxelize_first) {             // the band's values, which the relaxation reads
+        DCB_TRY(h, ensure(h->m_tmp, sizeof(float) * (size_t)nx * ny * nz), "alloc relaxation buffer");
+        P.out = as<float>(h->m_tmp);
+    }
     DCB_TRY(h, ensure(h->m_counters, sizeof(SdfCounters)), "alloc counters");
     if (!h->h_sdf_counters) DCB_TRY(h, host_malloc(&h->h_sdf_counters, sizeof(SdfCounters)), "alloc pinned counters");
     SdfCounters* dc = as<SdfCounters>(h->m_counters);
@@ -1034,7 +1037,8 @@ int run_mesh_sdf(dcb_context* h, const float* d_verts, int64_t nv, const int32_t
             if (passes > 1000000) return fail(h, DCB_ERR_INTERNAL, "exterior flood did not converge");
         }
         DCB_TRY(h, cudaEventRecord(ev[3], s), "event");
-        DCB_TRY(h, launch_sdf_finish(P, &dc->exterior, as<float>(h->m_tmp), h->num_sms, s), "launch finish");
+        P.out = out;
+        DCB_TRY(h, launch_sdf_finish(P, as<float>(h->m_tmp), &dc->exterior, h->num_sms, s), "launch finish");
     } else {
         // the voxel solid (:764-808): shell, dilation, exterior flood to its fixpoint; then the
         // far grid points take their sign from it (:826-832); no relaxation in this branch

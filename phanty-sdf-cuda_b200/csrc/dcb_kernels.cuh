@@ -381,7 +381,8 @@ cudaError_t launch_sdf_bins(const SdfParams& P, int num_sms, cudaStream_t s);
 cudaError_t launch_sdf_band(const SdfParams& P, int num_sms, cudaStream_t s);
 cudaError_t launch_sdf_masks(const SdfParams& P, int num_sms, cudaStream_t s);
 cudaError_t launch_sdf_flood(const SdfParams& P, int* changed, int num_sms, cudaStream_t s);
-cudaError_t launch_sdf_finish(const SdfParams& P, unsigned long long* filled, float* tmp, int num_sms, cudaStream_t s);
+// far values and relaxation: the band's values -> P.out
+cudaError_t launch_sdf_finish(const SdfParams& P, const float* band, unsigned long long* filled, int num_sms, cudaStream_t s);
 cudaError_t launch_vox_raster(const SdfParams& P, int num_sms, cudaStream_t s);
 cudaError_t launch_vox_dilate(const SdfParams& P, int num_sms, cudaStream_t s);
 // the exterior flood of the voxel grid (k_flood on vfar / vext)
