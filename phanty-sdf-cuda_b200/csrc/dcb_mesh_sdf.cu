@@ -1007,7 +1007,15 @@ __global__ void __launch_bounds__(kFloodThreads) k_flood(SdfParams P, int* chang
                 const uint32_t far = s_far[lz - 1][ly - 1][lx - 1];
                 const uint32_t nb = (cur << 1) | (cur >> 1) | (s_ext[lz][ly][lx - 1] >> 31) | (s_ext[lz][ly][lx + 1] << 31) |
                                     s_ext[lz][ly - 1][lx] | s_ext[lz][ly + 1][lx] | s_ext[lz - 1][ly][lx] | s_ext[lz + 1][ly][lx];
-                const uint32_t nxt = cur | (far & nb);
+                // along x the flood runs through the word's far points at once (both ways, doubling
+                // steps); y and z take a sweep a point
+                uint32_t nxt = cur | (far & nb);
+                uint32_t pass = far;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) { nxt |= pass & (nxt << o); pass &= pass << o; }
+                pass = far;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) { nxt |= pass & (nxt >> o); pass &= pass >> o; }
                 if (nxt != cur) { s_ext[lz][ly][lx] = nxt; mine = 1; }
             }
             const int any = __syncthreads_or(mine);
@@ -1157,28 +1165,32 @@ k_sdf_relax(const __grid_constant__ SdfParams P, const float* __restrict__ in, i
 
 // ---- voxelize-first (compute_mesh_sdf_device_cuda with voxelize_first, :764-832) -------------
 
-// A thread per triangle: every voxel corner of the triangle's voxel box whose squared distance
-// to the triangle is within (0.866 * largest voxel side)^2 joins the shell (:458-501).
+// A warp per triangle: every voxel corner of the triangle's voxel box whose squared distance
+// to the triangle is within (0.866 * largest voxel side)^2 joins the shell (:458-501). (10,240
+// triangles on 256^3 voxels: 253 us with a thread per triangle, 320 warps on the whole GPU.)
 __global__ void __launch_bounds__(256) k_vox_raster(SdfParams P) {
-    const int vr = P.vres;
+    const int vr = P.vres, lane = threadIdx.x & 31;
     const float mvd = fmaxf(P.vox_vx, fmaxf(P.vox_vy, P.vox_vz)) * 0.8660254f;
     const float lim = mvd * mvd;
-    for (long long f = (long long)blockIdx.x * blockDim.x + threadIdx.x; f < P.nf; f += (long long)gridDim.x * blockDim.x) {
+    for (long long f = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; f < P.nf;
+         f += ((long long)gridDim.x * blockDim.x) >> 5) {
         float3 a, b, c;
         if (!load_tri(P, f, a, b, c)) continue;
         const float mnx = fminf(a.x, fminf(b.x, c.x)), mny = fminf(a.y, fminf(b.y, c.y)), mnz = fminf(a.z, fminf(b.z, c.z));
         const float mxx = fmaxf(a.x, fmaxf(b.x, c.x)), mxy = fmaxf(a.y, fmaxf(b.y, c.y)), mxz = fmaxf(a.z, fmaxf(b.z, c.z));
-        const int bx0 = bin_coord(mnx, P.ox, P.vox_vx, vr), bx1 = bin_coord(mxx, P.ox, P.vox_vx, vr);
-        const int by0 = bin_coord(mny, P.oy, P.vox_vy, vr), by1 = bin_coord(mxy, P.oy, P.vox_vy, vr);
-        const int bz0 = bin_coord(mnz, P.oz, P.vox_vz, vr), bz1 = bin_coord(mxz, P.oz, P.vox_vz, vr);
-        for (int bz = bz0; bz <= bz1; ++bz)
-            for (int by = by0; by <= by1; ++by)
-                for (int bx = bx0; bx <= bx1; ++bx) {
-                    const float3 q = f3(P.ox + (float)bx * P.vox_vx, P.oy + (float)by * P.vox_vy, P.oz + (float)bz * P.vox_vz);
-                    float3 closest;
-                    if (point_triangle(q, a, b, c, closest) <= lim)
-                        atomicOr(P.vshell + ((long long)bz * vr + by) * P.Wv + (bx >> 5), 1u << (bx & 31));
-                }
+        const int bx0 = bin_coord(mnx, P.ox, P.vox_vx, vr), sx = bin_coord(mxx, P.ox, P.vox_vx, vr) - bx0 + 1;
+        const int by0 = bin_coord(mny, P.oy, P.vox_vy, vr), sy = bin_coord(mxy, P.oy, P.vox_vy, vr) - by0 + 1;
+        const int bz0 = bin_coord(mnz, P.oz, P.vox_vz, vr), sz = bin_coord(mxz, P.oz, P.vox_vz, vr) - bz0 + 1;
+        if (sx <= 0 || sy <= 0 || sz <= 0) continue;
+        const long long nvox = (long long)sx * sy * sz;
+        for (long long w = lane; w < nvox; w += 32) {
+            const int row = (int)(w / sx);
+            const int bx = bx0 + (int)(w - (long long)row * sx), by = by0 + row % sy, bz = bz0 + row / sy;
+            const float3 q = f3(P.ox + (float)bx * P.vox_vx, P.oy + (float)by * P.vox_vy, P.oz + (float)bz * P.vox_vz);
+            float3 closest;
+            if (point_triangle(q, a, b, c, closest) <= lim)
+                atomicOr(P.vshell + ((long long)bz * vr + by) * P.Wv + (bx >> 5), 1u << (bx & 31));
+        }
     }
 }
 
@@ -1322,7 +1334,7 @@ cudaError_t launch_sdf_finish(const SdfParams& P, const float* band, unsigned lo
 
 cudaError_t launch_vox_raster(const SdfParams& P, int num_sms, cudaStream_t s) {
     if (P.nf <= 0) return cudaSuccess;
-    k_vox_raster<<<grid_for(P.nf, 256, num_sms, 16), 256, 0, s>>>(P);
+    k_vox_raster<<<grid_for(P.nf, 8, num_sms, 16), 256, 0, s>>>(P);
     return cudaGetLastError();
 }
 
