@@ -58,7 +58,8 @@ struct dcb_context {
     int num_sms = 148;
     std::string last_error;
     cudaEvent_t ev[10] = {};
-    bool substage_events = false;     // ev[8] / ev[9] hold the face sub-stages of the last call
+    bool substage_events = false;     // ev[9] (and ev[8] with count_event) hold the face sub-stages of the last call
+    bool count_event = false;
     DevBuf grid, bits, super, list, seg_count, seg_start, counters, V, vclass, fmask, col_count, col_fill,
         col_start, partials, esc_list, hard_list, hard_data, stage_quad, stage_key, faces, wind_items,
         v64_index, v64_cells, V64, tris, tri_items, adj_rows, adj_owners, ours_ws, wt;
@@ -237,8 +238,12 @@ int layout_batch(dcb_context* h, const dcb_grid* in, int n, BatchLayout& L) {
         // About four CTAs per resident slot, each marching 8..64 planes (a single long wave
         // measured slower at 1024^3: 0.887 vs 0.848 ms).
         if (h->mark_ctas[n == 1] == 0) h->mark_ctas[n == 1] = mark_ctas_per_sm(n == 1);
-        const long long slots = (long long)h->num_sms * h->mark_ctas[n == 1] * h->tune_waves;
-        S.KZ = (int)std::max(8LL, std::min(64LL, (g.cz * S.nxt * (long long)S.nrb + slots - 1) / slots));
+        const long long wave = (long long)h->num_sms * h->mark_ctas[n == 1], slots = wave * h->tune_waves;
+        const long long planes = g.cz * S.nxt * (long long)S.nrb;      // one CTA each, marched plane by plane
+        // at least 8 planes (the plane above the last is read twice), fewer where a single grid
+        // would leave SMs idle: 32^3 has 20 CTAs of 8 planes (6.5 us), 80 of 2 (3.6)
+        const long long least = n == 1 ? std::max(2LL, std::min(8LL, (planes + wave - 1) / wave)) : 8LL;
+        S.KZ = (int)std::max(least, std::min(64LL, (planes + slots - 1) / slots));
         S.nzc = (g.cz + S.KZ - 1) / S.KZ;
         S.bits_off = L.bits;
         S.super_off = L.super;
@@ -305,6 +310,12 @@ void destroy_graph(dcb_context* h) {
 
 int upload_table(dcb_context* h, const BatchLayout& L, cudaStream_t s, TableView& T) {
     const int n = (int)L.slots.size();
+    if (n == 1) {                          // one grid: its slot travels in the kernel parameters
+        std::memset(&T, 0, sizeof(T));
+        T.B.s0 = L.slots[0];
+        T.B.n = 1;
+        return DCB_OK;
+    }
     const size_t o_slots = 0;
     const size_t o_seg = align_up(o_slots + sizeof(GridSlot) * n);
     const size_t o_col = align_up(o_seg + sizeof(long long) * (n + 1));
@@ -420,14 +431,24 @@ int batch_alloc(dcb_context* h, int n, long long cap, const dcb_opts* o, TableVi
 // first vertex of every grid.
 int batch_mark(dcb_context* h, const BatchLayout& L, const TableView& T, cudaStream_t s, bool events) {
     Counters* dc = as<Counters>(h->counters);
-    DCB_TRY(h, cudaMemsetAsync(h->counters.p, 0, sizeof(Counters), s), "memset counters");
+    DCB_TRY(h, launch_prepare(T.B, as<float>(h->wt), h->counters.p, sizeof(Counters), as<uint32_t>(h->col_count), L.ncol,
+                              h->num_sms, s), "launch prepare");
     int rc = launch_marks(h, L, T, s);
     if (rc != DCB_OK) return rc;
     if (events) DCB_TRY(h, cudaEventRecord(h->ev[6], s), "event");
     DCB_TRY(h, launch_scan(as<uint32_t>(h->seg_count), L.nseg, as<uint32_t>(h->partials), as<uint32_t>(h->seg_start),
                            &dc->total_active, s), "launch segment scan");
-    DCB_TRY(h, launch_vert_offsets(T.B, as<uint32_t>(h->seg_start), &dc->total_active, T.vert_off, s), "vertex offsets");
+    if (T.B.n > 1)
+        DCB_TRY(h, launch_vert_offsets(T.B, as<uint32_t>(h->seg_start), &dc->total_active, T.vert_off, s), "vertex offsets");
     if (events) DCB_TRY(h, cudaEventRecord(h->ev[2], s), "event");
+    return DCB_OK;
+}
+
+// Copies every grid's first vertex to h_offsets (one grid: batch_state knows them).
+int read_vert_offsets(dcb_context* h, const TableView& T, cudaStream_t s) {
+    if (T.B.n == 1) return DCB_OK;
+    DCB_TRY(h, cudaMemcpyAsync(h->h_offsets, T.vert_off, sizeof(unsigned long long) * (T.B.n + 1), cudaMemcpyDeviceToHost, s),
+            "read vertex offsets");
     return DCB_OK;
 }
 
@@ -447,7 +468,8 @@ void batch_state(dcb_context* h, const BatchLayout& L, int n, const dcb_opts* o,
     h->vert_offsets.assign(n + 1, 0);
     h->face_offsets.assign(n + 1, 0);
     for (int b = 0; b < n; ++b) { h->batch_cx[b] = L.slots[b].g.cx; h->batch_cy[b] = L.slots[b].g.cy; }
-    for (int b = 0; b <= n; ++b) h->vert_offsets[b] = (int64_t)h_vert_off[b];
+    if (n == 1) h->vert_offsets[1] = nv;
+    else for (int b = 0; b <= n; ++b) h->vert_offsets[b] = (int64_t)h_vert_off[b];
 }
 
 // Everything after the mark for up to `cap` active cells: ranks and list, vertices, faces.
@@ -460,9 +482,6 @@ int batch_rest(dcb_context* h, const BatchLayout& L, TableView& T, const dcb_opt
     Counters* dc = as<Counters>(h->counters);
     const long long wind_cap = std::min(0x7fffffffLL, 3 * cap);
     const long long v64_cap = cap;
-    DCB_TRY(h, cudaMemsetAsync(h->col_count.p, 0, sizeof(uint32_t) * ncol, s), "memset");
-    DCB_TRY(h, cudaMemsetAsync(h->v64_index.p, 0xff, sizeof(int) * cap, s), "memset");
-
     // 2) ranks + list, QEF with fused edge normals (rank-1 fast path, Jacobi list, FP64).
     ExpandParams xp;
     xp.B = T.B; xp.nseg = nseg; xp.bits = as<uint32_t>(h->bits); xp.seg_count = as<uint32_t>(h->seg_count);
@@ -471,11 +490,11 @@ int batch_rest(dcb_context* h, const BatchLayout& L, TableView& T, const dcb_opt
     xp.B.cell_slot = nullptr;                      // expand finds grids by segment
     xp.list_cap = cap;
     DCB_TRY(h, launch_expand(xp, h->num_sms, s), "launch expand");
-    DCB_TRY(h, launch_width_tables(T.B, as<float>(h->wt), s), "launch width tables");
     QefParams qp;
     qp.B = T.B; qp.list = xp.list; qp.nactive = cap; qp.live = live; qp.V = as<float>(h->V); qp.vclass = as<uint8_t>(h->vclass);
     qp.fmask = as<uint8_t>(h->fmask); qp.col_count = as<uint32_t>(h->col_count);
     qp.wt = as<float>(h->wt);
+    qp.v64_index = as<int>(h->v64_index);
     qp.esc_list = as<uint32_t>(h->esc_list); qp.esc_count = &dc->esc_count;
     qp.hard_list = as<uint32_t>(h->hard_list); qp.hard_data = as<float4>(h->hard_data); qp.hard_count = &dc->hard_count;
     qp.rank_hist = dc->rank_hist;
@@ -490,17 +509,14 @@ int batch_rest(dcb_context* h, const BatchLayout& L, TableView& T, const dcb_opt
     v64.Vf = qp.V; v64.vclass = qp.vclass; v64.V64 = nullptr; v64.thr = o->svd_threshold;
     DCB_TRY(h, launch_vertex_fp64(v64, cap, h->num_sms, s), "launch vertex fp64");
     if (events) DCB_TRY(h, cudaEventRecord(h->ev[3], s), "event");
-    // the faces were counted per column by k_cell_qef
-    if (events) DCB_TRY(h, cudaEventRecord(h->ev[8], s), "event");
 
-    // 3) faces: column scan, scatter with FP32 winding, FP64 re-decisions, in-column order.
+    // 3) faces (counted per column by k_cell_qef): column scan, scatter with FP32 winding, FP64 re-decisions, in-column order.
     DCB_TRY(h, launch_scan(as<uint32_t>(h->col_count), ncol, as<uint32_t>(h->partials),
-                           as<uint32_t>(h->col_start), &dc->face_total, s), "launch scan");
-    DCB_TRY(h, cudaMemcpyAsync(h->col_fill.p, h->col_start.p, sizeof(uint32_t) * ncol, cudaMemcpyDeviceToDevice, s),
-            "column slots");
+                           as<uint32_t>(h->col_start), &dc->face_total, s, as<uint32_t>(h->col_fill)), "launch scan");
     if (events) {
         DCB_TRY(h, cudaEventRecord(h->ev[9], s), "event");
         h->substage_events = true;
+        h->count_event = false;
     }
     if (n > 1)
         DCB_TRY(h, launch_face_offsets(T.B, as<uint32_t>(h->col_start), &dc->face_total, T.face_off, s), "face offsets");
@@ -605,7 +621,6 @@ int run_batch(dcb_context* h, const dcb_grid* in, int n, const dcb_opts* o, cuda
     if (rc != DCB_OK) return rc;
     Counters* dc = as<Counters>(h->counters);
     Counters* hc = reinterpret_cast<Counters*>(h->h_counters);
-    unsigned long long* h_vert_off = reinterpret_cast<unsigned long long*>(h->h_offsets);
 
     // 1) mark: active bits + per-segment counts; scan -> segment starts and the total.
     rc = batch_mark(h, L, T, s, true);
@@ -620,8 +635,8 @@ int run_batch(dcb_context* h, const dcb_grid* in, int n, const dcb_opts* o, cuda
         if (rc != DCB_OK) return rc;
         DCB_TRY(h, cudaEventRecord(h->ev[4], s), "event");
         DCB_TRY(h, cudaMemcpyAsync(hc, dc, sizeof(Counters), cudaMemcpyDeviceToHost, s), "read counters");
-        DCB_TRY(h, cudaMemcpyAsync(h_vert_off, T.vert_off, sizeof(unsigned long long) * (n + 1),
-                                   cudaMemcpyDeviceToHost, s), "read vertex offsets");
+        rc = read_vert_offsets(h, T, s);
+        if (rc != DCB_OK) return rc;
         DCB_TRY(h, cudaStreamSynchronize(s), "pipeline");
         const long long nv = (long long)hc->total_active;
         if (nv >= 0x7fffffffLL) return fail(h, DCB_ERR_TOO_LARGE, "more than 2^31-1 vertices");
@@ -640,8 +655,8 @@ int run_batch(dcb_context* h, const dcb_grid* in, int n, const dcb_opts* o, cuda
         DCB_TRY(h, cudaMemcpyAsync(dc, hc, sizeof(Counters), cudaMemcpyHostToDevice, s), "reset counters");
     }
     DCB_TRY(h, cudaMemcpyAsync(hc, dc, sizeof(Counters), cudaMemcpyDeviceToHost, s), "read count");
-    DCB_TRY(h, cudaMemcpyAsync(h_vert_off, T.vert_off, sizeof(unsigned long long) * (n + 1), cudaMemcpyDeviceToHost, s),
-            "read vertex offsets");
+    rc = read_vert_offsets(h, T, s);
+    if (rc != DCB_OK) return rc;
     DCB_TRY(h, cudaStreamSynchronize(s), "mark");
     const long long nv = (long long)hc->total_active;
     if (nv >= 0x7fffffffLL) return fail(h, DCB_ERR_TOO_LARGE, "more than 2^31-1 vertices");
@@ -877,6 +892,7 @@ int run_sparse(dcb_context* h, const dcb_grid* in, const dcb_opts* o, cudaStream
                                dcn + kScFaces, s), "launch face scan");
         DCB_TRY(h, cudaEventRecord(h->ev[9], s), "event");
         h->substage_events = true;
+        h->count_event = true;
         DCB_TRY(h, cudaMemcpyAsync(hcn, dcn, sizeof(unsigned long long) * kScSlots, cudaMemcpyDeviceToHost, s), "read totals");
         DCB_TRY(h, cudaStreamSynchronize(s), "sparse vertices");
         nverts = mvdc ? (long long)hcn[kScVertices] : na;
@@ -941,8 +957,10 @@ void fill_times(dcb_context* h, dcb_stats* st, bool upload) {
     st->active_brick_compaction_ms = 0.f;
     st->active_cell_marking_ms = st->marking_ms;
     st->active_cell_compaction_ms = st->compaction_ms;
-    st->face_count_ms = h->substage_events ? elapsed(h->ev[3], h->ev[8]) : 0.f;
-    st->face_prefix_sum_ms = h->substage_events ? elapsed(h->ev[8], h->ev[9]) : 0.f;
+    // (the dense path counts faces in the vertex kernel: no stage of its own)
+    const cudaEvent_t counted = h->ev[h->count_event ? 8 : 3];
+    st->face_count_ms = h->substage_events && h->count_event ? elapsed(h->ev[3], counted) : 0.f;
+    st->face_prefix_sum_ms = h->substage_events ? elapsed(counted, h->ev[9]) : 0.f;
     st->face_fill_ms = h->substage_events ? elapsed(h->ev[9], h->ev[4]) : 0.f;
     // the reference declares and reports bad_qef_count but never increments it
     // (dc_cuda_sparse.cu:41, 1481)
@@ -1198,7 +1216,6 @@ int dcb_extract_device(dcb_handle h, const dcb_grid* grid, const dcb_opts* opts,
     if (cudaSetDevice(h->device) != cudaSuccess) { cudaGetLastError(); return fail(h, DCB_ERR_CUDA, "set device"); }
     cudaStream_t s = reinterpret_cast<cudaStream_t>(cuda_stream);
     if (stats) std::memset(stats, 0, sizeof(*stats));
-    DCB_TRY(h, cudaEventRecord(h->ev[0], s), "event");
     DCB_TRY(h, cudaEventRecord(h->ev[1], s), "event");
     rc = run_method(h, grid, o, s, stats);
     if (rc != DCB_OK) return rc;
@@ -1332,10 +1349,8 @@ int dcb_batch_graph_create(dcb_handle h, const dcb_grid* grids, int n, const dcb
     if (rc == DCB_OK) rc = batch_rest(h, g->L, g->T, o, s, cap, &dc->total_active, false);
     if (rc == DCB_OK) {
         e = cudaMemcpyAsync(h->h_counters, dc, sizeof(Counters), cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(h->h_offsets, g->T.vert_off, sizeof(unsigned long long) * (n + 1),
-                                cudaMemcpyDeviceToHost, s);
         if (e != cudaSuccess) rc = cuda_fail(h, e, "capture read-back");
+        else rc = read_vert_offsets(h, g->T, s);
     }
     const cudaError_t ee = cudaStreamEndCapture(s, &g->graph);
     if (rc == DCB_OK && ee != cudaSuccess) rc = cuda_fail(h, ee, "end capture");
@@ -1449,8 +1464,10 @@ int dcb_copy_mesh_device(dcb_handle h, float* vertices, int32_t* faces, void* cu
     if (!h) return DCB_ERR_INVALID_ARGUMENT;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(cuda_stream);
     if (cudaSetDevice(h->device) != cudaSuccess) { cudaGetLastError(); return fail(h, DCB_ERR_CUDA, "set device"); }
-    if (vertices && h->nv) DCB_TRY(h, cudaMemcpyAsync(vertices, h->V.p, sizeof(float) * 3 * h->nv, cudaMemcpyDeviceToDevice, s), "copy vertices");
-    if (faces && h->nf) DCB_TRY(h, cudaMemcpyAsync(faces, face_ptr(h), sizeof(int32_t) * h->vpf * h->nf, cudaMemcpyDeviceToDevice, s), "copy faces");
+    const long long nv = vertices ? 3 * h->nv : 0, nf = faces ? (long long)h->vpf * h->nf : 0;
+    if (nv || nf)
+        DCB_TRY(h, launch_copy_mesh(as<float>(h->V), nv ? vertices : nullptr, nv, nf ? face_ptr(h) : nullptr, nf ? faces : nullptr,
+                                    nf, h->num_sms, s), "copy mesh");
     return DCB_OK;
 }
 

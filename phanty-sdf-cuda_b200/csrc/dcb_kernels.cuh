@@ -25,7 +25,7 @@ struct GridSlot {
     long long wt_off;              // first entry of the grid's cell-width tables (width_tables)
 };
 
-// Cell-width tables of a grid (k_width_tables): for each axis the widths of cells -1..n (n the
+// Cell-width tables of a grid (k_prepare): for each axis the widths of cells -1..n (n the
 // cells along it), entry c + 1 for cell c, then their reciprocals: w_x, w_y, w_z, r_x, r_y, r_z.
 __host__ __device__ inline long long width_table_len(int cx, int cy, int cz) {
     return 2LL * ((long long)cx + cy + cz + 6);
@@ -33,7 +33,7 @@ __host__ __device__ inline long long width_table_len(int cx, int cy, int cz) {
 
 struct BatchTable {
     GridSlot s0;                           // the grid when n == 1 (read from kernel parameters)
-    const GridSlot* slots;                 // [n], device
+    const GridSlot* slots;                 // [n], device (n > 1)
     int n;
     const long long* seg_off;              // [n+1] first segment per grid
     const long long* col_off;              // [n+1] first face column per grid
@@ -56,6 +56,10 @@ __device__ __forceinline__ int slot_search(const T* __restrict__ offs, int n, T 
 template <bool ONE>
 __device__ __forceinline__ const GridSlot& slot_ref(const BatchTable& B, int gi) {
     return ONE ? B.s0 : B.slots[gi];
+}
+// Kernels of both kinds of launch: the table in device memory exists for batches only.
+__device__ __forceinline__ const GridSlot& slot_at(const BatchTable& B, int gi) {
+    return B.n == 1 ? B.s0 : B.slots[gi];
 }
 __device__ __forceinline__ int slot_of_rank(const BatchTable& B, unsigned long long r) {
     if (B.n == 1) return 0;
@@ -109,6 +113,9 @@ cudaError_t launch_vert_offsets(const BatchTable& B, const uint32_t* seg_start, 
 cudaError_t launch_face_offsets(const BatchTable& B, const uint32_t* col_start, const unsigned long long* total,
                                 unsigned long long* face_off, cudaStream_t s);
 // Global vertex ranks in the faces -> ranks within each face's grid (vpf ints per face).
+// Vertices (nv floats) and faces (nf ints) to the caller's device arrays in one launch.
+cudaError_t launch_copy_mesh(const float* V, float* out_V, long long nv, const int* F, int* out_F, long long nf, int num_sms,
+                             cudaStream_t s);
 cudaError_t launch_localize_faces(const unsigned long long* vert_off, const unsigned long long* face_off, int n,
                                   int* faces, int vpf, long long max_faces, int num_sms, cudaStream_t s);
 
@@ -122,7 +129,8 @@ struct QefParams {
     long long nactive;             // active cells (capacity when live is set)
     const unsigned long long* live; // device count of active cells (a captured graph; above
                                     // nactive, nothing is processed), or null
-    const float* wt;                // cell-width tables of every grid (k_width_tables)
+    const float* wt;                // cell-width tables of every grid (k_prepare)
+    int* v64_index;                 // set to -1 (no FP64 vertex asked for) at every rank
     float* V;
     uint8_t* vclass;                // [active] VertexClass
     uint8_t* fmask;                 // bit a: cell owns a face on its min-corner edge a
@@ -141,9 +149,11 @@ struct QefParams {
     float cond_max;
     int force64;
 };
+// Before the mark: every grid's cell-width tables, zeros for the counters and the column counts.
+cudaError_t launch_prepare(const BatchTable& B, float* wt, void* counters, size_t counter_bytes, uint32_t* col_count,
+                           long long ncol, int num_sms, cudaStream_t s);
 // minb: k_cell_qef's register cap (resident blocks per SM: 4, 5 or 6); blocks_per_sm: the width
 // of its grid-stride launch
-cudaError_t launch_width_tables(const BatchTable& B, float* wt, cudaStream_t s);
 cudaError_t launch_cell_qef(const QefParams& P, int num_sms, cudaStream_t s, int minb = 5, int blocks_per_sm = 32);
 cudaError_t launch_cell_jacobi(const QefParams& P, long long max_items, int num_sms, cudaStream_t s);
 
@@ -172,8 +182,9 @@ struct Winding64Params {
 };
 cudaError_t launch_winding_fp64(const Winding64Params& P, long long max_items, int num_sms, cudaStream_t s);
 
+// Exclusive sums of n counts into out and, if given, copy; their total.
 cudaError_t launch_scan(const uint32_t* in, long long n, uint32_t* partials, uint32_t* out,
-                        unsigned long long* grand_total, cudaStream_t s);
+                        unsigned long long* grand_total, cudaStream_t s, uint32_t* copy = nullptr);
 long long scan_partials_len(long long n);
 
 struct FaceParams {
@@ -189,7 +200,7 @@ struct FaceParams {
     const uint32_t* super;
     const uint32_t* col_start;     // per grid [3][cx*cy] (global column index)
     const uint32_t* col_count;
-    uint32_t* col_fill;            // next free slot of each column (starts as a copy of col_start)
+    uint32_t* col_fill;            // next free slot of each column (the scan's copy of col_start)
     int4* stage_quad;
     uint2* stage_key;              // {k, column}
     uint4* wind_items;             // {slot, axis | grid << 2, packed lo, packed hi}

@@ -113,32 +113,43 @@ __device__ float3 edge_normal(const GridDesc& g, int3 lo, int axis, int o1, int 
     return normalized(acc);
 }
 
-// ---- cell-width tables ------------------------------------------------------------------
+// ---- what precedes the mark ---------------------------------------------------------------
 
-// Block row b fills grid b's tables: the width of cell c along an axis is the difference of
-// the float positions of its two planes (grid.ox + i * grid.vx rounded in float, as the CPU
-// backend forms positions, dc_backend.cpp:63-65), its reciprocal 1 / width.
-__global__ void __launch_bounds__(256) k_width_tables(const BatchTable B, float* __restrict__ wt) {
-    const GridSlot& S = B.n == 1 ? B.s0 : B.slots[blockIdx.y];
-    const GridDesc& g = S.g;
-    const int nx = g.cx + 2, ny = g.cy + 2, nz = g.cz + 2;
-    const int total = nx + ny + nz;
-    float* const t = wt + S.wt_off;
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
-        float o, vv;
-        int c;
-        if (e < nx)           { o = g.ox; vv = g.vx; c = e - 1; }
-        else if (e < nx + ny) { o = g.oy; vv = g.vy; c = e - nx - 1; }
-        else                  { o = g.oz; vv = g.vz; c = e - nx - ny - 1; }
-        const float w = pos_axis(o, vv, c + 1) - pos_axis(o, vv, c);
-        t[e] = w;
-        t[total + e] = 1.f / w;
+// Zeros for the counters and the column counts, and every grid's cell-width tables: the width
+// of cell c along an axis is the difference of the float positions of its two planes
+// (grid.ox + i * grid.vx rounded in float, as the CPU backend forms positions,
+// dc_backend.cpp:63-65), its reciprocal 1 / width. One launch for what were two memsets and a
+// kernel.
+__global__ void __launch_bounds__(256) k_prepare(const __grid_constant__ BatchTable B, float* __restrict__ wt, uint32_t* counters,
+                                                 int counter_words, uint32_t* __restrict__ col_count, long long ncol) {
+    const long long first = (long long)blockIdx.x * blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
+    if (first < counter_words) counters[first] = 0;
+    for (long long q = first; q < ncol; q += stride) col_count[q] = 0;
+    for (long long part = blockIdx.x; part < 4LL * B.n; part += gridDim.x) {      // four blocks a grid
+        const GridSlot& S = slot_at(B, (int)(part >> 2));
+        const GridDesc& g = S.g;
+        const int nx = g.cx + 2, ny = g.cy + 2, nz = g.cz + 2;
+        const int total = nx + ny + nz;
+        float* const t = wt + S.wt_off;
+        for (int e = (int)(part & 3) * blockDim.x + threadIdx.x; e < total; e += 4 * blockDim.x) {
+            float o, vv;
+            int c;
+            if (e < nx)           { o = g.ox; vv = g.vx; c = e - 1; }
+            else if (e < nx + ny) { o = g.oy; vv = g.vy; c = e - nx - 1; }
+            else                  { o = g.oz; vv = g.vz; c = e - nx - ny - 1; }
+            const float w = pos_axis(o, vv, c + 1) - pos_axis(o, vv, c);
+            t[e] = w;
+            t[total + e] = 1.f / w;
+        }
     }
 }
 
-cudaError_t launch_width_tables(const BatchTable& B, float* wt, cudaStream_t s) {
-    if (B.n <= 0) return cudaSuccess;
-    k_width_tables<<<dim3(4, (unsigned)B.n), 256, 0, s>>>(B, wt);
+cudaError_t launch_prepare(const BatchTable& B, float* wt, void* counters, size_t counter_bytes, uint32_t* col_count,
+                           long long ncol, int num_sms, cudaStream_t s) {
+    long long blocks = (ncol + 1023) / 1024;
+    if (blocks < 4LL * B.n) blocks = 4LL * B.n;
+    if (blocks > (long long)num_sms * 8) blocks = (long long)num_sms * 8;
+    k_prepare<<<(unsigned)blocks, 256, 0, s>>>(B, wt, static_cast<uint32_t*>(counters), (int)(counter_bytes / 4), col_count, ncol);
     return cudaGetLastError();
 }
 
@@ -192,6 +203,7 @@ k_cell_qef(const __grid_constant__ QefParams P) {
         // (contouring.cpp:560-594); the host reports DCB_ERR_INVALID_ARGUMENT
         if (((fm & 1) && isinf(c[1])) || ((fm & 6) && isinf(c[0]))) set_error(P.err, kErrNonFinite);
         P.fmask[r] = fm;
+        P.v64_index[r] = -1;
 
         // Pass 1: crossing edges and the centroid in local units.
         uint32_t hmask = 0;
@@ -348,7 +360,7 @@ __device__ __forceinline__ void jacobi3f(float a[3][3], float V[3][3]) {
 }
 
 __global__ void __launch_bounds__(128)
-k_cell_jacobi(QefParams P) {
+k_cell_jacobi(const __grid_constant__ QefParams P) {
     __shared__ unsigned int s_hist[4];
     if (threadIdx.x < 4) s_hist[threadIdx.x] = 0;
     __syncthreads();
@@ -383,7 +395,7 @@ k_cell_jacobi(QefParams P) {
             const unsigned int slot = atomicAdd(P.esc_count, 1u);
             P.esc_list[slot] = r;
         }
-        const GridDesc g = P.B.slots[slot_of_rank(P.B, r)].g;
+        const GridDesc& g = slot_at(P.B, slot_of_rank(P.B, r)).g;
         const float wx1 = width_axis(g, 0, i), wy1 = width_axis(g, 1, j), wz1 = width_axis(g, 2, k);
         store_vertex(P.V, g, r, i, j, k, d2.y + wx, d2.z + wy * (wx1 / wy1), d2.w + wz * (wx1 / wz1));
         P.vclass[r] = kVcJacobi;

@@ -188,16 +188,18 @@ __device__ __forceinline__ void store64(const Vertex64Params& P, uint32_t r, uns
 }
 
 // Listed cells' FP64 vertices: Vf[rank] (float) and/or V64[t] (double). The launch holds as
-// many warps as fit on the GPU at once. With up to kGroupMax cells per warp, the warp's lanes
-// take its cells' crossing edges, one (cell, edge) each: the Hermite sample with its averaged
-// normal and the normalised row, into shared memory; then a lane per cell sums the rows in
-// edge order and solves. With more cells, a thread takes a whole cell. Both give the bits
-// of the CPU's double arithmetic.
+// many warps as fit on the GPU at once. With up to kGroupMax cells per warp, four lanes take
+// a (cell, crossing edge) of the warp's cells, one lane for each of the edge's four cells: the
+// Hermite sample with its averaged normal and the normalised row, into shared memory; then a
+// lane per cell sums the rows in edge order and solves. With more cells, a thread takes a whole
+// cell. Both give the bits of the CPU's double arithmetic. Bound: the chain of double divisions
+// and roots, the solve's above all (32^3 CSG scene: 14.0 us a launch; 17.6 with a lane per
+// (cell, edge) that formed the four samples one after the other).
 constexpr int kGroupMax = 8;
 constexpr int kV64Threads = 128;
 
 __global__ void __launch_bounds__(kV64Threads)
-k_vertex_fp64(Vertex64Params P) {
+k_vertex_fp64(const __grid_constant__ Vertex64Params P) {
     __shared__ double s_rows[kV64Threads / 32][kGroupMax][12][8];
     __shared__ uint32_t s_mask[kV64Threads / 32][kGroupMax];
     __shared__ uint8_t s_pair[kV64Threads / 32][kGroupMax * 12];
@@ -215,7 +217,7 @@ k_vertex_fp64(Vertex64Params P) {
             const uint32_t r = P.cells[t0 + lane];
             int i, j, k;
             unpack_cell(P.list[r], i, j, k);
-            const GridDesc g = P.B.slots[slot_of_rank(P.B, r)].g;
+            const GridDesc& g = slot_at(P.B, slot_of_rank(P.B, r)).g;
             double cs[8];
 #pragma unroll
             for (int c = 0; c < 8; ++c)
@@ -235,22 +237,49 @@ k_vertex_fp64(Vertex64Params P) {
         off -= __popc(emask);
         for (uint32_t m = emask; m; m &= m - 1) s_pair[wb][off++] = (uint8_t)((lane << 4) | (__ffs(m) - 1));
         __syncwarp();
-        for (unsigned int pr = lane; pr < total; pr += 32) {
-            const int q = s_pair[wb][pr] >> 4, e = s_pair[wb][pr] & 15;
+        const int q4 = lane & 3;
+        for (unsigned int p0 = 0; p0 < total; p0 += 8) {                 // warp-uniform
+            const unsigned int pr = p0 + (lane >> 2);
+            const bool on = pr < total;
+            const int q = on ? s_pair[wb][pr] >> 4 : 0, e = on ? s_pair[wb][pr] & 15 : 0;
             const uint32_t r = P.cells[t0 + q];
             int i, j, k;
             unpack_cell(P.list[r], i, j, k);
-            const GridDesc g = P.B.slots[slot_of_rank(P.B, r)].g;
-            f64::Cell64 C;
-            f64::load_cell(g, i, j, k, C);
-            double p[3], nn[3];
-            f64::edge_sample(g, C, i, j, k, e, p, nn);
-            // Cell::update row (Cell.cpp:298-311): normalise, b = n.p
-            if (sqrt(f64::sq3(nn)) > 0.0) f64::normalize3(nn);
-            double* R = s_rows[wb][q][e];
-            R[0] = p[0]; R[1] = p[1]; R[2] = p[2];
-            R[3] = nn[0]; R[4] = nn[1]; R[5] = nn[2];
-            R[6] = nn[0] * p[0] + nn[1] * p[1] + nn[2] * p[2];
+            const GridDesc& g = slot_at(P.B, slot_of_rank(P.B, r)).g;
+            int cc[4][3], ex[4];
+            const bool shared = f64::edge_cells(g, i, j, k, e, cc, ex);    // else the cell's own normal
+            int own = 0;
+            for (int u = 0; u < 4; ++u)
+                if (shared && cc[u][0] == i && cc[u][1] == j && cc[u][2] == k) own = u;
+            // lane u of the four: cell u's sample; its own cell's needs no test
+            const bool self = q4 == own;
+            double p[3] = {0.0, 0.0, 0.0}, nn[3] = {0.0, 0.0, 0.0};
+            bool good = false;
+            if (on && (shared || self)) {
+                f64::Cell64 C;
+                if (shared) f64::load_cell(g, cc[q4][0], cc[q4][1], cc[q4][2], C);
+                else f64::load_cell(g, i, j, k, C);
+                good = (self || f64::active(C)) && f64::hermite(C, self ? e : ex[q4], p, nn);
+            }
+            const unsigned int votes = __ballot_sync(0xffffffffu, good) >> (lane & ~3) & 15u;
+            double acc[3] = {0.0, 0.0, 0.0};
+            for (int u = 0; u < 4; ++u) {
+                double nu[3];
+                for (int d = 0; d < 3; ++d) nu[d] = f64::shfl_d(nn[d], (lane & ~3) | u);
+                if (sqrt(f64::sq3(nu)) > 0) { acc[0] += nu[0]; acc[1] += nu[1]; acc[2] += nu[2]; }
+            }
+            if (on && self) {
+                if (shared && votes == 15u) {
+                    f64::normalize3(acc);
+                    for (int d = 0; d < 3; ++d) nn[d] = acc[d];
+                }
+                // Cell::update row (Cell.cpp:298-311): normalise, b = n.p
+                if (sqrt(f64::sq3(nn)) > 0.0) f64::normalize3(nn);
+                double* R = s_rows[wb][q][e];
+                R[0] = p[0]; R[1] = p[1]; R[2] = p[2];
+                R[3] = nn[0]; R[4] = nn[1]; R[5] = nn[2];
+                R[6] = nn[0] * p[0] + nn[1] * p[1] + nn[2] * p[2];
+            }
         }
         __syncwarp();
         if ((unsigned)lane < cnt) {
@@ -264,7 +293,7 @@ k_vertex_fp64(Vertex64Params P) {
         const uint32_t r = P.cells[t];
         int i, j, k;
         unpack_cell(P.list[r], i, j, k);
-        const GridDesc g = P.B.slots[slot_of_rank(P.B, r)].g;
+        const GridDesc& g = slot_at(P.B, slot_of_rank(P.B, r)).g;
         double x[3];
         f64::cell_vertex_thread(g, i, j, k, P.thr, x);
         store64(P, r, t, x);
@@ -291,12 +320,12 @@ cudaError_t launch_vertex_fp64(const Vertex64Params& P, long long max_items, int
 // (contouring.cpp:624-641) from the FP64 vertices of its four cells and FP64 gradients.
 // Uncertain faces were staged in canonical order c0, c1, c2, c3.
 __global__ void __launch_bounds__(128)
-k_winding_fp64(Winding64Params P) {
+k_winding_fp64(const __grid_constant__ Winding64Params P) {
     const unsigned int n = min(*P.count, P.cap);
     for (unsigned int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
         const uint4 it = P.items[t];
         const int axis = (int)(it.y & 3u);
-        const GridDesc g = P.B.slots[it.y >> 2].g;
+        const GridDesc& g = slot_at(P.B, (int)(it.y >> 2)).g;
         int i, j, k;
         unpack_cell(((uint64_t)it.w << 32) | it.z, i, j, k);
         const int4 q4 = P.quads[it.x];
