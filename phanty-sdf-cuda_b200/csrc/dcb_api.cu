@@ -851,7 +851,7 @@ int run_sparse(dcb_context* h, const dcb_grid* in, const dcb_opts* o, cudaStream
         // 2) ranks + list, vertices
         DCB_TRY(h, ensure(h->list, sizeof(uint64_t) * na), "alloc active list");
         DCB_TRY(h, ensure(h->V, sizeof(float) * 3 * (mvdc ? 2 * na : na)), "alloc vertices");
-        DCB_TRY(h, ensure(h->sp_fcount, sizeof(uint32_t) * na), "alloc face counts");
+        DCB_TRY(h, ensure(h->sp_fcount, (sizeof(uint32_t) + 1) * na), "alloc face counts");
         DCB_TRY(h, ensure(h->sp_fstart, sizeof(uint32_t) * na), "alloc face starts");
         DCB_TRY(h, ensure(h->sp_stage, sizeof(int4) * 6 * na), "alloc face staging");
         plen = std::max(plen, scan_partials_len(na));
@@ -884,6 +884,7 @@ int run_sparse(dcb_context* h, const dcb_grid* in, const dcb_opts* o, cudaStream
         DCB_TRY(h, cudaEventRecord(h->ev[3], s), "event");
         // 3) faces: per-cell staging with counts, scan, compaction
         P.fcount = as<uint32_t>(h->sp_fcount);
+        P.fslots = reinterpret_cast<uint8_t*>(P.fcount + na);
         P.fstart = as<uint32_t>(h->sp_fstart);
         P.stage = as<int4>(h->sp_stage);
         DCB_TRY(h, launch_sparse_faces(P, h->num_sms, s), "launch faces");

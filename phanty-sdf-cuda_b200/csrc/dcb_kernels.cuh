@@ -439,6 +439,7 @@ struct SparseParams {
     float* N;                      // multi-vertex: [vertices][3]
     uint64_t* vcell;               // multi-vertex: [vertices] packed cell of each vertex
     uint32_t* fcount;              // [nactive] faces of the cell
+    uint8_t* fslots;               // [nactive] its staging slots in use
     const uint32_t* fstart;        // [nactive] first face (scan of fcount)
     int4* stage;                   // [nactive][6] faces of each cell before the scan
     int4* faces;
