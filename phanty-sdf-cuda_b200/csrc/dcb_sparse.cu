@@ -268,78 +268,43 @@ __device__ int face_vertex(const SparseParams& P, uint32_t r, float3 gn) {
 // ---- marking ----------------------------------------------------------------------------
 
 // Negative / positive / near-zero bit words of every point row (32 points a word), a warp
-// per 32 consecutive words of a row. VEC4 (rows 16-byte aligned, nx % 4 == 0): lane l loads
-// points 4l..4l+3 of each 128-point chunk as one float4, builds the three nibbles and an
-// 8-lane shuffle-OR forms each word; otherwise one coalesced scalar load and three ballots
-// per word.
-template <bool VEC4>
+// per 32 consecutive words of a row: a coalesced load and three ballots per word, eight loads in
+// flight; lane u keeps word u. (Four points a lane with the words put together by shuffles took
+// half as many instructions again: 210 us for 512^3.)
 __global__ void __launch_bounds__(256) k_sparse_points(const __grid_constant__ SparseParams P) {
     const GridDesc& g = P.g;
     const int lane = threadIdx.x & 31;
-    const int cpr = (P.Wp + 31) / 32;
-    const long long nchunks = (long long)g.ny * g.nz * cpr;
-    for (long long c = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < nchunks;
-         c += ((long long)gridDim.x * blockDim.x) >> 5) {
-        const long long row = c / cpr;
+    const uint32_t cpr = (P.Wp + 31) / 32, nchunks = (uint32_t)g.ny * g.nz * cpr;      // grids here are below 2^31 points
+    for (uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < nchunks; c += (gridDim.x * blockDim.x) >> 5) {
+        const uint32_t row = cpr == 1 ? c : c / cpr;
         const int w0 = (int)(c - row * cpr) * 32;
-        const float* src = g.v + row * g.nx;
+        const float* src = g.v + (size_t)row * g.nx;
+        const int nw = min(32, P.Wp - w0);
         uint32_t mn = 0, mp = 0, mc = 0;
-        if (VEC4) {
-            float4 v[8];
+        for (int u0 = 0; u0 < nw; u0 += 8) {
+            float v[8];
+            const int x0 = (w0 + u0) * 32 + lane;
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                const int x = w0 * 32 + 128 * q + 4 * lane;
-                v[q] = x < g.nx ? __ldg(reinterpret_cast<const float4*>(src + x)) : make_float4(0.f, 0.f, 0.f, 0.f);
-            }
+            for (int u = 0; u < 8; ++u) v[u] = x0 + 32 * u < g.nx ? __ldg(src + x0 + 32 * u) : __int_as_float(0x7fc00000);
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                const bool in = w0 * 32 + 128 * q + 4 * lane < g.nx;
-                const float e[4] = {v[q].x, v[q].y, v[q].z, v[q].w};
-                uint32_t n = 0, p = 0, z = 0;
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    n |= (e[u] < 0.f ? 1u : 0u) << u;
-                    p |= (e[u] > 0.f ? 1u : 0u) << u;
-                    z |= (fabsf(e[u]) <= P.close ? 1u : 0u) << u;
-                }
-                if (!in) n = p = z = 0;
-                const int sh = 4 * (lane & 7);
-                n <<= sh; p <<= sh; z <<= sh;
-#pragma unroll
-                for (int o = 1; o < 8; o <<= 1) {
-                    n |= __shfl_xor_sync(0xffffffffu, n, o);
-                    p |= __shfl_xor_sync(0xffffffffu, p, o);
-                    z |= __shfl_xor_sync(0xffffffffu, z, o);
-                }
-                // word 4q + (l >> 3) is complete in lanes 8*(l >> 3)..; lane L keeps word L
-                const int src_lane = 8 * (lane & 3);
-                const uint32_t tn = __shfl_sync(0xffffffffu, n, src_lane);
-                const uint32_t tp = __shfl_sync(0xffffffffu, p, src_lane);
-                const uint32_t tz = __shfl_sync(0xffffffffu, z, src_lane);
-                if ((lane >> 2) == q) { mn = tn; mp = tp; mc = tz; }
-            }
-        } else {
-#pragma unroll 8
-            for (int u = 0; u < 32; ++u) {
-                const int x = (w0 + u) * 32 + lane;
-                const bool in = x < g.nx;
-                const float v = in ? __ldg(src + x) : 0.f;
-                const uint32_t bn = __ballot_sync(0xffffffffu, in && v < 0.f);
-                const uint32_t bp = __ballot_sync(0xffffffffu, in && v > 0.f);
-                const uint32_t bc = __ballot_sync(0xffffffffu, in && fabsf(v) <= P.close);
-                if (lane == u) { mn = bn; mp = bp; mc = bc; }
+            for (int u = 0; u < 8; ++u) {                        // beyond the row: NaN, in no word
+                const uint32_t bn = __ballot_sync(0xffffffffu, v[u] < 0.f);
+                const uint32_t bp = __ballot_sync(0xffffffffu, v[u] > 0.f);
+                const uint32_t bc = __ballot_sync(0xffffffffu, fabsf(v[u]) <= P.close);
+                if (lane == u0 + u) { mn = bn; mp = bp; mc = bc; }
             }
         }
-        if (w0 + lane < P.Wp) {
-            const long long o = row * P.Wp + w0 + lane;
+        if (lane < nw) {
+            const size_t o = (size_t)row * P.Wp + w0 + lane;
             P.pn[o] = mn; P.pp[o] = mp; P.pc[o] = mc;
         }
     }
 }
 
 // Brick flags from the point words (:271-308): a block per row of bricks (by, bz). Its threads
-// OR the point words of the brick row's (s+1)^2 point rows, word by word (coalesced), into
-// shared memory; then a thread per brick tests its x-range of points in those words.
+// OR the point words of the brick row's (s+1)^2 point rows into shared memory, a word each
+// (coalesced) and, where the rows are short, several threads a word with every so many rows (512
+// points: 16 words, 8 threads each); then a thread per brick tests its x-range of points.
 constexpr int kBrickThreads = 128;
 constexpr int kMaxPointWords = 2048;           // nx <= 65536
 
@@ -354,16 +319,21 @@ __global__ void __launch_bounds__(kBrickThreads) k_sparse_bricks(const __grid_co
         const int j0 = by * P.bs, k0 = bz * P.bs;
         const int j1 = min(j0 + P.bs + 1, g.ny), k1 = min(k0 + P.bs + 1, g.nz);
         __syncthreads();
-        for (int w = threadIdx.x; w < P.Wp; w += blockDim.x) {
-            uint32_t n = 0, p = 0;
-            for (int k = k0; k < k1; ++k)
-                for (int j = j0; j < j1; ++j) {
-                    const long long o = ((long long)j + (long long)g.ny * k) * P.Wp + w;
+        for (int w = threadIdx.x; w < P.Wp; w += blockDim.x) s_n[w] = s_p[w] = 0;
+        __syncthreads();
+        const int parts = max(1, (int)blockDim.x / P.Wp), sj = j1 - j0, rows = sj * (k1 - k0);
+        const int part = (int)threadIdx.x / P.Wp;
+        if (part < parts) {
+            for (int w = (int)threadIdx.x - part * P.Wp; w < P.Wp; w += blockDim.x) {
+                uint32_t n = 0, p = 0;
+                for (int q = part; q < rows; q += parts) {
+                    const size_t o = ((size_t)(j0 + q % sj) + (size_t)g.ny * (k0 + q / sj)) * P.Wp + w;
                     n |= __ldg(P.pn + o);
                     p |= __ldg(P.pp + o);
                 }
-            s_n[w] = n;
-            s_p[w] = p;
+                if (n) atomicOr(&s_n[w], n);
+                if (p) atomicOr(&s_p[w], p);
+            }
         }
         __syncthreads();
         for (int bx = threadIdx.x; bx < P.nbx; bx += blockDim.x) {
@@ -383,48 +353,53 @@ __global__ void __launch_bounds__(kBrickThreads) k_sparse_bricks(const __grid_co
     if (threadIdx.x == 0 && s_active) atomicAdd(P.counters + kScActiveBricks, (unsigned long long)s_active);
 }
 
-// Active-cell words (:321-377) in the dense path's layout: a warp per (cell row, 32 words),
-// lane w builds cell word w from the point words of the four point rows around it.
+// Active-cell words (:321-377) in the dense path's layout: a lane builds a cell word from the
+// point words of the four point rows around it. A warp takes 32 words of a cell row or, where
+// rows have at most 8 or 16 words, four or two rows.
 __global__ void __launch_bounds__(256) k_sparse_cells(const __grid_constant__ SparseParams P) {
     const GridDesc& g = P.g;
     const int lane = threadIdx.x & 31;
-    const long long nseg = (long long)g.cy * g.cz * P.nxt;
-    for (long long sg = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; sg < nseg;
-         sg += ((long long)gridDim.x * blockDim.x) >> 5) {
-        const long long row = sg / P.nxt;
+    const uint32_t nseg = (uint32_t)g.cy * g.cz * P.nxt;
+    const int lanes = g.W <= 8 ? 8 : g.W <= 16 ? 16 : 32, wl = lane & (lanes - 1);
+    const uint32_t per = 32 / lanes;
+    for (uint32_t s0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * per; s0 < nseg;
+         s0 += ((gridDim.x * blockDim.x) >> 5) * per) {                // warp-uniform
+        const uint32_t sg = s0 + lane / lanes;
+        const uint32_t row = P.nxt == 1 ? sg : sg / P.nxt;
         const int xt = (int)(sg - row * P.nxt);
-        const int j = (int)(row % g.cy), k = (int)(row / g.cy);
-        const int w = xt * 32 + lane;
+        const int k = (int)(row / g.cy), j = (int)(row - (uint32_t)k * g.cy);
+        const int w = sg < nseg ? xt * 32 + wl : g.W;
         uint32_t act = 0;
         if (w < g.W && 32 * w < g.cx) {
-            const long long r00 = ((long long)j + (long long)g.ny * k) * P.Wp;
-            const long long r10 = r00 + P.Wp, r01 = r00 + (long long)g.ny * P.Wp, r11 = r01 + P.Wp;
+            const size_t r00 = ((size_t)j + (size_t)g.ny * k) * P.Wp;
+            const size_t r10 = r00 + P.Wp, r01 = r00 + (size_t)g.ny * P.Wp, r11 = r01 + P.Wp;
             const bool nxw = w + 1 < P.Wp;
-            uint32_t m[3];
-            const uint32_t* src[3] = {P.pn, P.pp, P.pc};
-#pragma unroll
-            for (int q = 0; q < 3; ++q) {
-                const uint32_t* a = src[q];
+            // some corner of the cells in a word of points
+            auto corners = [&](const uint32_t* a) {
                 const uint32_t lo = __ldg(a + r00 + w) | __ldg(a + r10 + w) | __ldg(a + r01 + w) | __ldg(a + r11 + w);
                 const uint32_t hi = nxw ? (__ldg(a + r00 + w + 1) | __ldg(a + r10 + w + 1) | __ldg(a + r01 + w + 1) |
                                            __ldg(a + r11 + w + 1)) : 0u;
-                m[q] = lo | (lo >> 1) | (hi << 31);
-            }
-            act = (m[0] & m[1]) | m[2];
+                return lo | (lo >> 1) | (hi << 31);
+            };
+            // most words have no negative or no near-zero point: nothing more to load or to mask
+            const uint32_t neg = corners(P.pn), near = corners(P.pc);
+            act = near;
+            if (neg) act |= neg & corners(P.pp);
             const int c0 = 32 * w, c1 = min(32 * w + 32, g.cx);
             act &= range_bits(0, c1 - c0);
-            const int by = j / P.bs, bz = k / P.bs;
-            uint32_t bm = 0;
-            for (int bx = c0 / P.bs; bx * P.bs < c1; ++bx)
-                if (__ldg(P.brick + bx + (long long)P.nbx * (by + (long long)P.nby * bz)))
-                    bm |= range_bits(max(bx * P.bs, c0) - c0, min(bx * P.bs + P.bs, c1) - c0);
-            act &= bm;
+            if (act) {
+                const int by = j / P.bs, bz = k / P.bs;
+                uint32_t bm = 0;
+                for (int bx = c0 / P.bs; bx * P.bs < c1; ++bx)
+                    if (__ldg(P.brick + bx + (long long)P.nbx * (by + (long long)P.nby * bz)))
+                        bm |= range_bits(max(bx * P.bs, c0) - c0, min(bx * P.bs + P.bs, c1) - c0);
+                act &= bm;
+            }
         }
-        if (w < g.W) P.bits[row * g.W + w] = act;
+        if (w < g.W) P.bits[(size_t)row * g.W + w] = act;
         uint32_t cnt = __popc(act);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-        if (lane == 0) P.seg_count[row * P.nxt + xt] = cnt;
+        for (int o = lanes >> 1; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+        if (wl == 0 && sg < nseg) P.seg_count[sg] = cnt;
     }
 }
 
@@ -710,13 +685,12 @@ unsigned blocks_for(long long items, int threads, int num_sms, int per_sm) {
 
 cudaError_t launch_sparse_mark(const SparseParams& P, int num_sms, cudaStream_t s) {
     const long long chunks = (long long)P.g.ny * P.g.nz * ((P.Wp + 31) / 32);
-    const bool vec4 = P.g.nx % 4 == 0 && (reinterpret_cast<uintptr_t>(P.g.v) % 16) == 0;
-    if (vec4) k_sparse_points<true><<<blocks_for(chunks * 32, 256, num_sms, 16), 256, 0, s>>>(P);
-    else      k_sparse_points<false><<<blocks_for(chunks * 32, 256, num_sms, 16), 256, 0, s>>>(P);
+    k_sparse_points<<<blocks_for(chunks * 32, 256, num_sms, 16), 256, 0, s>>>(P);
     const long long nrow = (long long)P.nby * P.nbz;
     k_sparse_bricks<<<(unsigned)std::min<long long>(nrow, (long long)num_sms * 16), kBrickThreads, 0, s>>>(P);
     const long long nseg = (long long)P.g.cy * P.g.cz * P.nxt;
-    k_sparse_cells<<<blocks_for(nseg * 32, 256, num_sms, 16), 256, 0, s>>>(P);
+    const int lanes = P.g.W <= 8 ? 8 : P.g.W <= 16 ? 16 : 32;
+    k_sparse_cells<<<blocks_for(nseg * lanes, 256, num_sms, 16), 256, 0, s>>>(P);
     return cudaGetLastError();
 }
 
