@@ -770,7 +770,8 @@ int run_ours(dcb_context* h, const dcb_grid* in, const dcb_opts* o, cudaStream_t
 // The sparse (brick) backends (src/cuda/dc_cuda_sparse.cu:1171-1415) on one device grid:
 // point words -> bricks -> active-cell bits, scan + rank expansion, vertices (and, for the
 // multi-vertex variant, their scan and placement), faces into per-cell slots, scan,
-// compaction. Two host read-backs: the active-cell count and the vertex and face totals.
+// compaction. One host read-back at the end on the buffers of an earlier call; a first call, or
+// a grid with more active cells than those hold, reads the active count first.
 int run_sparse(dcb_context* h, const dcb_grid* in, const dcb_opts* o, cudaStream_t s, dcb_stats* st) {
     ++h->gen;
     if (o->emit_triangles) return fail(h, DCB_ERR_NOT_SUPPORTED, "the sparse backends emit quads only");
@@ -829,11 +830,56 @@ int run_sparse(dcb_context* h, const dcb_grid* in, const dcb_opts* o, cudaStream
     DCB_TRY(h, launch_scan(P.seg_count, nseg, as<uint32_t>(h->partials), as<uint32_t>(h->seg_start),
                            dcn + kScActiveCells, s), "launch segment scan");
     DCB_TRY(h, cudaEventRecord(h->ev[2], s), "event");
-    DCB_TRY(h, cudaMemcpyAsync(hcn, dcn, sizeof(unsigned long long) * kScSlots, cudaMemcpyDeviceToHost, s), "read counts");
-    DCB_TRY(h, cudaStreamSynchronize(s), "sparse mark");
-    const long long na = (long long)hcn[kScActiveCells];
-    if (na >= (mvdc ? 0x3fffffffLL : 0x7fffffffLL)) return fail(h, DCB_ERR_TOO_LARGE, "more than 2^31-1 vertices");
 
+    // 2) everything after the mark, for up to `cap` active cells and the buffers in place; with
+    // live, the kernels read the count on the device
+    auto rest = [&](long long cap, const unsigned long long* live) -> int {
+        plen = std::max(plen, scan_partials_len(cap));
+        DCB_TRY(h, ensure(h->partials, sizeof(uint32_t) * plen), "alloc scan");
+        ExpandParams xp{};
+        xp.B.s0 = S; xp.B.n = 1;
+        xp.nseg = nseg; xp.bits = P.bits; xp.seg_count = P.seg_count; xp.seg_start = as<uint32_t>(h->seg_start);
+        xp.super = P.super; xp.list = as<uint64_t>(h->list); xp.cell_slot = nullptr;
+        xp.list_cap = cap;
+        DCB_TRY(h, launch_expand(xp, h->num_sms, s), "launch expand");
+        P.list = xp.list;
+        P.nactive = cap;
+        P.live = live;
+        P.V = as<float>(h->V);
+        if (mvdc) {
+            P.vcount = as<uint32_t>(h->sp_vcount); P.vstart = as<uint32_t>(h->sp_vstart);
+            P.vtmp = as<float>(h->sp_vtmp); P.ntmp = as<float>(h->sp_ntmp);
+            P.N = as<float>(h->sp_N); P.vcell = as<uint64_t>(h->sp_vcell);
+        }
+        DCB_TRY(h, launch_sparse_vertices(P, h->num_sms, s), "launch sparse vertices");
+        if (mvdc) {
+            DCB_TRY(h, launch_scan(P.vcount, cap, as<uint32_t>(h->partials), as<uint32_t>(h->sp_vstart),
+                                   dcn + kScVertices, s, nullptr, live), "launch vertex scan");
+            DCB_TRY(h, launch_sparse_place(P, h->num_sms, s), "launch vertex placement");
+        }
+        DCB_TRY(h, cudaEventRecord(h->ev[3], s), "event");
+        // 3) faces: per-cell staging with counts, scan, compaction
+        P.fcount = as<uint32_t>(h->sp_fcount);
+        P.fslots = reinterpret_cast<uint8_t*>(P.fcount + cap);
+        P.fstart = as<uint32_t>(h->sp_fstart);
+        P.stage = as<int4>(h->sp_stage);
+        DCB_TRY(h, launch_sparse_faces(P, h->num_sms, s), "launch faces");
+        DCB_TRY(h, cudaEventRecord(h->ev[8], s), "event");
+        DCB_TRY(h, launch_scan(P.fcount, cap, as<uint32_t>(h->partials), as<uint32_t>(h->sp_fstart),
+                               dcn + kScFaces, s, nullptr, live), "launch face scan");
+        DCB_TRY(h, cudaEventRecord(h->ev[9], s), "event");
+        h->substage_events = true;
+        h->count_event = true;
+        P.faces = as<int4>(h->faces);
+        P.faces_cap = (long long)(h->faces.bytes / sizeof(int4));
+        DCB_TRY(h, launch_sparse_compact(P, h->num_sms, s), "launch face compaction");
+        return DCB_OK;
+    };
+    auto read_counters = [&](const char* what) -> int {
+        DCB_TRY(h, cudaMemcpyAsync(hcn, dcn, sizeof(unsigned long long) * kScSlots, cudaMemcpyDeviceToHost, s), what);
+        DCB_TRY(h, cudaStreamSynchronize(s), what);
+        return DCB_OK;
+    };
     h->last_kind = 1;
     h->cells_per_vertex = mvdc ? 1 : 0;
     h->nv = 0; h->nf = 0; h->vpf = 4;
@@ -841,29 +887,33 @@ int run_sparse(dcb_context* h, const dcb_grid* in, const dcb_opts* o, cudaStream
     h->batch_n = 1;
     h->vert_offsets.assign(2, 0);
     h->face_offsets.assign(2, 0);
+    // The buffers of an earlier call hold this many active cells (0 before the first): all is
+    // launched at once and the count read with the results; a larger grid runs again below.
+    long long cap = std::min((long long)(h->list.bytes / sizeof(uint64_t)), (long long)(h->sp_stage.bytes / (6 * sizeof(int4))));
+    auto lim = [&cap](const DevBuf& b, size_t per) { cap = std::min(cap, (long long)(b.bytes / per)); };
+    lim(h->V, (mvdc ? 6 : 3) * sizeof(float));
+    lim(h->sp_fcount, sizeof(uint32_t) + 1); lim(h->sp_fstart, sizeof(uint32_t));
+    if (mvdc) {
+        lim(h->sp_vcount, sizeof(uint32_t)); lim(h->sp_vstart, sizeof(uint32_t)); lim(h->sp_vtmp, 6 * sizeof(float));
+        lim(h->sp_ntmp, 6 * sizeof(float)); lim(h->sp_N, 6 * sizeof(float)); lim(h->sp_vcell, 2 * sizeof(uint64_t));
+    }
+    int rc = DCB_OK;
+    if (cap > 0 && (rc = rest(cap, dcn + kScActiveCells)) != DCB_OK) return rc;
+    if (cap > 0) DCB_TRY(h, cudaEventRecord(h->ev[4], s), "event");
+    if ((rc = read_counters("sparse mark")) != DCB_OK) return rc;
+    const long long na = (long long)hcn[kScActiveCells];
+    if (na >= (mvdc ? 0x3fffffffLL : 0x7fffffffLL)) return fail(h, DCB_ERR_TOO_LARGE, "more than 2^31-1 vertices");
     if (st) {
         st->nx = g.nx; st->ny = g.ny; st->nz = g.nz;
         st->total_cells = (long long)g.cx * crow; st->active_cells = na;
         st->total_bricks = nb;
     }
-    long long nverts = 0, nf = 0;
-    if (na > 0) {
-        // 2) ranks + list, vertices
+    if (na > 0 && na > cap) {
         DCB_TRY(h, ensure(h->list, sizeof(uint64_t) * na), "alloc active list");
         DCB_TRY(h, ensure(h->V, sizeof(float) * 3 * (mvdc ? 2 * na : na)), "alloc vertices");
         DCB_TRY(h, ensure(h->sp_fcount, (sizeof(uint32_t) + 1) * na), "alloc face counts");
         DCB_TRY(h, ensure(h->sp_fstart, sizeof(uint32_t) * na), "alloc face starts");
         DCB_TRY(h, ensure(h->sp_stage, sizeof(int4) * 6 * na), "alloc face staging");
-        plen = std::max(plen, scan_partials_len(na));
-        DCB_TRY(h, ensure(h->partials, sizeof(uint32_t) * plen), "alloc scan");
-        ExpandParams xp{};
-        xp.B.s0 = S; xp.B.n = 1;
-        xp.nseg = nseg; xp.bits = P.bits; xp.seg_count = P.seg_count; xp.seg_start = as<uint32_t>(h->seg_start);
-        xp.super = P.super; xp.list = as<uint64_t>(h->list); xp.cell_slot = nullptr;
-        DCB_TRY(h, launch_expand(xp, h->num_sms, s), "launch expand");
-        P.list = xp.list;
-        P.nactive = na;
-        P.V = as<float>(h->V);
         if (mvdc) {
             DCB_TRY(h, ensure(h->sp_vcount, sizeof(uint32_t) * na), "alloc vertex counts");
             DCB_TRY(h, ensure(h->sp_vstart, sizeof(uint32_t) * na), "alloc vertex starts");
@@ -871,43 +921,26 @@ int run_sparse(dcb_context* h, const dcb_grid* in, const dcb_opts* o, cudaStream
             DCB_TRY(h, ensure(h->sp_ntmp, sizeof(float) * 6 * na), "alloc normal staging");
             DCB_TRY(h, ensure(h->sp_N, sizeof(float) * 6 * na), "alloc vertex normals");
             DCB_TRY(h, ensure(h->sp_vcell, sizeof(uint64_t) * 2 * na), "alloc vertex cells");
-            P.vcount = as<uint32_t>(h->sp_vcount); P.vstart = as<uint32_t>(h->sp_vstart);
-            P.vtmp = as<float>(h->sp_vtmp); P.ntmp = as<float>(h->sp_ntmp);
-            P.N = as<float>(h->sp_N); P.vcell = as<uint64_t>(h->sp_vcell);
         }
-        DCB_TRY(h, launch_sparse_vertices(P, h->num_sms, s), "launch sparse vertices");
-        if (mvdc) {
-            DCB_TRY(h, launch_scan(P.vcount, na, as<uint32_t>(h->partials), as<uint32_t>(h->sp_vstart),
-                                   dcn + kScVertices, s), "launch vertex scan");
-            DCB_TRY(h, launch_sparse_place(P, h->num_sms, s), "launch vertex placement");
-        }
+        if ((rc = rest(na, nullptr)) != DCB_OK) return rc;
+        DCB_TRY(h, cudaEventRecord(h->ev[4], s), "event");
+        if ((rc = read_counters("sparse vertices")) != DCB_OK) return rc;
+    } else if (cap <= 0) {
         DCB_TRY(h, cudaEventRecord(h->ev[3], s), "event");
-        // 3) faces: per-cell staging with counts, scan, compaction
-        P.fcount = as<uint32_t>(h->sp_fcount);
-        P.fslots = reinterpret_cast<uint8_t*>(P.fcount + na);
-        P.fstart = as<uint32_t>(h->sp_fstart);
-        P.stage = as<int4>(h->sp_stage);
-        DCB_TRY(h, launch_sparse_faces(P, h->num_sms, s), "launch faces");
-        DCB_TRY(h, cudaEventRecord(h->ev[8], s), "event");
-        DCB_TRY(h, launch_scan(P.fcount, na, as<uint32_t>(h->partials), as<uint32_t>(h->sp_fstart),
-                               dcn + kScFaces, s), "launch face scan");
-        DCB_TRY(h, cudaEventRecord(h->ev[9], s), "event");
-        h->substage_events = true;
-        h->count_event = true;
-        DCB_TRY(h, cudaMemcpyAsync(hcn, dcn, sizeof(unsigned long long) * kScSlots, cudaMemcpyDeviceToHost, s), "read totals");
-        DCB_TRY(h, cudaStreamSynchronize(s), "sparse vertices");
-        nverts = mvdc ? (long long)hcn[kScVertices] : na;
-        nf = (long long)hcn[kScFaces];
-        if (nf >= 0x7fffffffLL) return fail(h, DCB_ERR_TOO_LARGE, "more than 2^31-1 faces");
-        DCB_TRY(h, ensure(h->faces, sizeof(int4) * std::max(1LL, nf)), "alloc faces");
-        P.faces = as<int4>(h->faces);
-        DCB_TRY(h, launch_sparse_compact(P, h->num_sms, s), "launch face compaction");
-    } else {
-        DCB_TRY(h, cudaEventRecord(h->ev[3], s), "event");
+        DCB_TRY(h, cudaEventRecord(h->ev[4], s), "event");
+        DCB_TRY(h, cudaStreamSynchronize(s), "sparse mark");
     }
-    DCB_TRY(h, cudaEventRecord(h->ev[4], s), "event");
-    DCB_TRY(h, cudaMemcpyAsync(hcn, dcn, sizeof(unsigned long long) * kScSlots, cudaMemcpyDeviceToHost, s), "read counters");
-    DCB_TRY(h, cudaStreamSynchronize(s), "sparse faces");
+    const long long nverts = mvdc ? (long long)hcn[kScVertices] : na;
+    const long long nf = na > 0 ? (long long)hcn[kScFaces] : 0;
+    if (nf >= 0x7fffffffLL) return fail(h, DCB_ERR_TOO_LARGE, "more than 2^31-1 faces");
+    if ((size_t)nf * sizeof(int4) > h->faces.bytes) {          // the faces wait in their staging slots
+        DCB_TRY(h, ensure(h->faces, sizeof(int4) * nf), "alloc faces");
+        P.faces = as<int4>(h->faces);
+        P.faces_cap = nf;
+        DCB_TRY(h, launch_sparse_compact(P, h->num_sms, s), "launch face compaction");
+        DCB_TRY(h, cudaEventRecord(h->ev[4], s), "event");
+        DCB_TRY(h, cudaStreamSynchronize(s), "sparse faces");
+    }
     h->nv = nverts;
     h->nf = nf;
     h->vert_offsets[1] = nverts;

@@ -84,8 +84,14 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* s_warp
     return base + incl - v;
 }
 
+// The counts to scan: n, or the device's number of them (none when they exceed n).
+__device__ __forceinline__ long long scan_length(long long n, const unsigned long long* live) {
+    return !live ? n : (long long)*live > n ? 0 : (long long)*live;
+}
+
 __global__ void __launch_bounds__(kScanThreads)
-k_scan_partials(const uint32_t* __restrict__ in, long long n, uint32_t* partials) {
+k_scan_partials(const uint32_t* __restrict__ in, long long n, const unsigned long long* live, uint32_t* partials) {
+    n = scan_length(n, live);
     __shared__ uint32_t s_warp[kScanThreads / 32];
     const long long base = (long long)blockIdx.x * kScanTile + (long long)threadIdx.x * kScanItems;
     uint32_t v[kScanItems], s = 0;
@@ -116,8 +122,9 @@ k_scan_single(uint32_t* partials, long long nb, unsigned long long* grand_total)
 // the last one knows the total.
 template <bool SUMMED>
 __global__ void __launch_bounds__(kScanThreads)
-k_scan_apply(const uint32_t* __restrict__ in, long long n, const uint32_t* __restrict__ partials,
+k_scan_apply(const uint32_t* __restrict__ in, long long n, const unsigned long long* live, const uint32_t* __restrict__ partials,
              uint32_t* __restrict__ out, uint32_t* __restrict__ copy, unsigned long long* grand_total) {
+    n = scan_length(n, live);
     __shared__ uint32_t s_warp[kScanThreads / 32];
     const long long base = (long long)blockIdx.x * kScanTile + (long long)threadIdx.x * kScanItems;
     uint32_t before = 0;
@@ -142,8 +149,9 @@ k_scan_apply(const uint32_t* __restrict__ in, long long n, const uint32_t* __res
 }
 
 __global__ void __launch_bounds__(kScanOneThreads)
-k_scan_one(const uint32_t* __restrict__ in, long long n, uint32_t* __restrict__ out, uint32_t* __restrict__ copy,
-           unsigned long long* grand_total) {
+k_scan_one(const uint32_t* __restrict__ in, long long n, const unsigned long long* live, uint32_t* __restrict__ out,
+           uint32_t* __restrict__ copy, unsigned long long* grand_total) {
+    n = scan_length(n, live);
     __shared__ uint32_t s_warp[kScanOneThreads / 32];
     uint32_t carry = 0;
     for (long long c0 = 0; c0 < n; c0 += kScanOneThreads * kScanOneItems) {
@@ -164,19 +172,19 @@ k_scan_one(const uint32_t* __restrict__ in, long long n, uint32_t* __restrict__ 
 }
 
 cudaError_t launch_scan(const uint32_t* in, long long n, uint32_t* partials, uint32_t* out,
-                        unsigned long long* grand_total, cudaStream_t s, uint32_t* copy) {
+                        unsigned long long* grand_total, cudaStream_t s, uint32_t* copy, const unsigned long long* live) {
     const long long nb = (n + kScanTile - 1) / kScanTile;
     if (nb <= 0) return cudaSuccess;
     if (n <= kScanOne) {
-        k_scan_one<<<1, kScanOneThreads, 0, s>>>(in, n, out, copy, grand_total);
+        k_scan_one<<<1, kScanOneThreads, 0, s>>>(in, n, live, out, copy, grand_total);
         return cudaGetLastError();
     }
-    k_scan_partials<<<(unsigned)nb, kScanThreads, 0, s>>>(in, n, partials);
+    k_scan_partials<<<(unsigned)nb, kScanThreads, 0, s>>>(in, n, live, partials);
     if (nb <= kScanFew) {
-        k_scan_apply<false><<<(unsigned)nb, kScanThreads, 0, s>>>(in, n, partials, out, copy, grand_total);
+        k_scan_apply<false><<<(unsigned)nb, kScanThreads, 0, s>>>(in, n, live, partials, out, copy, grand_total);
     } else {
         k_scan_single<<<1, kScanThreads, 0, s>>>(partials, nb, grand_total);
-        k_scan_apply<true><<<(unsigned)nb, kScanThreads, 0, s>>>(in, n, partials, out, copy, nullptr);
+        k_scan_apply<true><<<(unsigned)nb, kScanThreads, 0, s>>>(in, n, live, partials, out, copy, nullptr);
     }
     return cudaGetLastError();
 }

@@ -182,9 +182,11 @@ struct Winding64Params {
 };
 cudaError_t launch_winding_fp64(const Winding64Params& P, long long max_items, int num_sms, cudaStream_t s);
 
-// Exclusive sums of n counts into out and, if given, copy; their total.
+// Exclusive sums of n counts into out and, if given, copy; their total. live: the number of
+// counts on the device, at most n (more: nothing is scanned, the total is 0).
 cudaError_t launch_scan(const uint32_t* in, long long n, uint32_t* partials, uint32_t* out,
-                        unsigned long long* grand_total, cudaStream_t s, uint32_t* copy = nullptr);
+                        unsigned long long* grand_total, cudaStream_t s, uint32_t* copy = nullptr,
+                        const unsigned long long* live = nullptr);
 long long scan_partials_len(long long n);
 
 struct FaceParams {
@@ -430,7 +432,8 @@ struct SparseParams {
     uint32_t* super;               // [cy*cz][W8] ranks (after the rank expansion)
     uint32_t* seg_count;           // [cy*cz][nxt]
     const uint64_t* list;          // [nactive] packed active cells, ascending
-    long long nactive;
+    long long nactive;             // active cells (capacity when live is set)
+    const unsigned long long* live; // device count of active cells (above nactive nothing is processed), or null
     uint32_t* vcount;              // multi-vertex: [nactive] vertices of the cell (1 or 2)
     const uint32_t* vstart;        // multi-vertex: [nactive] first vertex (scan of vcount)
     float* vtmp;                   // multi-vertex: [nactive][2][3] vertices before placing
@@ -443,6 +446,7 @@ struct SparseParams {
     const uint32_t* fstart;        // [nactive] first face (scan of fcount)
     int4* stage;                   // [nactive][6] faces of each cell before the scan
     int4* faces;
+    long long faces_cap;           // entries of faces (more faces: none is placed)
     unsigned long long* counters;  // [kScSlots], indexed by SparseCounter
 };
 cudaError_t launch_sparse_mark(const SparseParams& P, int num_sms, cudaStream_t s);

@@ -245,6 +245,10 @@ __device__ __forceinline__ float3 unit_or(float3 a, float3 fb) {
     return l > 1e-6f ? mul3(1.0f / l, a) : fb;
 }
 
+__device__ __forceinline__ long long live_cells(const SparseParams& P) {
+    return !P.live ? P.nactive : (long long)*P.live > P.nactive ? 0 : (long long)*P.live;
+}
+
 // Active-cell bit of cell (i,j,k) and its rank.
 __device__ __forceinline__ bool cell_active(const SparseParams& P, int i, int j, int k) {
     const uint32_t w = __ldg(P.bits + ((int64_t)j + (int64_t)P.g.cy * k) * P.g.W + (i >> 5));
@@ -418,14 +422,15 @@ __global__ void __launch_bounds__(32 * kSparseWarps) k_sparse_vertices(const __g
     __shared__ SparseWarp s_warp[kSparseWarps];
     if (threadIdx.x < kScCount) s_cnt[threadIdx.x] = 0;
     __syncthreads();
+    const long long nact = live_cells(P);
     const GridDesc& g = P.g;
     const float3 half = mul3(0.5f, f3(g.vx, g.vy, g.vz));
     const int lane = threadIdx.x & 31;
     SparseWarp& W = s_warp[threadIdx.x >> 5];
-    for (long long base = (long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < P.nactive;
+    for (long long base = (long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < nact;
          base += (long long)gridDim.x * blockDim.x) {                 // warp-uniform
         const long long r = base + lane;
-        const bool mine = r < P.nactive;
+        const bool mine = r < nact;
         int i = 0, j = 0, k = 0;
         uint32_t cross = 0, cand = 0;
         __syncwarp();
@@ -556,7 +561,8 @@ __global__ void __launch_bounds__(32 * kSparseWarps) k_sparse_vertices(const __g
 // Multi-vertex variant: each cell's vertices (and normals, and the cell of each vertex) at
 // their scanned positions.
 __global__ void __launch_bounds__(256) k_sparse_place(const __grid_constant__ SparseParams P) {
-    for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < P.nactive;
+    const long long nact = live_cells(P);
+    for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < nact;
          r += (long long)gridDim.x * blockDim.x) {
         const uint32_t st = P.vstart[r], c = P.vcount[r];
         const uint64_t cell = P.list[r];
@@ -585,15 +591,16 @@ __global__ void __launch_bounds__(32 * kSparseWarps) k_sparse_faces(const __grid
     __shared__ uint32_t s_slots[kSparseWarps][32], s_missing[kSparseWarps][32];
     if (threadIdx.x == 0) s_skipped = 0;
     __syncthreads();
+    const long long nact = live_cells(P);
     const GridDesc& g = P.g;
     const int lane = threadIdx.x & 31, wb = threadIdx.x >> 5;
-    for (long long base = (long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < P.nactive;
+    for (long long base = (long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < nact;
          base += (long long)gridDim.x * blockDim.x) {                 // warp-uniform
         const long long r = base + lane;
         int i = 0, j = 0, k = 0;
         float s0 = 0.f;
         uint32_t edges = 0, sure = 0;
-        if (r < P.nactive) {
+        if (r < nact) {
             unpack_cell(P.list[r], i, j, k);
             s0 = sval(g, i, j, k);
 #pragma unroll
@@ -651,7 +658,7 @@ __global__ void __launch_bounds__(32 * kSparseWarps) k_sparse_faces(const __grid
             atomicOr(&s_slots[wb][src], (crossed ? 1u : 3u) << (2 * axis));
         }
         __syncwarp();
-        if (r < P.nactive) {
+        if (r < nact) {
             const uint32_t slots = s_slots[wb][lane], missing = s_missing[wb][lane];
             P.fslots[r] = (uint8_t)slots;
             P.fcount[r] = __popc(slots);
@@ -665,7 +672,9 @@ __global__ void __launch_bounds__(32 * kSparseWarps) k_sparse_faces(const __grid
 
 // Each cell's staged faces, in slot order, to their scanned positions.
 __global__ void __launch_bounds__(256) k_sparse_compact(const __grid_constant__ SparseParams P) {
-    for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < P.nactive;
+    const long long nact = live_cells(P);
+    if ((long long)P.counters[kScFaces] > P.faces_cap) return;        // the host places them once it has room
+    for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < nact;
          r += (long long)gridDim.x * blockDim.x) {
         uint32_t at = P.fstart[r];
         for (uint32_t m = P.fslots[r]; m; m &= m - 1) P.faces[at++] = P.stage[6 * r + __ffs(m) - 1];
