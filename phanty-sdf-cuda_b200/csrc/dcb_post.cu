@@ -70,6 +70,9 @@ struct PostCounters {
     unsigned long long nout;            // vertices after renumbering
     unsigned long long cursor;          // ring vertices reserved in the fill scratch
     unsigned long long nrings;          // ring records written
+    unsigned int nlong;                 // vertices with long edge buckets
+    unsigned int ntoo_long;             // of them beyond what a block compares
+    int linked[8];                      // round r of the face links changed something
     int fill_overflow;                  // the scratch or the record list was too small
     int pad3;
 };
@@ -125,7 +128,8 @@ __global__ void k_iota(int* a, long long n) {
 // After all unions: every parent becomes its root. The walk up only reads (a path-halving
 // write here could replace a root that another thread just stored with an intermediate
 // ancestor); the only writes are roots.
-__global__ void k_flatten(int* parent, long long n) {
+__global__ void k_flatten(int* parent, long long n, const int* wanted = nullptr) {
+    if (wanted && !*wanted) return;
     volatile int* p = parent;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         int x = (int)i, up;
@@ -182,8 +186,18 @@ __global__ void k_weld_params(PostCounters* C) {
     for (int a = 0; a < 3; ++a) C->qlo[a] = (long long)roundf(lo[a] * inv);
 }
 
-__global__ void k_weld_keys(const float* __restrict__ V, long long nv, PostCounters* C,
-                            unsigned long long* key, int* idx) {
+// Vertices of one grid key are welded to the first of them, and the welded ones are numbered in
+// index order. A hash table (linear probing, at most half full) holds every key with its smallest
+// index; vertices of a mesh come in nearly that order, so most keep the entry they find without
+// an atomic. (A radix sort of the 51-bit keys took seven passes of five launches each.)
+__device__ __forceinline__ unsigned long long mix_key(unsigned long long x) {     // finaliser of SplitMix64
+    x = (x ^ (x >> 30)) * 0xbf58476d1ce4e5b9ull;
+    x = (x ^ (x >> 27)) * 0x94d049bb133111ebull;
+    return x ^ (x >> 31);
+}
+
+__global__ void k_weld_insert(const float* __restrict__ V, long long nv, PostCounters* C, unsigned long long* table,
+                              unsigned int* first, unsigned int mask, unsigned int* slot) {
     const float inv = C->inv;
     const long long q0 = C->qlo[0], q1 = C->qlo[1], q2 = C->qlo[2];
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nv; i += (long long)gridDim.x * blockDim.x) {
@@ -192,42 +206,41 @@ __global__ void k_weld_keys(const float* __restrict__ V, long long nv, PostCount
         const long long d2 = (long long)roundf(V[3 * i + 2] * inv) - q2;
         const long long lim = 1LL << kKeyBits;
         if (d0 < 0 || d0 >= lim || d1 < 0 || d1 >= lim || d2 < 0 || d2 >= lim) atomicOr(&C->err, kPostWeldSpan);
-        key[i] = ((unsigned long long)(d0 & (lim - 1))) | ((unsigned long long)(d1 & (lim - 1)) << kKeyBits) |
-                 ((unsigned long long)(d2 & (lim - 1)) << (2 * kKeyBits));
-        idx[i] = (int)i;
+        const unsigned long long key = ((unsigned long long)(d0 & (lim - 1))) | ((unsigned long long)(d1 & (lim - 1)) << kKeyBits) |
+                                       ((unsigned long long)(d2 & (lim - 1)) << (2 * kKeyBits));
+        unsigned int h = (unsigned int)mix_key(key) & mask;
+        for (;;) {                                       // ends: more slots than keys
+            unsigned long long have = __ldcg(table + h);
+            if (have == ~0ull) have = atomicCAS(table + h, ~0ull, key);
+            if (have == ~0ull || have == key) break;
+            h = (h + 1) & mask;
+        }
+        if (__ldcg(first + h) > (unsigned int)i) atomicMin(first + h, (unsigned int)i);
+        slot[i] = h;
     }
 }
 
-// head[p]: sorted position p starts a key; rep[i]: vertex i is the first of its key.
-__global__ void k_weld_heads(const unsigned long long* __restrict__ skey, const int* __restrict__ sidx, long long n,
-                             unsigned int* head, unsigned int* rep) {
-    for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
-        const unsigned int h = (p == 0 || skey[p] != skey[p - 1]) ? 1u : 0u;
-        head[p] = h;
-        rep[sidx[p]] = h;
-    }
+// rep[i]: vertex i is the first of its key.
+__global__ void k_weld_reps(const unsigned int* __restrict__ slot, const unsigned int* __restrict__ first, long long nv,
+                            unsigned int* rep) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nv; i += (long long)gridDim.x * blockDim.x)
+        rep[i] = first[slot[i]] == (unsigned int)i ? 1u : 0u;
 }
 
-// group g (1-based inclusive scan of heads) -> new index of its representative; welded vertices.
-__global__ void k_weld_groups(const int* __restrict__ sidx, const unsigned int* __restrict__ head,
-                              const unsigned int* __restrict__ gid, const unsigned int* __restrict__ newid,
-                              const float* __restrict__ V, long long n, unsigned int* grp, float* Vw, PostCounters* C) {
-    for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
-        if (p == n - 1) C->nvw = gid[p];
-        if (!head[p]) continue;
-        const int i = sidx[p];
-        const unsigned int nid = newid[i];
-        grp[gid[p] - 1] = nid;
-        Vw[3 * (long long)nid] = V[3 * (long long)i];
-        Vw[3 * (long long)nid + 1] = V[3 * (long long)i + 1];
-        Vw[3 * (long long)nid + 2] = V[3 * (long long)i + 2];
+// newid: exclusive scan of rep. The welded vertices, and every vertex's new index.
+__global__ void k_weld_place(const unsigned int* __restrict__ slot, const unsigned int* __restrict__ first,
+                             const unsigned int* __restrict__ newid, const float* __restrict__ V, long long nv, int* remap,
+                             float* Vw, PostCounters* C) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nv; i += (long long)gridDim.x * blockDim.x) {
+        const unsigned int f = first[slot[i]], nid = newid[f];
+        remap[i] = (int)nid;
+        if (f == (unsigned int)i) {
+            Vw[3 * (long long)nid] = V[3 * i];
+            Vw[3 * (long long)nid + 1] = V[3 * i + 1];
+            Vw[3 * (long long)nid + 2] = V[3 * i + 2];
+        }
+        if (i == nv - 1) C->nvw = (unsigned long long)newid[i] + (f == (unsigned int)i ? 1u : 0u);
     }
-}
-
-__global__ void k_weld_remap(const int* __restrict__ sidx, const unsigned int* __restrict__ gid,
-                             const unsigned int* __restrict__ grp, long long n, int* remap) {
-    for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x)
-        remap[sidx[p]] = (int)grp[gid[p] - 1];
 }
 
 __global__ void k_weld_faces(const int32_t* __restrict__ F, long long nf, long long nv, const int* __restrict__ remap,
@@ -303,6 +316,111 @@ __global__ void k_edge_runs(EdgeRunParams P) {
         } else if (P.close && P.remove) {
             for (long long x = p; x < q; ++x) push_boundary(P, P.val[x]);
         }
+    }
+}
+
+// ---- the same from buckets: edge uses grouped by the edge's smaller vertex (about four a vertex on
+// a mesh), so that a thread finds the runs among its vertex's few uses. A radix sort of the
+// uses by both vertices took six passes of five launches (512^3 CSG: 0.9 ms). No order of the runs
+// or in them reaches the output. Vertices with more than kBucketFew uses are taken by a block each;
+// beyond kBucketMany the sorted form above serves the whole mesh.
+constexpr unsigned int kBucketFew = 32, kBucketMany = 8192;
+
+struct BucketParams {
+    const int4* Fw;
+    long long nf, nv;
+    unsigned int *count, *fill;         // [nv] uses by smaller vertex; placed so far
+    const unsigned int* start;          // [nv] exclusive scan of count
+    uint2* use;                         // larger vertex, use (face << 2 | corner), by bucket
+    int2* pair;                         // per use: the faces of a two-use edge at its first use, else (-1, -1)
+    unsigned int* longs;                // vertices with long buckets
+    int* parent;
+    PostCounters* C;
+};
+
+template <bool PLACE>
+__global__ void k_bucket_uses(BucketParams P) {
+    for (long long f = blockIdx.x * (long long)blockDim.x + threadIdx.x; f < P.nf; f += (long long)gridDim.x * blockDim.x) {
+        const int4 q = P.Fw[f];
+        for (int e = 0; e < 4; ++e) {
+            const int u = corner(q, e), v = corner(q, (e + 1) & 3);
+            if (u == v) continue;
+            const int lo = min(u, v);
+            if (PLACE) P.use[P.start[lo] + atomicAdd(P.fill + lo, 1u)] = make_uint2((unsigned int)max(u, v), (unsigned int)(f << 2 | e));
+            else atomicAdd(P.count + lo, 1u);
+        }
+    }
+}
+
+// Use x of a bucket: what its edge's run asks for, if x is the run's first use.
+__device__ __forceinline__ void bucket_use(const BucketParams& P, const EdgeRunParams& E, const uint2* use, int2* pair,
+                                           unsigned int n, unsigned int x) {
+    const unsigned int v = use[x].x;
+    unsigned int c = 0, second = 0;
+    for (unsigned int y = 0; y < n; ++y) {
+        if (use[y].x != v) continue;
+        if (y < x) { pair[x] = make_int2(-1, -1); return; }
+        if (++c == 2) second = y;
+    }
+    int2 both = make_int2(-1, -1);
+    if (c == 1) {
+        push_boundary(E, (int)use[x].y);
+    } else if (c == 2) {
+        both = make_int2((int)(use[x].y >> 2), (int)(use[second].y >> 2));
+        if (E.remove && both.x != both.y) atomicMin(&P.parent[max(both.x, both.y)], min(both.x, both.y));
+    } else if (E.close && E.remove) {
+        for (unsigned int y = x; y < n; ++y)
+            if (use[y].x == v) push_boundary(E, (int)use[y].y);
+    }
+    pair[x] = both;
+}
+
+__global__ void k_bucket_runs(BucketParams P, EdgeRunParams E) {
+    for (long long u = blockIdx.x * (long long)blockDim.x + threadIdx.x; u < P.nv; u += (long long)gridDim.x * blockDim.x) {
+        const unsigned int n = P.count[u], at = P.start[u];
+        if (n > kBucketFew) {
+            P.longs[atomicAdd(&P.C->nlong, 1u)] = (unsigned int)u;
+            if (n > kBucketMany) atomicAdd(&P.C->ntoo_long, 1u);
+            continue;
+        }
+        for (unsigned int x = 0; x < n; ++x) bucket_use(P, E, P.use + at, P.pair + at, n, x);
+    }
+}
+
+__global__ void k_bucket_long(BucketParams P, EdgeRunParams E) {
+    for (unsigned int w = blockIdx.x; w < P.C->nlong; w += gridDim.x) {
+        const unsigned int u = P.longs[w], n = P.count[u], at = P.start[u];
+        if (n > kBucketMany) continue;
+        for (unsigned int x = threadIdx.x; x < n; x += blockDim.x) bucket_use(P, E, P.use + at, P.pair + at, n, x);
+    }
+}
+
+// Face components from the pairs. With every parent a root (k_flatten), a round links the larger
+// root of each pair to the smallest root it meets; rounds and flattenings alternate, and what
+// is left after kLinkRounds is united one by one. Linking pairs as they come, each with its own
+// finds in a growing forest, took 1.24 ms for 3M pairs of the 512^3 CSG mesh (3% issue,
+// 300 cycles a load).
+constexpr int kLinkRounds = 6;
+__global__ void k_pair_link(const int2* __restrict__ pair, long long n, int* parent, PostCounters* C, int round) {
+    if (round > 0 && !C->linked[round - 1]) return;
+    bool any = false;
+    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
+        const int2 q = pair[t];
+        if (q.x < 0) continue;
+        const int a = __ldcg(parent + q.x), b = __ldcg(parent + q.y);
+        if (a == b) continue;
+        const int hi = max(a, b), lo = min(a, b);
+        if (__ldcg(parent + hi) > lo) atomicMin(parent + hi, lo);
+        any = true;
+    }
+    if (__any_sync(0xffffffffu, any) && (threadIdx.x & 31) == 0) C->linked[round] = 1;
+}
+
+__global__ void k_pair_unite(const int2* __restrict__ pair, long long n, int* parent, PostCounters* C) {
+    if (!C->linked[kLinkRounds - 1]) return;
+    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
+        const int2 q = pair[t];
+        if (q.x >= 0 && __ldcg(parent + q.x) != __ldcg(parent + q.y)) uf_unite(parent, q.x, q.y, &C->err);
     }
 }
 
@@ -912,11 +1030,11 @@ const PostCounters& host_counters(const PostWork& W) { return *reinterpret_cast<
 cudaError_t weld(PostWork& W, PostRun& R, const float* V, long long nv, const int32_t* F, long long nf, PostBuf& Vout,
                  PostBuf& Fout, long long& nvw, long long& nfw, int sms, cudaStream_t s) {
     PostCounters* C = as<PostCounters>(W.count);
-    PP_TRY(grow(W.key, sizeof(unsigned long long) * nv));
-    PP_TRY(grow(W.key2, sizeof(unsigned long long) * nv));
+    size_t slots = 1024;
+    while (slots < 2 * (size_t)nv) slots *= 2;
+    PP_TRY(grow(W.key, sizeof(unsigned long long) * slots));       // the table's keys
+    PP_TRY(grow(W.u0, sizeof(unsigned int) * slots));              // and their first vertices
     PP_TRY(grow(W.val, sizeof(int) * nv));
-    PP_TRY(grow(W.val2, sizeof(int) * nv));
-    PP_TRY(grow(W.u0, sizeof(unsigned int) * nv));
     PP_TRY(grow(W.u1, sizeof(unsigned int) * nv));
     PP_TRY(grow(W.u2, sizeof(unsigned int) * nv));
     PP_TRY(grow(W.u3, sizeof(unsigned int) * nv));
@@ -924,29 +1042,19 @@ cudaError_t weld(PostWork& W, PostRun& R, const float* V, long long nv, const in
     PP_TRY(grow(W.flag8, nf));
     PP_TRY(grow(Vout, sizeof(float) * 3 * nv));
     PP_TRY(grow(Fout, sizeof(int4) * nf));
-    size_t t0 = 0, t1 = 0, t2 = 0;
-    t0 = radix_sort_temp_bytes(nv, 8, true);
-    t1 = scan_temp_bytes(nv);
-    t2 = select_temp_bytes(nf);
-    const size_t tb = std::max(t0, std::max(t1, t2));
-    PP_TRY(grow(W.scratch, tb));
+    PP_TRY(grow(W.scratch, std::max(scan_temp_bytes(nv), select_temp_bytes(nf))));
     const unsigned g = grid_for(nv, kThreads, sms);
     k_post_reset<<<1, 32, 0, s>>>(C);
     k_bbox<<<g, kThreads, 0, s>>>(V, nv, C);
     k_weld_params<<<1, 32, 0, s>>>(C);
-    k_weld_keys<<<g, kThreads, 0, s>>>(V, nv, C, as<unsigned long long>(W.key), as<int>(W.val));
+    PP_TRY(cudaMemsetAsync(W.key.p, 0xff, sizeof(unsigned long long) * slots, s));
+    PP_TRY(cudaMemsetAsync(W.u0.p, 0xff, sizeof(unsigned int) * slots, s));
+    unsigned int *first = as<unsigned int>(W.u0), *rep = as<unsigned int>(W.u1), *newid = as<unsigned int>(W.u2), *slot = as<unsigned int>(W.u3);
+    k_weld_insert<<<g, kThreads, 0, s>>>(V, nv, C, as<unsigned long long>(W.key), first, (unsigned int)(slots - 1), slot);
+    k_weld_reps<<<g, kThreads, 0, s>>>(slot, first, nv, rep);
     PP_TRY(cudaGetLastError());
-    PP_TRY(radix_sort_pairs(W.scratch.p, W.scratch.bytes, as<unsigned long long>(W.key),
-                            as<unsigned long long>(W.key2), as<uint32_t>(W.val), as<uint32_t>(W.val2), nv, 0, 3 * kKeyBits, s));
-    k_weld_heads<<<g, kThreads, 0, s>>>(as<unsigned long long>(W.key2), as<int>(W.val2), nv, as<unsigned int>(W.u0),
-                                        as<unsigned int>(W.u1));
-    PP_TRY(exclusive_sum(W.scratch.p, W.scratch.bytes, as<unsigned int>(W.u1), as<unsigned int>(W.u2), nv, s));
-    PP_TRY(inclusive_sum(W.scratch.p, W.scratch.bytes, as<unsigned int>(W.u0), as<unsigned int>(W.u3), nv, s));
-    // u0 head, u3 group (1-based), u2 new index of representatives; u1 -> group's new index
-    k_weld_groups<<<g, kThreads, 0, s>>>(as<int>(W.val2), as<unsigned int>(W.u0), as<unsigned int>(W.u3),
-                                         as<unsigned int>(W.u2), V, nv, as<unsigned int>(W.u1), as<float>(Vout), C);
-    k_weld_remap<<<g, kThreads, 0, s>>>(as<int>(W.val2), as<unsigned int>(W.u3), as<unsigned int>(W.u1), nv,
-                                        as<int>(W.val));
+    PP_TRY(exclusive_sum(W.scratch.p, W.scratch.bytes, rep, newid, nv, s));
+    k_weld_place<<<g, kThreads, 0, s>>>(slot, first, newid, V, nv, as<int>(W.val), as<float>(Vout), C);
     k_weld_faces<<<grid_for(nf, kThreads, sms), kThreads, 0, s>>>(F, nf, nv, as<int>(W.val), as<int4>(W.ft),
                                                                    as<unsigned char>(W.flag8), C);
     PP_TRY(cudaGetLastError());
@@ -1009,55 +1117,98 @@ cudaError_t post_run(PostWork& W, PostRun& R, cudaStream_t s) {
     R.stats[kPostWeldedFaces] = nfw;
     if (nvw == 0 || nfw == 0) return passthrough();
 
-    // edges: uses sorted by undirected key; runs -> boundary edges and face unions
+    // edges: uses grouped by undirected edge -> boundary edges and face unions
     const int b = bits_for(nvw);
     const long long ne = 4 * nfw;
     const unsigned long long inval = (b >= 32) ? ~0ull : ((1ull << (2 * b)) - 1);
     PP_TRY(grow(W.key, sizeof(unsigned long long) * ne));
     PP_TRY(grow(W.key2, sizeof(unsigned long long) * ne));
-    PP_TRY(grow(W.val, sizeof(int) * ne));
-    PP_TRY(grow(W.val2, sizeof(int) * ne));
     PP_TRY(grow(W.bnd, sizeof(int4) * ne));
     PP_TRY(grow(W.parent, sizeof(int) * nfw));
     PP_TRY(grow(W.csize, sizeof(unsigned int) * nfw));
     PP_TRY(grow(W.kept, sizeof(int4) * nfw));
     PP_TRY(grow(W.flag8, nfw));
-    {
-        size_t t0 = 0, t1 = 0;
-        t0 = radix_sort_temp_bytes(ne, 8, true);
-        t1 = select_temp_bytes(nfw);
-        PP_TRY(grow(W.scratch, std::max(t0, t1)));
-    }
+    PP_TRY(grow(W.u0, sizeof(unsigned int) * nvw));
+    PP_TRY(grow(W.u1, sizeof(unsigned int) * nvw));
+    PP_TRY(grow(W.u2, sizeof(unsigned int) * nvw));
+    PP_TRY(grow(W.u3, sizeof(unsigned int) * nvw));
+    PP_TRY(grow(W.scratch, std::max(scan_temp_bytes(nvw), select_temp_bytes(nfw))));
     const int4* Fw = as<int4>(W.Fw);
-    k_edge_uses<<<grid_for(ne, kThreads, sms), kThreads, 0, s>>>(Fw, nfw, b, as<unsigned long long>(W.key), as<int>(W.val));
-    PP_TRY(radix_sort_pairs(W.scratch.p, W.scratch.bytes, as<unsigned long long>(W.key),
-                            as<unsigned long long>(W.key2), as<uint32_t>(W.val), as<uint32_t>(W.val2), ne, 0, 2 * b, s));
-    if (R.remove_floaters) {
-        k_iota<<<grid_for(nfw, kThreads, sms), kThreads, 0, s>>>(as<int>(W.parent), nfw);
-        PP_TRY(cudaMemsetAsync(W.csize.p, 0, sizeof(unsigned int) * nfw, s));
-    }
+    int* const parent = as<int>(W.parent);
     EdgeRunParams ep;
-    ep.key = as<unsigned long long>(W.key2); ep.val = as<int>(W.val2); ep.n = ne; ep.invalid = inval; ep.Fw = Fw;
-    ep.close = R.close_holes; ep.remove = R.remove_floaters; ep.parent = as<int>(W.parent); ep.bnd = as<int4>(W.bnd);
+    ep.key = nullptr; ep.val = nullptr; ep.n = ne; ep.invalid = inval; ep.Fw = Fw;
+    ep.close = R.close_holes; ep.remove = R.remove_floaters; ep.parent = parent; ep.bnd = as<int4>(W.bnd);
     ep.C = C;
-    if (R.remove_floaters) k_first_links<<<grid_for(ne, kThreads, sms), kThreads, 0, s>>>(ep);
-    k_edge_runs<<<grid_for(ne, kThreads, sms), kThreads, 0, s>>>(ep);
-    PP_TRY(cudaGetLastError());
+    auto reset_faces = [&]() -> cudaError_t {
+        if (!R.remove_floaters) return cudaSuccess;
+        k_iota<<<grid_for(nfw, kThreads, sms), kThreads, 0, s>>>(parent, nfw);
+        return cudaMemsetAsync(W.csize.p, 0, sizeof(unsigned int) * nfw, s);
+    };
+    PP_TRY(reset_faces());
+    {
+        BucketParams bp;
+        bp.Fw = Fw; bp.nf = nfw; bp.nv = nvw;
+        bp.count = as<unsigned int>(W.u0); bp.fill = as<unsigned int>(W.u1); bp.longs = as<unsigned int>(W.u3);
+        bp.start = as<unsigned int>(W.u2);
+        bp.use = as<uint2>(W.key); bp.pair = as<int2>(W.key2);
+        bp.parent = parent; bp.C = C;
+        PP_TRY(cudaMemsetAsync(bp.count, 0, sizeof(unsigned int) * nvw, s));
+        PP_TRY(cudaMemsetAsync(bp.fill, 0, sizeof(unsigned int) * nvw, s));
+        PP_TRY(cudaMemsetAsync(bp.pair, 0xff, sizeof(int2) * ne, s));      // degenerate edges leave slots unused
+        k_bucket_uses<false><<<grid_for(nfw, kThreads, sms), kThreads, 0, s>>>(bp);
+        PP_TRY(exclusive_sum(W.scratch.p, W.scratch.bytes, bp.count, as<unsigned int>(W.u2), nvw, s));
+        k_bucket_uses<true><<<grid_for(nfw, kThreads, sms), kThreads, 0, s>>>(bp);
+        k_bucket_runs<<<grid_for(nvw, kThreads, sms), kThreads, 0, s>>>(bp, ep);
+        k_bucket_long<<<(unsigned)sms, kThreads, 0, s>>>(bp, ep);
+        if (R.remove_floaters) {
+            k_flatten<<<grid_for(nfw, kThreads, sms), kThreads, 0, s>>>(parent, nfw);
+            for (int r = 0; r < kLinkRounds; ++r) {
+                k_pair_link<<<grid_for(ne, kThreads, sms), kThreads, 0, s>>>(bp.pair, ne, parent, C, r);
+                k_flatten<<<grid_for(nfw, kThreads, sms), kThreads, 0, s>>>(parent, nfw, &C->linked[r]);
+            }
+            k_pair_unite<<<grid_for(ne, kThreads, sms), kThreads, 0, s>>>(bp.pair, ne, parent, C);
+        }
+        PP_TRY(cudaGetLastError());
+    }
     long long nkept = nfw;
     const int4* kept = Fw;
-    if (R.remove_floaters) {
-        k_flatten<<<grid_for(nfw, kThreads, sms), kThreads, 0, s>>>(as<int>(W.parent), nfw);
-        k_comp_size<<<grid_for(nfw, kThreads, sms), kThreads, 0, s>>>(as<int>(W.parent), nfw, as<unsigned int>(W.csize));
-        k_comp_pick<<<grid_for(nfw, kThreads, sms), kThreads, 0, s>>>(as<int>(W.parent), as<unsigned int>(W.csize), nfw, C);
-        k_keep_flags<<<grid_for(nfw, kThreads, sms), kThreads, 0, s>>>(as<int>(W.parent), nfw, C, as<unsigned char>(W.flag8));
+    auto components = [&]() -> cudaError_t {
+        if (!R.remove_floaters) return cudaSuccess;
+        k_flatten<<<grid_for(nfw, kThreads, sms), kThreads, 0, s>>>(parent, nfw);
+        k_comp_size<<<grid_for(nfw, kThreads, sms), kThreads, 0, s>>>(parent, nfw, as<unsigned int>(W.csize));
+        k_comp_pick<<<grid_for(nfw, kThreads, sms), kThreads, 0, s>>>(parent, as<unsigned int>(W.csize), nfw, C);
+        k_keep_flags<<<grid_for(nfw, kThreads, sms), kThreads, 0, s>>>(parent, nfw, C, as<unsigned char>(W.flag8));
         PP_TRY(cudaGetLastError());
         PP_TRY(cudaMemsetAsync(&C->nsel, 0, sizeof(unsigned long long), s));
         PP_TRY(select_flagged(W.scratch.p, W.scratch.bytes, Fw, as<unsigned char>(W.flag8), as<int4>(W.kept), &C->nsel,
                                           (int)nfw, s));
         kept = as<int4>(W.kept);
-    }
+        return cudaSuccess;
+    };
+    e = components();
+    if (e != cudaSuccess) return e;
     e = read_counters(W, R, s);
     if (e != cudaSuccess) return e;
+    if (host_counters(W).ntoo_long) {
+        // a vertex with more uses than a block compares: everything again from the sorted uses
+        PP_TRY(grow(W.val, sizeof(int) * ne));
+        PP_TRY(grow(W.val2, sizeof(int) * ne));
+        PP_TRY(grow(W.scratch, std::max(radix_sort_temp_bytes(ne, 8, true), select_temp_bytes(nfw))));
+        PP_TRY(cudaMemsetAsync(&C->nb, 0, sizeof(C->nb) + sizeof(C->ncomp) + sizeof(C->best), s));
+        PP_TRY(reset_faces());
+        ep.key = as<unsigned long long>(W.key2);
+        ep.val = as<int>(W.val2);
+        k_edge_uses<<<grid_for(ne, kThreads, sms), kThreads, 0, s>>>(Fw, nfw, b, as<unsigned long long>(W.key), as<int>(W.val));
+        PP_TRY(radix_sort_pairs(W.scratch.p, W.scratch.bytes, as<unsigned long long>(W.key), as<unsigned long long>(W.key2),
+                                as<uint32_t>(W.val), as<uint32_t>(W.val2), ne, 0, 2 * b, s));
+        if (R.remove_floaters) k_first_links<<<grid_for(ne, kThreads, sms), kThreads, 0, s>>>(ep);
+        k_edge_runs<<<grid_for(ne, kThreads, sms), kThreads, 0, s>>>(ep);
+        PP_TRY(cudaGetLastError());
+        e = components();
+        if (e != cudaSuccess) return e;
+        e = read_counters(W, R, s);
+        if (e != cudaSuccess) return e;
+    }
     {
         const PostCounters& h = host_counters(W);
         R.err = h.err;

@@ -265,6 +265,41 @@ k_radix_scatter(const K* __restrict__ kin, const uint32_t* __restrict__ vin, K* 
     }
 }
 
+// Up to kSortOne items: one block, a bitonic network over (sorted bits, position) in shared memory,
+// which is the same stable order. A pass of the radix sort is five launches whatever the size.
+constexpr int kSortOne = 2048, kSortOneThreads = 1024;
+template <typename K, bool PAIRS>
+__global__ void __launch_bounds__(kSortOneThreads)
+k_sort_one(const K* __restrict__ kin, const uint32_t* __restrict__ vin, K* __restrict__ kout, uint32_t* __restrict__ vout, int n,
+           int begin_bit, int bits) {
+    __shared__ K s_key[kSortOne];
+    __shared__ uint32_t s_pos[kSortOne];
+    const K mask = bits >= (int)(8 * sizeof(K)) ? ~K(0) : (K(1) << bits) - 1;
+    int size = 2;
+    while (size < n) size *= 2;
+    for (int x = threadIdx.x; x < size; x += kSortOneThreads) {
+        s_key[x] = x < n ? (kin[x] >> begin_bit) & mask : ~K(0);
+        s_pos[x] = x;                                    // padding: last by position
+    }
+    for (int k = 2; k <= size; k *= 2)
+        for (int j = k / 2; j > 0; j /= 2) {
+            __syncthreads();
+            for (int t = threadIdx.x; t < size / 2; t += kSortOneThreads) {
+                const int a = 2 * t - (t & (j - 1)), b = a + j;
+                const K ka = s_key[a], kb = s_key[b];
+                const uint32_t pa = s_pos[a], pb = s_pos[b];
+                const bool greater = ka > kb || (ka == kb && pa > pb);
+                if (greater == ((a & k) == 0)) { s_key[a] = kb; s_key[b] = ka; s_pos[a] = pb; s_pos[b] = pa; }
+            }
+        }
+    __syncthreads();
+    for (int x = threadIdx.x; x < n; x += kSortOneThreads) {
+        const uint32_t from = s_pos[x];
+        kout[x] = kin[from];
+        if (PAIRS) vout[x] = vin[from];
+    }
+}
+
 template <typename K, bool PAIRS>
 cudaError_t sort_impl(void* temp, size_t temp_bytes, const K* kin, K* kout, const uint32_t* vin, uint32_t* vout, long long n,
                       int begin_bit, int end_bit, cudaStream_t s) {
@@ -287,6 +322,10 @@ cudaError_t sort_impl(void* temp, size_t temp_bytes, const K* kin, K* kout, cons
         cudaError_t e = cudaMemcpyAsync(kout, kin, sizeof(K) * (size_t)n, cudaMemcpyDeviceToDevice, s);
         if (e == cudaSuccess && PAIRS) e = cudaMemcpyAsync(vout, vin, sizeof(uint32_t) * (size_t)n, cudaMemcpyDeviceToDevice, s);
         return e;
+    }
+    if (n <= kSortOne) {
+        k_sort_one<K, PAIRS><<<1, kSortOneThreads, 0, s>>>(kin, vin, kout, vout, (int)n, begin_bit, end_bit - begin_bit);
+        return cudaGetLastError();
     }
     // the last pass writes the output: an odd count starts there, an even one in the scratch
     const K* sk = kin;
