@@ -401,14 +401,14 @@ __global__ void k_bucket_long(BucketParams P, EdgeRunParams E) {
 // finds in a growing forest, took 1.24 ms for 3M pairs of the 512^3 CSG mesh (3% issue,
 // 300 cycles a load).
 constexpr int kLinkRounds = 6;
-__global__ void k_pair_link(const int2* __restrict__ pair, long long n, int* parent, PostCounters* C, int round) {
+__global__ void k_pair_link(int2* __restrict__ pair, long long n, int* parent, PostCounters* C, int round) {
     if (round > 0 && !C->linked[round - 1]) return;
     bool any = false;
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
         const int2 q = pair[t];
         if (q.x < 0) continue;
         const int a = __ldcg(parent + q.x), b = __ldcg(parent + q.y);
-        if (a == b) continue;
+        if (a == b) { pair[t].x = -1; continue; }             // done: the next rounds do not look again
         const int hi = max(a, b), lo = min(a, b);
         if (__ldcg(parent + hi) > lo) atomicMin(parent + hi, lo);
         any = true;
@@ -551,6 +551,30 @@ __global__ void k_cycle_rank_jump(const unsigned long long* __restrict__ skey, l
         moved = true;
     }
     if (__any_sync(0xffffffffu, moved) && (threadIdx.x & 31) == 0) changed[r] = 1;
+}
+
+// All rounds in one block, for few starts (a launch a round otherwise: 61 us of kernels and 31
+// gaps, most of them rounds with nothing left to move).
+constexpr long long kRankOne = 16384;
+__global__ void __launch_bounds__(1024) k_cycle_rank_one(const unsigned long long* __restrict__ skey, long long ns, int b,
+                                                         const unsigned int* __restrict__ bad, const int* __restrict__ root,
+                                                         unsigned long long* rank) {
+    const unsigned long long m = (1ull << b) - 1;
+    volatile unsigned long long* R = rank;
+    for (int r = 0; r < kRankRounds; ++r) {
+        bool moved = false;
+        for (long long p = threadIdx.x; p < ns; p += blockDim.x) {
+            const unsigned int u = (unsigned int)(skey[p] & m);
+            if (bad[root[u]]) continue;
+            const unsigned long long me = R[u];
+            const unsigned int nx = (unsigned int)me;
+            if (nx == 0xffffffffu) continue;
+            const unsigned long long there = R[nx];
+            R[u] = (((me >> 32) + (there >> 32)) << 32) | (there & 0xffffffffull);
+            moved = true;
+        }
+        if (!__syncthreads_or(moved)) break;
+    }
 }
 
 // The loop region of every component: base[root] = its first entry (the starts' scan).
@@ -1303,7 +1327,10 @@ cudaError_t post_run(PostWork& W, PostRun& R, cudaStream_t s) {
             k_cycle_rank_init<<<grid_for(ns, kThreads, sms), kThreads, 0, s>>>(starts, ns, b, as<unsigned int>(W.cbad),
                                                                                 as<int>(W.vparent), as<int>(W.succ),
                                                                                 as<unsigned long long>(W.crank));
-            for (int r = 0; r < kRankRounds; ++r)
+            if (ns <= kRankOne)
+                k_cycle_rank_one<<<1, 1024, 0, s>>>(starts, ns, b, as<unsigned int>(W.cbad), as<int>(W.vparent),
+                                                    as<unsigned long long>(W.crank));
+            else for (int r = 0; r < kRankRounds; ++r)
                 k_cycle_rank_jump<<<grid_for(ns, kThreads, sms), kThreads, 0, s>>>(starts, ns, b, as<unsigned int>(W.cbad),
                                                                                     as<int>(W.vparent),
                                                                                     as<unsigned long long>(W.crank),

@@ -266,14 +266,16 @@ k_radix_scatter(const K* __restrict__ kin, const uint32_t* __restrict__ vin, K* 
 }
 
 // Up to kSortOne items: one block, a bitonic network over (sorted bits, position) in shared memory,
-// which is the same stable order. A pass of the radix sort is five launches whatever the size.
-constexpr int kSortOne = 2048, kSortOneThreads = 1024;
+// which is the same stable order. A pass of the radix sort is five launches whatever the size
+// (4,000 boundary edges of 42 bits: 30 launches, 140 us).
+constexpr int kSortOne = 8192, kSortOneThreads = 1024;
 template <typename K, bool PAIRS>
 __global__ void __launch_bounds__(kSortOneThreads)
 k_sort_one(const K* __restrict__ kin, const uint32_t* __restrict__ vin, K* __restrict__ kout, uint32_t* __restrict__ vout, int n,
            int begin_bit, int bits) {
-    __shared__ K s_key[kSortOne];
-    __shared__ uint32_t s_pos[kSortOne];
+    extern __shared__ __align__(16) unsigned char s_sort[];
+    K* const s_key = reinterpret_cast<K*>(s_sort);
+    uint32_t* const s_pos = reinterpret_cast<uint32_t*>(s_key + kSortOne);
     const K mask = bits >= (int)(8 * sizeof(K)) ? ~K(0) : (K(1) << bits) - 1;
     int size = 2;
     while (size < n) size *= 2;
@@ -324,7 +326,10 @@ cudaError_t sort_impl(void* temp, size_t temp_bytes, const K* kin, K* kout, cons
         return e;
     }
     if (n <= kSortOne) {
-        k_sort_one<K, PAIRS><<<1, kSortOneThreads, 0, s>>>(kin, vin, kout, vout, (int)n, begin_bit, end_bit - begin_bit);
+        constexpr int kBytes = kSortOne * (sizeof(K) + sizeof(uint32_t));
+        cudaError_t e = cudaFuncSetAttribute(k_sort_one<K, PAIRS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes);
+        if (e != cudaSuccess) return e;
+        k_sort_one<K, PAIRS><<<1, kSortOneThreads, kBytes, s>>>(kin, vin, kout, vout, (int)n, begin_bit, end_bit - begin_bit);
         return cudaGetLastError();
     }
     // the last pass writes the output: an odd count starts there, an even one in the scratch
