@@ -395,7 +395,7 @@ k_cell_jacobi(const __grid_constant__ QefParams P) {
             const unsigned int slot = atomicAdd(P.esc_count, 1u);
             P.esc_list[slot] = r;
         }
-        const GridDesc& g = slot_at(P.B, slot_of_rank(P.B, r)).g;
+        const GridDesc g = slot_at(P.B, slot_of_rank(P.B, r)).g;
         const float wx1 = width_axis(g, 0, i), wy1 = width_axis(g, 1, j), wz1 = width_axis(g, 2, k);
         store_vertex(P.V, g, r, i, j, k, d2.y + wx, d2.z + wy * (wx1 / wy1), d2.w + wz * (wx1 / wz1));
         P.vclass[r] = kVcJacobi;

@@ -217,7 +217,7 @@ k_vertex_fp64(const __grid_constant__ Vertex64Params P) {
             const uint32_t r = P.cells[t0 + lane];
             int i, j, k;
             unpack_cell(P.list[r], i, j, k);
-            const GridDesc& g = slot_at(P.B, slot_of_rank(P.B, r)).g;
+            const GridDesc g = slot_at(P.B, slot_of_rank(P.B, r)).g;       // a copy: registers
             double cs[8];
 #pragma unroll
             for (int c = 0; c < 8; ++c)
@@ -245,7 +245,7 @@ k_vertex_fp64(const __grid_constant__ Vertex64Params P) {
             const uint32_t r = P.cells[t0 + q];
             int i, j, k;
             unpack_cell(P.list[r], i, j, k);
-            const GridDesc& g = slot_at(P.B, slot_of_rank(P.B, r)).g;
+            const GridDesc g = slot_at(P.B, slot_of_rank(P.B, r)).g;       // a copy: registers
             int cc[4][3], ex[4];
             const bool shared = f64::edge_cells(g, i, j, k, e, cc, ex);    // else the cell's own normal
             int own = 0;
@@ -293,7 +293,7 @@ k_vertex_fp64(const __grid_constant__ Vertex64Params P) {
         const uint32_t r = P.cells[t];
         int i, j, k;
         unpack_cell(P.list[r], i, j, k);
-        const GridDesc& g = slot_at(P.B, slot_of_rank(P.B, r)).g;
+        const GridDesc g = slot_at(P.B, slot_of_rank(P.B, r)).g;
         double x[3];
         f64::cell_vertex_thread(g, i, j, k, P.thr, x);
         store64(P, r, t, x);
@@ -325,7 +325,7 @@ k_winding_fp64(const __grid_constant__ Winding64Params P) {
     for (unsigned int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
         const uint4 it = P.items[t];
         const int axis = (int)(it.y & 3u);
-        const GridDesc& g = slot_at(P.B, (int)(it.y >> 2)).g;
+        const GridDesc g = slot_at(P.B, (int)(it.y >> 2)).g;
         int i, j, k;
         unpack_cell(((uint64_t)it.w << 32) | it.z, i, j, k);
         const int4 q4 = P.quads[it.x];
