@@ -233,7 +233,7 @@ int layout_batch(dcb_context* h, const dcb_grid* in, int n, BatchLayout& L) {
         // grids at most 256 cells wide march 256-cell x-tiles (less idle width)
         S.tw = g.cx <= h->tune_narrow_cells ? mark_narrow_tile_words() : mark_tile_words();
         S.nxt = (g.cx + 32 * S.tw - 1) / (32 * S.tw);
-        S.R = std::min(mark_max_rows(), g.cy);
+        S.R = mark_rows(S.tw, g.cy, n == 1);
         S.nrb = (g.cy + S.R - 1) / S.R;
         // About four CTAs per resident slot, each marching 8..64 planes (a single long wave
         // measured slower at 1024^3: 0.887 vs 0.848 ms).

@@ -15,7 +15,7 @@ struct GridSlot {
     long long super_off;           // first super word (rows * W8)
     long long seg_off;             // first segment (rows * nxt)
     long long col_off;             // first face column (3 * cx * cy)
-    int R;                         // mark: cell rows per tile (point rows = R + 1 <= 8)
+    int R;                         // mark: cell rows per tile (mark_rows)
     int KZ;                        // mark: cell planes per tile
     int nxt;                       // mark: x-tiles of 1024 cells per row
     int nrb;                       // mark: row blocks
@@ -91,7 +91,7 @@ cudaError_t launch_mark(const MarkParams& P, int tw, cudaStream_t s);
 int mark_tile_words();
 int mark_narrow_tile_words();
 int mark_ctas_per_sm(bool one);   // resident CTAs of the mark kernel per SM (single grid / batch)
-int mark_max_rows();
+int mark_rows(int tw, int cy, bool one);   // cell rows per tile (GridSlot::R)
 
 struct ExpandParams {
     BatchTable B;

@@ -86,7 +86,7 @@ extern "C" int dcb_mark_active_cells_noalloc(const dcb_grid* grid, int64_t* cell
     slot.nxt = nxt;
     slot.tw = mark_tile_words();
     slot.hmax = std::max(std::fabs(g.vx), std::max(std::fabs(g.vy), std::fabs(g.vz)));
-    slot.R = std::min(mark_max_rows(), g.cy);
+    slot.R = mark_rows(slot.tw, g.cy, true);
     slot.nrb = (g.cy + slot.R - 1) / slot.R;
     slot.KZ = (int)std::max(8LL, std::min(64LL, ((long long)g.cz * nxt * slot.nrb + (long long)sms * 12 - 1) / ((long long)sms * 12)));
     slot.nzc = (g.cz + slot.KZ - 1) / slot.KZ;
