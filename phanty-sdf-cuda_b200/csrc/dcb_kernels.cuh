@@ -321,7 +321,7 @@ struct OursParams {
     uint32_t* cell_spheres;         // grid points by cell, by radius
     float4* cell_centres;           // their positions and values
     int* prev_tri;                  // [npts] closest triangle of each grid point last time
-    uint32_t* team_list[3];         // cells by number of spheres (the inner loop's team sizes)
+    uint32_t* team_list[3];         // cells by number of spheres
     unsigned int* team_count;       // [3] their numbers, [3] next to take
     uint32_t* long_query;           // selected points whose search exceeded a thread's budget
     unsigned int* long_count;

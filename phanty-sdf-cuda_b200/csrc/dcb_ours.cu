@@ -23,7 +23,7 @@
 //      than 1e-6 (contouring.cpp:1288-1309).
 // Everything is FP64 and compiled with --fmad=false, like the CPU restatement it is checked
 // against. One thread per cell (steps 3, 4), per quad (1), per grid point (2; a warp for the
-// points with long searches), a team of lanes per cell (5).
+// points with long searches), a lane per (cell, sphere), (cell, sum) and cell (5).
 #include <cfloat>
 #include "dcb_f64.cuh"
 #include "dcb_sort.cuh"
@@ -195,8 +195,8 @@ __device__ __forceinline__ unsigned long long splitmix64(unsigned long long x) {
 
 }  // namespace
 
-// Lanes that work on one cell's inner loop, by its number of spheres (below kTeamSpheres[i]).
-constexpr int kTeamLanes[3] = {8, 16, 256};
+// Cells of the inner loop by their number of spheres (below kTeamSpheres[i]): few, some tens (both
+// packed into a block's rows, the larger ones first), a block per cell.
 constexpr unsigned int kTeamSpheres[2] = {16, 128};
 
 // ---- setup -------------------------------------------------------------------------------
@@ -912,35 +912,46 @@ __device__ void inner_solve(const OursParams& P, const double Acc[9], const doub
 // (vertex_refinement.cpp:201-280) + Cell::minimize_qef (Cell.cpp:364-473) until the vertex
 // moves less than 1e-6. A sphere's row is skipped or adds to the 6 entries of the symmetric
 // A^T A (00 01 02 11 12 22) and the 3 of A^T b; rows are summed in 32 chunks of consecutive
-// spheres, each from zero, added in chunk order: the same sums for every team size.
+// spheres, each from zero, added in chunk order: the same sums however the rows are dealt.
 //
-// A team of T lanes per cell, cells from a counter: each lane forms rows of the team's next T
-// spheres (the distances to the local fan, most of the work), then the nine sums are
-// spread over the lanes, then every lane solves. Cells differ a hundredfold in work (1 to
-// 1,600 spheres, 2 to 100 iterations): with a thread per cell below 8 spheres and a warp above,
-// 3 and 18 lanes were active and the longest cells kept the launch. An outer iteration on a
-// 128^3 perturbed sphere: 12.4 ms before, 4.7 now; 72^3 (cells of up to 1,600 spheres) 20.1 and
-// 6.8. Eight lanes for the short cells because their 100 iterations are a chain (4 lanes: 5.3,
-// 16: 4.8). Bound: FP64 instructions (45% of the pipe) and the chain of the solve's divisions.
-// Loads cell r; how many triangles its local fan has: (vertex, Hermite point on edge e, face
-// point d) for each face d with a point and each of its four edges with a Hermite point, in
-// face then edge order. 0: nothing to do. By the T lanes of a team; a team synchronisation has
-// to follow.
-template <int T>
-__device__ int team_load(const OursParams& P, const OursCell& S, TeamCell& C, int tl) {
-    const int hmask = S.hmask, fmask = S.fmask;
+// A block holds up to kSlots cells, of at most kRows spheres together, and takes more from a
+// counter as cells finish. An iteration of all of them: a lane per (cell, sphere) forms the rows
+// (the distances to the local fan, most of the work), a lane per (cell, sum) adds them up,
+// one warp solves, a lane per cell.
+//
+// What bounds it: FP64 instructions at their latency (43% of the issue slots of busy SMs), then cells
+// of 100 iterations, a chain each. An outer iteration of a 128^3 perturbed sphere takes 2.7 ms
+// (72^3, with cells of up to 1,600 spheres: 5.3; a 128^3 sphere 0.6). A team of 8 lanes per cell,
+// each lane solving, took 4.7 (6.8): half the instructions were the same solves again, and 10 of
+// 32 lanes were active (now 20). 28 slots because all cells of such grids are then in flight at
+// once (32: 2.8, 24 with five blocks an SM 2.8); 8 or 16 cells to a warp without block
+// synchronisations: 5.0 (a warp's chain is too long); four lanes a sphere: 3.0-3.4. The cells are
+// dealt by columns so that no block gets the large ones (taken in list order: 3.0).
+constexpr int kInnerThreads = 128;
+constexpr int kSlots = 28;                 // a lane of the solving warp each
+constexpr unsigned int kRows = 512;
+constexpr unsigned int kRefill = 4;        // free slots that are worth a fill
+static_assert(kSlots <= 32 && kTeamSpheres[1] - 1 <= kRows && kRows >= kInnerThreads, "");
+struct InnerShared {
+    TeamCell cell[kSlots];
+    double row[4][kRows];                  // entries 0..2 and the right-hand side
+    double part[32][9];
+    unsigned int first[kSlots + 1];        // each slot's first row; at the end their number
+    unsigned int sphere[kSlots], source[kSlots];
+    int nfan[kSlots];
+    unsigned int fresh, next;
+    bool done;
+};
+
+// The local fan of a cell: (vertex, Hermite point on edge e, face point d) for each face d with a
+// point and each of its four edges with a Hermite point, in face then edge order. Its length;
+// 0: nothing to do.
+__device__ __forceinline__ int local_fan(int hmask, int fmask, unsigned char* fan) {
     int nfan = 0;
     for (int x = 0; x < 24; ++x) {
         const int d = x >> 2, e = kFaceEdges[d][x & 3];
-        if ((fmask & (1 << d)) && (hmask & (1 << e))) {
-            if (tl == 0) C.fan[nfan] = (unsigned char)(e | d << 4);
-            ++nfan;
-        }
+        if ((fmask & (1 << d)) && (hmask & (1 << e))) fan[nfan++] = (unsigned char)(e | d << 4);
     }
-    if (!nfan) return 0;
-    for (int x = tl; x < 36; x += T) (&C.hp[0][0])[x] = (&S.hp[0][0])[x];
-    for (int x = tl; x < 18; x += T) (&C.fi[0][0])[x] = (&S.fi[0][0])[x];
-    if (tl == 0) hermite_rows(P, S, C.h0, C.cen);
     return nfan;
 }
 
@@ -948,126 +959,167 @@ __device__ int team_load(const OursParams& P, const OursCell& S, TeamCell& C, in
 __device__ __forceinline__ int sum_left(int q) { return q < 3 ? 0 : q < 5 ? 1 : q == 5 ? 2 : q - 6; }
 __device__ __forceinline__ int sum_right(int q) { return q < 3 ? q : q < 5 ? q - 2 : q == 5 ? 2 : 3; }
 
-constexpr int kInnerThreads = 256;
-struct InnerShared {
-    TeamCell cell[kInnerThreads / kTeamLanes[0]];
-    double row[kInnerThreads][4];
-    unsigned char ok[kInnerThreads];
-    double part[32][9];
-    unsigned int next;
-};
+// Row `at` of the block from one sphere; a skipped row is zero (a sum that starts from zero is
+// unchanged by +0).
+__device__ __forceinline__ void put_row(InnerShared& S, unsigned int at, const TeamCell& C, int nfan, const float4* sphere,
+                                        double ssw) {
+    double row[4];
+    const bool ok = sphere_row(C, nfan, sphere, ssw, row);
+    for (int q = 0; q < 4; ++q) S.row[q][at] = ok ? row[q] : 0.0;
+}
 
-template <int T>
-__device__ void inner_teams(const OursParams& P, InnerShared& S, int team) {
-    constexpr int kSums = (9 + T - 1) / T;
-    static_assert(T >= 3 && T <= 16, "three lanes hand on the vertex; a team lies within a warp");
-    const int tl = threadIdx.x % T, tm = threadIdx.x / T;
-    const unsigned int lanes = ((1u << T) - 1u) << (threadIdx.x & 31 & ~(T - 1));
-    TeamCell& C = S.cell[tm];
-    double (*const rows)[4] = S.row + tm * T;
-    const unsigned char* const oks = S.ok + tm * T;
-    const unsigned int ncells = P.team_count[team];
+__device__ void inner_packed(const OursParams& P, InnerShared& S) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // the warp that solves: another one in each of the blocks that share an SM (they share its schedulers)
+    const bool solver = warp == (int)(blockIdx.x / ((gridDim.x + 3) / 4)) % (kInnerThreads / 32);
+    const unsigned int big = P.team_count[1], ncells = big + P.team_count[0], share = min((ncells + gridDim.x - 1) / gridDim.x, (unsigned int)kSlots);
+    // every take of `share` cells has one of each size class: the list, in pieces of share * blocks, by columns
+    const unsigned int piece = share * gridDim.x;
     const double ssw = sqrt(P.sphere_weight), smu = sqrt(P.mu);
-    bool active = false, more = true;
-    long long r = 0;
-    unsigned int nsph = 0, cs = 1;
-    int nfan = 0, it = 0;
-    const float4* sph = nullptr;
-    double v[3] = {0.0, 0.0, 0.0};
+    TeamCell& C = S.cell[lane % kSlots];
+    bool have = false, runs = false, more = ncells > 0;      // this lane's slot holds a cell; takes part; cells are left
+    unsigned int r = 0, n = 0;
+    int it = 0;
     for (;;) {
-        if (!active && more) {
-            unsigned int w = 0;
-            if (tl == 0) w = atomicAdd(P.team_count + 3 + team, 1u);
-            w = __shfl_sync(lanes, w, 0, T);
-            more = w < ncells;
-            if (more) {
-                r = P.team_list[team][w];
-                const OursCell& cell = P.cells[r];
-                nfan = team_load<T>(P, cell, C, tl);
-                active = nfan > 0;
-                nsph = P.cell_count[r];
-                cs = (nsph + 31) / 32;
-                sph = P.cell_centres + P.cell_start[r];
-                for (int a = 0; a < 3; ++a) v[a] = cell.v[a];
-                it = 0;
-            }
-        }
-        __syncwarp();
-        if (!__any_sync(0xffffffffu, active || more)) break;
-        const double prev[3] = {v[0], v[1], v[2]};
-        if (tl < 3) C.prev[tl] = tl == 0 ? v[0] : tl == 1 ? v[1] : v[2];
-        __syncwarp();
-        double sum[kSums], part[kSums];
-        for (int q = 0; q < kSums; ++q) { sum[q] = active && tl + q * T < 9 ? C.h0[tl + q * T] : 0.0; part[q] = 0.0; }
-        const unsigned int steps = __reduce_max_sync(0xffffffffu, active ? (nsph + T - 1) / T : 0u);
-        unsigned int edge = cs;                          // first sphere of the next chunk
-        for (unsigned int k = 0; k < steps; ++k) {
-            const unsigned int s0 = k * T;
-            if (active && s0 + tl < nsph)
-                S.ok[threadIdx.x] = sphere_row(C, nfan, sph + s0 + tl, ssw, rows[tl]);
-            __syncwarp();
-            if (active && s0 < nsph) {
-                const unsigned int m = min((unsigned int)T, nsph - s0);
-                for (unsigned int j = 0; j < m; ++j) {
-                    if (s0 + j == edge) {
-                        for (int q = 0; q < kSums; ++q) { sum[q] += part[q]; part[q] = 0.0; }
-                        edge += cs;
+        if (solver) {
+            const unsigned int held = __ballot_sync(0xffffffffu, have), waiting = __ballot_sync(0xffffffffu, have && !runs);
+            const unsigned int rows = __reduce_add_sync(0xffffffffu, runs ? n : 0u);
+            const unsigned int room = kSlots - __popc(held);
+            bool fresh = false;
+            if (more && !waiting && (room >= kRefill || !held)) {
+                const unsigned int want = min(min(room, share), max((kRows - rows) / 8, held ? 0u : 1u));
+                if (want) {
+                    unsigned int w = 0;
+                    if (lane == 0) w = atomicAdd(P.team_count + 3, want);
+                    w = __shfl_sync(0xffffffffu, w, 0);
+                    const unsigned int k = __popc(~held & ((1u << lane) - 1u));
+                    const unsigned int at = (w + k) % piece, x = w + k - at + at % share * gridDim.x + at / share;
+                    if (lane < kSlots && !have && k < want && x < ncells) {
+                        r = x < big ? P.team_list[1][x] : P.team_list[0][x - big];
+                        const OursCell& cell = P.cells[r];
+                        const int nfan = local_fan(cell.hmask, cell.fmask, C.fan);
+                        fresh = have = nfan > 0;
+                        if (have) {
+                            n = P.cell_count[r];
+                            it = 0;
+                            S.sphere[lane] = P.cell_start[r];
+                            S.source[lane] = r;
+                            S.nfan[lane] = nfan;
+                            for (int a = 0; a < 3; ++a) C.prev[a] = cell.v[a];
+                            hermite_rows(P, cell, C.h0, C.cen);
+                        }
                     }
-                    if (!oks[j]) continue;
-                    for (int q = 0; q < kSums; ++q) {
-                        const int e = min(tl + q * T, 8);
-                        part[q] += rows[j][sum_left(e)] * rows[j][sum_right(e)];
-                    }
+                    more = w + want < (ncells + piece - 1) / piece * piece;
                 }
             }
-            __syncwarp();
+            // cells wait until their rows have room
+            unsigned int before = have && !runs ? n : 0u;
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned int t = __shfl_up_sync(0xffffffffu, before, o);
+                if (lane >= o) before += t;
+            }
+            runs = have && (runs || rows + before <= kRows);
+            unsigned int end = runs ? n : 0u;
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned int t = __shfl_up_sync(0xffffffffu, end, o);
+                if (lane >= o) end += t;
+            }
+            if (lane < kSlots) S.first[lane + 1] = end;
+            const unsigned int loads = __ballot_sync(0xffffffffu, fresh), left = __ballot_sync(0xffffffffu, have);
+            if (lane == 0) { S.first[0] = 0; S.fresh = loads; S.done = !more && !left; }
         }
-        for (int q = 0; q < kSums; ++q)
-            if (active && tl + q * T < 9) C.sums[tl + q * T] = sum[q] + part[q];
-        __syncwarp();
-        if (active) {
+        __syncthreads();
+        if (S.done) break;
+        if (S.fresh) {
+            for (int t = warp; t < kSlots; t += kInnerThreads / 32) {
+                if (!(S.fresh >> t & 1)) continue;
+                const OursCell& cell = P.cells[S.source[t]];
+                for (int x = lane; x < 36; x += 32) (&S.cell[t].hp[0][0])[x] = (&cell.hp[0][0])[x];
+                if (lane < 18) (&S.cell[t].fi[0][0])[lane] = (&cell.fi[0][0])[lane];
+            }
+            __syncthreads();
+        }
+        const unsigned int total = S.first[kSlots];
+        for (unsigned int x = threadIdx.x; x < total; x += kInnerThreads) {
+            int t = 0;                                  // the last slot that begins at or before x
+            for (int st = 16; st; st >>= 1) if (t + st < kSlots && S.first[t + st] <= x) t += st;
+            put_row(S, x, S.cell[t], S.nfan[t], P.cell_centres + S.sphere[t] + (x - S.first[t]), ssw);
+        }
+        __syncthreads();
+        for (int x = threadIdx.x; x < 9 * kSlots; x += kInnerThreads) {
+            const int t = x / 9, q = x % 9;
+            const unsigned int b = S.first[t], m = S.first[t + 1] - b;
+            if (!m) continue;
+            const double* const l = S.row[sum_left(q)] + b;
+            const double* const g = S.row[sum_right(q)] + b;
+            double sum = S.cell[t].h0[q];
+            if (m <= 32) {                              // a row a chunk
+#pragma unroll 8
+                for (unsigned int j = 0; j < m; ++j) sum += l[j] * g[j];
+            } else {
+                const unsigned int cs = (m + 31) / 32;
+                for (unsigned int j = 0; j < m;) {
+                    const unsigned int e = min(m, j + cs);
+                    double part = 0.0;
+                    for (; j < e; ++j) part += l[j] * g[j];
+                    sum += part;
+                }
+            }
+            S.cell[t].sums[q] = sum;
+        }
+        __syncthreads();
+        if (solver && runs) {
+            const double prev[3] = {C.prev[0], C.prev[1], C.prev[2]};
+            double v[3];
             inner_solve(P, C.sums, prev, C.cen, smu, v);
-            double dm[3] = {v[0] - prev[0], v[1] - prev[1], v[2] - prev[2]};
+            const double dm[3] = {v[0] - prev[0], v[1] - prev[1], v[2] - prev[2]};
+            for (int a = 0; a < 3; ++a) C.prev[a] = v[a];
             if (norm3(dm) < 1e-6 || ++it >= P.inner_iters) {
-                active = false;
-                if (tl == 0) for (int a = 0; a < 3; ++a) P.cells[r].v[a] = v[a];
+                have = runs = false;
+                for (int a = 0; a < 3; ++a) P.cells[r].v[a] = v[a];
             }
         }
-        __syncwarp();
     }
 }
 
-// The same with the block as one team: 8 lanes a chunk.
-__device__ void inner_block(const OursParams& P, InnerShared& S, int team) {
+// The same for one cell with a whole block: 4 lanes a chunk.
+__device__ void inner_block(const OursParams& P, InnerShared& S) {
     constexpr int T = kInnerThreads, kLanes = T / 32;
     TeamCell& C = S.cell[0];
     const int tid = threadIdx.x, chunk = tid / kLanes, sub = tid % kLanes;
-    const unsigned int ncells = P.team_count[team];
+    const unsigned int ncells = P.team_count[2];
     const double ssw = sqrt(P.sphere_weight), smu = sqrt(P.mu);
     for (;;) {
         __syncthreads();
-        if (tid == 0) S.next = atomicAdd(P.team_count + 3 + team, 1u);
+        if (tid == 0) S.next = atomicAdd(P.team_count + 4, 1u);
         __syncthreads();
         if (S.next >= ncells) break;
-        const long long r = P.team_list[team][S.next];
+        const long long r = P.team_list[2][S.next];
         const OursCell& cell = P.cells[r];
-        const int nfan = team_load<T>(P, cell, C, tid);
-        if (!nfan) continue;
+        if (tid == 0) {
+            S.nfan[0] = local_fan(cell.hmask, cell.fmask, C.fan);
+            hermite_rows(P, cell, C.h0, C.cen);
+        }
+        for (int x = tid; x < 36; x += T) (&C.hp[0][0])[x] = (&cell.hp[0][0])[x];
+        for (int x = tid; x < 18; x += T) (&C.fi[0][0])[x] = (&cell.fi[0][0])[x];
         const unsigned int nsph = P.cell_count[r], cs = (nsph + 31) / 32, nchunks = (nsph + cs - 1) / cs;
         const float4* const sph = P.cell_centres + P.cell_start[r];
         if (tid < 3) C.prev[tid] = cell.v[tid];
         __syncthreads();
+        const int nfan = S.nfan[0];
+        if (!nfan) continue;
         for (int it = 0; it < P.inner_iters; ++it) {
             for (int x = tid; x < 32 * 9; x += T) (&S.part[0][0])[x] = 0.0;
             for (unsigned int k = 0; k < cs; k += kLanes) {
                 const unsigned int s = chunk * cs + k + sub;
-                S.ok[tid] = k + sub < cs && s < nsph && sphere_row(C, nfan, sph + s, ssw, S.row[tid]);
+                if (k + sub < cs && s < nsph) put_row(S, tid, C, nfan, sph + s, ssw);
+                else for (int q = 0; q < 4; ++q) S.row[q][tid] = 0.0;
                 __syncthreads();
                 for (int x = tid; x < 32 * 9; x += T) {
                     const int l = x / 9, e = x % 9;
                     double part = S.part[l][e];
                     for (int j = l * kLanes; j < (l + 1) * kLanes; ++j)
-                        if (S.ok[j]) part += S.row[j][sum_left(e)] * S.row[j][sum_right(e)];
+                        part += S.row[sum_left(e)][j] * S.row[sum_right(e)][j];
                     S.part[l][e] = part;
                 }
                 __syncthreads();
@@ -1096,13 +1148,13 @@ __device__ void inner_block(const OursParams& P, InnerShared& S, int team) {
 
 // Longest cells first; every block that fits on the GPU takes cells from the counters, so a block
 // with a long cell keeps only itself.
-__global__ void __launch_bounds__(kInnerThreads, 2) k_ours_inner(const __grid_constant__ OursParams P) {
+constexpr int kInnerBlocks = 4;            // per SM
+__global__ void __launch_bounds__(kInnerThreads, kInnerBlocks) k_ours_inner(const __grid_constant__ OursParams P) {
     extern __shared__ __align__(16) unsigned char s_raw[];
     InnerShared& S = *reinterpret_cast<InnerShared*>(s_raw);
-    inner_block(P, S, 2);
-    inner_teams<kTeamLanes[1]>(P, S, 1);
+    inner_block(P, S);
     __syncthreads();
-    inner_teams<kTeamLanes[0]>(P, S, 0);
+    inner_packed(P, S);
 }
 
 __global__ void k_ours_mesh(OursParams P) {
@@ -1153,7 +1205,7 @@ size_t ours_workspace_bytes(long long nv, long long nq, long long npts, size_t* 
     b += al(sizeof(unsigned long long) * npts) * 2 + al(sizeof(uint32_t) * npts);  // fill keys/values
     b += 3 * al(sizeof(unsigned int) * (nv + 1)) + al(sizeof(uint32_t) * npts);    // count/start/fill, spheres
     b += al(sizeof(float4) * npts);                                          // their centres
-    b += 3 * al(sizeof(uint32_t) * (nv + 1));                                // cells by team size
+    b += 3 * al(sizeof(uint32_t) * (nv + 1));                                // cells by number of spheres
     b += al(sizeof(uint32_t) * npts);                                        // points with long searches
     b += al(sizeof(uint32_t) * npts);                                        // selected points, sorted
     b += al(sizeof(int) * npts);                                             // last closest triangle per point
@@ -1260,7 +1312,7 @@ cudaError_t ours_run(OursRun& R, cudaStream_t s) {
         }
         k_ours_faces<<<grid_for(nv, 128, sms), 128, 0, s>>>(P);
         if (R.hermite_update && it > 0) k_ours_hermite<<<grid_for(12 * nv, 128, sms), 128, 0, s>>>(P);
-        if (P.inner_iters > 0) k_ours_inner<<<(unsigned)sms * 2, kInnerThreads, sizeof(InnerShared), s>>>(P);
+        if (P.inner_iters > 0) k_ours_inner<<<(unsigned)sms * kInnerBlocks, kInnerThreads, sizeof(InnerShared), s>>>(P);
         k_ours_mesh<<<grid_for(nv, 128, sms), 128, 0, s>>>(P);
         OURS_TRY(cudaGetLastError());
     }
