@@ -1,0 +1,24 @@
+"""The refinement's random fill: some, most and all but one of the points away from the surface, in
+grid order and sorted (more than 8,192), against the oracle, which sorts all keys. Tolerance: the
+output's float rounding of coordinates up to 0.5 (3e-8) in cell widths of 1/32 and the oracle's
+own FP64 noise, below 1e-5 of a cell; another set of spheres moves vertices by far more."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("batch", [12000, 20000, 33 ** 3 - 1])
+def test_fill_matches_oracle(batch):
+    import oracle as O
+    from contouring_b200 import B200DualContouringBackend, ContouringMethod, ContouringOptions, synth
+    vals, dims, sp, org = synth.sphere(33, radius=0.3)
+    o = ContouringOptions()
+    o.method = ContouringMethod.Ours
+    o.outer_iters, o.inner_iters, o.batch_size = 2, 20, batch
+    be = B200DualContouringBackend(0, o)
+    V, F, _ = be.extract_tensor(vals.cuda(), dims, sp, org)
+    r = O.ours(vals.numpy(), dims, sp, org, outer_iters=2, inner_iters=20, batch_size=batch)
+    be.close()
+    assert np.array_equal(F.cpu().numpy(), r["F"])
+    assert np.abs(V.cpu().numpy().astype(np.float64) - r["V"]).max() <= 1e-5 * sp[0]
