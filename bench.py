@@ -27,11 +27,11 @@ import time
 ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, os.path.join(ROOT, "phanty-sdf-cuda_b200"))
 
-# Launches of the engine's own kernels per extraction: mark, 3 segment-scan passes, vertex
-# offsets, rank expansion, cell-width tables, QEF (with the edge normals), Jacobi list, FP64
-# vertices, 3 column-scan passes, face scatter, FP64 vertices for windings, FP64 windings,
+# Launches of the engine's own kernels per extraction: preparation (cell widths, cleared counters),
+# mark, 2 segment-scan passes, rank expansion, QEF (with the edge normals), Jacobi list, FP64
+# vertices, 2 column-scan passes, face scatter, FP64 vertices for windings, FP64 windings,
 # face order.
-KERNELS_PER_STEP = 17
+KERNELS_PER_STEP = 14
 # DRAM traffic of k_mark_zmarch per grid point, from a single-kernel ncu capture of the 512^3
 # CSG workload (dram__bytes_read.sum + dram__bytes_write.sum divided by the grid points of
 # that capture; the kernel streams the grid once, so traffic scales with the number of
@@ -518,7 +518,7 @@ def run_adjoint_workload(args):
     _side_line("dc_fwd_bwd_mcells_per_s", ncell / (ms_fb / 1e3) / 1e6, "Mcells/s", ms_fb, args,
                {"workload": "rbf_sphere128_adjoint", "grid": list(dims), "vertices": st.vertex_count,
                 "targets": 50000},
-               forward_ms=round(ms_f, 4), fwd_bwd_over_fwd=round(ms_fb / ms_f, 3), gpu_launches=KERNELS_PER_STEP + 5)
+               forward_ms=round(ms_f, 4), fwd_bwd_over_fwd=round(ms_fb / ms_f, 3), gpu_launches=KERNELS_PER_STEP + 4)
     be.close()
     return 0
 

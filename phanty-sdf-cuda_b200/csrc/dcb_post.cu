@@ -5,12 +5,12 @@
 // Stages, on one stream, with a few host reads of counts between them (sizes of what follows):
 //   weld     bounding box by ordered-integer atomics; the quantisation step in the reference's
 //            float expression order (one thread); a 51-bit grid-point key per vertex (17 bits per
-//            axis relative to the box's low corner: the box spans at most ~1e5 steps); a stable
-//            radix sort; the first vertex of each key represents it; representatives numbered by
-//            a scan in index order; faces remapped, those with < 3 distinct indices dropped with
+//            axis relative to the box's low corner: the box spans at most ~1e5 steps); a hash
+//            table of the keys; the first vertex of each key represents it; representatives
+//            numbered by a scan in index order; faces remapped, those with < 3 distinct indices dropped with
 //            the order kept (dc_backend.cpp:127-215).
-//   edges    the 4 edge uses of every face keyed by (min, max) vertex and radix sorted; a run of
-//            one use is a boundary edge, a run of two joins its faces in a union-find whose roots
+//   edges    the 4 edge uses of every face in buckets by smaller vertex; a run of one use of an
+//            edge is a boundary edge, a run of two joins its faces in a union-find whose roots
 //            are the smallest face index (dc_backend.cpp:231-310).
 //   keep     the component with the most faces, the one with the smallest first face on ties
 //            (the reference numbers components by their first face: dc_backend.cpp:312-361).

@@ -101,7 +101,7 @@ static __constant__ uint32_t c_edge_geo[12] = {edge_geo(0), edge_geo(1), edge_ge
 
 // Widths (and reciprocals) of the cells i-1, i, i+1 along each axis, exact float
 // differences of the float grid positions (the CPU forms positions the same way), read from
-// the per-grid tables of k_width_tables.
+// the per-grid tables of k_prepare.
 struct Widths {
     float w[3][3];   // [axis][offset+1]
     float r[3][3];
