@@ -270,8 +270,8 @@ k_radix_scatter(const K* __restrict__ kin, const uint32_t* __restrict__ vin, K* 
 // (4,000 boundary edges of 42 bits: 30 launches, 140 us).
 // Three stages of the network at a time: a thread takes the eight items they connect. Shared-memory
 // traffic bounds it (a stage at a time: 91 passes at 8,192 items); a word of padding per eight items
-// keeps the strides free of bank conflicts. Three sorts of a
-// 512^3 mesh (up to 8,192 edges): 168 us a stage at a time, now 110.
+// keeps the strides free of bank conflicts. The post-pass's three sorts of a 512^3 mesh: 168 us
+// a stage at a time, now 110.
 constexpr int kSortOne = 8192, kSortOneThreads = 1024, kSortOneSlots = kSortOne + kSortOne / 8;
 
 __device__ __forceinline__ int sort_slot(int i) { return i + (i >> 3); }
