@@ -293,6 +293,12 @@ constexpr int kBandCtasPerSm = 6;
 // sends more bins through several lists: 11.8 ms against 11.3 at 512^3).
 constexpr int kBandList = 336;
 constexpr int kBandTies = 7;       // triangles within the tie window of a point's minimum
+// Bricks that need the full walk have a bit each, by their number modulo kBandBits. Evenly spaced
+// bins have at most 15 points an axis (125 bricks, most bins 16); where the spacing is small
+// against the origin, positions round together and a bin can hold any number of points. So an item
+// is worked on in pieces of kBandPiece bricks, whose groups of kBandWarps fall on different bits.
+constexpr int kBandBits = 128, kBandPiece = kBandBits - kBandWarps;
+static_assert(kBandBits % 32 == 0 && 32 % kBandWarps == 0, "a group of bricks lies in one word");
 
 // Running closest-triangle state of one grid point: squared distance, closest point, summed normals.
 struct BandPoint {
@@ -411,7 +417,8 @@ struct BandShared {
     int seq_bin[27];
     uint32_t seq_start[28];
     uint32_t next, n, reach, votes[kBandWarps], brick_next;
-    uint32_t redo[4];              // bricks for the full walk (a bin has at most 15 points an axis: 125)
+    int piece;                     // of the item
+    uint32_t redo[kBandBits / 32]; // bricks of the piece for the full walk
     int brick[3];
 };
 
@@ -621,13 +628,15 @@ __global__ void __launch_bounds__(kBandThreads, kBandCtasPerSm) k_band(SdfParams
     const float far1 = (2.5f * P.min_box) * (2.5f * P.min_box);
     const float far2 = far1 > FLT_MIN && far1 < 1e37f ? far1 * 1.001f + 2.f * kWindow * tie_tol(far1) : kFar;
     const bool packed = P.gx <= kPackedBins && P.gy <= kPackedBins && P.gz <= kPackedBins;
+    if (threadIdx.x == 0) S.piece = 0;
     for (;;) {
         // next item from the shared work counter (bins differ a lot in cost: the parts of the long
         // ones come first, the others stand at the end of the list)
         __syncthreads();
-        if (threadIdx.x == 0) S.next = atomicAdd(P.work_next, 1u);
+        if (threadIdx.x == 0 && S.piece == 0) S.next = atomicAdd(P.work_next, 1u);
         __syncthreads();
         const uint32_t ai = S.next;
+        const int piece = S.piece;
         if (ai >= nitems) break;
         const uint2 item = P.items[ai < nlong ? ai : P.items_cap - 1 - (ai - nlong)];
         const long long bin = item.x;
@@ -664,22 +673,24 @@ __global__ void __launch_bounds__(kBandThreads, kBandCtasPerSm) k_band(SdfParams
             const int kx = (sx + 1 + t % 3) / (2 + t % 3), ky = (sy + 1 + t / 3 % 3) / (2 + t / 3 % 3),
                       kz = (sz + 1 + t / 9) / (2 + t / 9);
             const int wx = (sx + kx - 1) / kx, wy = (sy + ky - 1) / ky, wz = (sz + kz - 1) / kz;
-            int cost = t < 27 && wx * wy * wz <= 32 ? 32 * kx * ky * kz + t : 0x7fffffff;
+            const long long count = (long long)kx * ky * kz;
+            int cost = t < 27 && wx * wy * wz <= 32 ? 32 * (int)min(count, 0x3fffffdLL) + t : 0x7fffffff;
             const int mine_cost = cost;
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) cost = min(cost, __shfl_xor_sync(0xffffffffu, cost, o));
             if (mine_cost == cost) { S.brick[0] = wx; S.brick[1] = wy; S.brick[2] = wz; }
             if (t == 0) S.reach = __float_as_uint(kFar);
-            if (t < 4) S.redo[t] = 0;
+            if (t < kBandBits / 32) S.redo[t] = 0;
         }
         __syncthreads();
         const uint32_t L = S.seq_start[27];
         const int wx = S.brick[0], wy = S.brick[1], wz = S.brick[2];
         const int nbx = (sx + wx - 1) / wx, nby = (sy + wy - 1) / wy, nbz = (sz + wz - 1) / wz;
         const int nbricks = nbx * nby * nbz;
-        const int brick_lo = nbricks * part / parts, brick_hi = nbricks * (part + 1) / parts;
+        const int item_hi = (int)((long long)nbricks * (part + 1) / parts);
+        const int brick_lo = (int)((long long)nbricks * part / parts) + piece * kBandPiece, brick_hi = min(item_hi, brick_lo + kBandPiece);
         if (brick_lo >= brick_hi) continue;
-        if (threadIdx.x == 0) S.brick_next = brick_lo;
+        if (threadIdx.x == 0) { S.brick_next = brick_lo; S.piece = brick_hi < item_hi ? piece + 1 : 0; }
         const int zlo = z0 + wz * (brick_lo / (nbx * nby)), zhi = min(z0 + sz, z0 + wz * ((brick_hi - 1) / (nbx * nby) + 1)) - 1;
         // the item's points, and a bound of their distances: to the centroid nearest their middle
         const float3 blo = f3(P.ox + (float)x0 * P.vx, P.oy + (float)y0 * P.vy, P.oz + (float)zlo * P.vz);
@@ -895,7 +906,7 @@ __global__ void __launch_bounds__(kBandThreads, kBandCtasPerSm) k_band(SdfParams
         };
         auto finish = [&](int brick) {
             if (__ballot_sync(0xffffffffu, serial) && lane == 0 && brick < brick_hi)
-                atomicOr(&S.redo[brick >> 5], 1u << (brick & 31));
+                atomicOr(&S.redo[(brick & (kBandBits - 1)) >> 5], 1u << (brick & 31));
             if (mine) P.out[at] = val;
         };
         // With one list the warps take bricks as they come; with several they go through the
@@ -925,8 +936,8 @@ __global__ void __launch_bounds__(kBandThreads, kBandCtasPerSm) k_band(SdfParams
         }
         __syncthreads();
         if (S.redo[0] | S.redo[1] | S.redo[2] | S.redo[3]) {
-            for (int brick0 = 0; brick0 < nbricks; brick0 += kBandWarps) {
-                const uint32_t flags = (S.redo[brick0 >> 5] >> (brick0 & 31)) & ((1u << kBandWarps) - 1u);
+            for (int brick0 = brick_lo / kBandWarps * kBandWarps; brick0 < brick_hi; brick0 += kBandWarps) {
+                const uint32_t flags = (S.redo[(brick0 & (kBandBits - 1)) >> 5] >> (brick0 & 31)) & ((1u << kBandWarps) - 1u);
                 if (!flags) continue;
                 const bool want = (flags >> warp) & 1u;
                 take(brick0 + warp);
