@@ -260,14 +260,19 @@ __global__ void __launch_bounds__(256) k_bin_active(SdfParams P) {
     }
 }
 
-// First grid point along an axis whose bin coordinate is >= b (bins are monotone in the point
-// index); searched around the nominal b*n/g.
+// First grid point along an axis whose bin coordinate is >= b: bisection, since bins are monotone in
+// the point index. (Not a search from near the nominal b*n/g: where the spacing is small against the
+// origin, positions round together and a bin can begin any number of points earlier.)
 __device__ int first_point_of_bin(int b, int n, int g, float o, float v, float bd) {
     if (b <= 0) return 0;
     if (b >= g) return n;
-    int x = max(0, (int)(((long long)b * n) / g) - 3);
-    while (x < n && bin_coord(o + (float)x * v, o, bd, g) < b) ++x;
-    return x;
+    int lo = 0, hi = n;                          // the first one is in [lo, hi]
+    while (lo < hi) {
+        const int x = lo + (hi - lo) / 2;
+        if (bin_coord(o + (float)x * v, o, bd, g) < b) lo = x + 1;
+        else hi = x;
+    }
+    return lo;
 }
 
 // axis_start = [x: gx+1][y: gy+1][z: gz+1] first points of the bins along each axis.

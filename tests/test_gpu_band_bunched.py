@@ -1,6 +1,6 @@
 """The mesh -> SDF band kernel on grids whose spacing is small against the origin, so that points
-round to one position and a bin holds more of them than the 15 an axis of even spacing: more than
-128 bricks of points, repeats of the full walk among them. Its float operations are the oracle's,
+round to one position: a bin holds more of them than the 15 an axis of even spacing (more than 128
+bricks of points, repeats of the full walk among them) and begins far from its nominal first point. Its float operations are the oracle's,
 and ties only decide signs, so the values are equal."""
 import numpy as np
 import pytest
@@ -19,7 +19,22 @@ def _one_column():
     return V, F, (40, 40, 64), (0.0005, 0.0005, 0.004), (1e6, 1e6, 0.0)
 
 
-SCENES = {"one_column": _one_column}
+def _sheet(dims, sp, org, pitch):
+    """A wavy sheet across the grid's middle in z, facets of `pitch` a side."""
+    n = [int(np.ceil(d * h / pitch)) + 2 for d, h in zip(dims, sp)]
+    x, y = np.meshgrid(np.arange(n[0] + 1) * pitch - pitch, np.arange(n[1] + 1) * pitch - pitch, indexing="ij")
+    z = dims[2] * sp[2] * (0.5 + 0.15 * np.sin(3 * x / (dims[0] * sp[0])) * np.cos(4 * y / (dims[1] * sp[1])))
+    V = np.stack([x + org[0], y + org[1], z + org[2]], 2).reshape(-1, 3)
+    at = np.arange(V.shape[0]).reshape(n[0] + 1, n[1] + 1)
+    a, b, c, d = at[:-1, :-1].ravel(), at[1:, :-1].ravel(), at[1:, 1:].ravel(), at[:-1, 1:].ravel()
+    return V, np.concatenate([np.stack([a, b, c], 1), np.stack([a, c, d], 1)]), dims, sp, org
+
+
+# projected coordinates of a scan; every axis bunched
+SCENES = {"one_column": _one_column,
+          "scan": lambda: _sheet((256, 512, 64), (0.005,) * 3, (5e5, 4.2e6, 0.0), 0.05),
+          "cube64": lambda: _sheet((64, 64, 64), (0.001,) * 3, (1e6, 1e6, 1e6), 0.0625),
+          "cube100": lambda: _sheet((100, 100, 100), (0.01,) * 3, (1e7, 1e7, 1e7), 1.0)}
 
 
 @pytest.mark.parametrize("name", sorted(SCENES))
