@@ -1096,9 +1096,10 @@ k_sdf_relax(const __grid_constant__ SdfParams P, const float* __restrict__ in, i
     RelaxShared& S = *reinterpret_cast<RelaxShared*>(s_relax);
     const float inf = __int_as_float(0x7f800000);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int x = (int)blockIdx.x * kRelaxOwnW - kRelaxPasses + 2 * lane;
-    const int y0 = (int)blockIdx.y * kRelaxOwnH - kRelaxPasses + warp * kRelaxRows;
-    const int zlo = (int)blockIdx.z * depth, zhi = min(P.nz, zlo + depth);
+    const unsigned int ntx = (P.nx + kRelaxOwnW - 1) / kRelaxOwnW;          // x tiles fastest, then y
+    const int x = (int)(blockIdx.x % ntx) * kRelaxOwnW - kRelaxPasses + 2 * lane;
+    const int y0 = (int)(blockIdx.x / ntx) * kRelaxOwnH - kRelaxPasses + warp * kRelaxRows;
+    const int zlo = (int)blockIdx.y * depth, zhi = min(P.nz, zlo + depth);
     const float keep = fminf(P.vx, fminf(P.vy, P.vz)) * 1.5f;
     const bool inx[2] = {x >= 0 && x < P.nx, x + 1 >= 0 && x + 1 < P.nx};
     const bool ownx = lane >= kRelaxPasses / 2 && lane < 32 - kRelaxPasses / 2;
@@ -1342,8 +1343,7 @@ cudaError_t launch_sdf_finish(const SdfParams& P, const float* band, unsigned lo
     while ((P.nz + depth - 1) / depth > 65535) depth *= 2;
     cudaError_t e = cudaFuncSetAttribute(k_sdf_relax, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RelaxShared));
     if (e != cudaSuccess) return e;
-    const dim3 grid((unsigned)((P.nx + kRelaxOwnW - 1) / kRelaxOwnW), (unsigned)((P.ny + kRelaxOwnH - 1) / kRelaxOwnH),
-                    (unsigned)((P.nz + depth - 1) / depth));
+    const dim3 grid((unsigned)tiles, (unsigned)((P.nz + depth - 1) / depth));     // 65,535 at most in y
     k_sdf_relax<<<grid, kRelaxThreads, sizeof(RelaxShared), s>>>(P, band, depth, filled);
     return cudaGetLastError();
 }
