@@ -1501,7 +1501,7 @@ int dcb_copy_mesh_device(dcb_handle h, float* vertices, int32_t* faces, void* cu
     const long long nv = vertices ? 3 * h->nv : 0, nf = faces ? (long long)h->vpf * h->nf : 0;
     if (nv || nf)
         DCB_TRY(h, launch_copy_mesh(as<float>(h->V), nv ? vertices : nullptr, nv, nf ? face_ptr(h) : nullptr, nf ? faces : nullptr,
-                                    nf, h->num_sms, s), "copy mesh");
+                                    nf, h->device, h->num_sms, s), "copy mesh");
     return DCB_OK;
 }
 

@@ -448,9 +448,18 @@ __global__ void __launch_bounds__(256) k_copy_mesh(const float* __restrict__ V, 
     if (first < nf % 4) out_F[nf - 1 - first] = F[nf - 1 - first];
 }
 
-cudaError_t launch_copy_mesh(const float* V, float* out_V, long long nv, const int* F, int* out_F, long long nf, int num_sms,
-                             cudaStream_t s) {
-    if (((uintptr_t)V | (uintptr_t)out_V | (uintptr_t)F | (uintptr_t)out_F) % 16) {     // a caller's odd array
+// Whether a kernel may store to p: memory of this GPU. (Another GPU's may not be mapped here; the copy
+// engine reaches it, and refuses what is no device memory.)
+static bool own_memory(const void* p, int device) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) { cudaGetLastError(); return false; }
+    return a.type == cudaMemoryTypeDevice && a.device == device;
+}
+
+cudaError_t launch_copy_mesh(const float* V, float* out_V, long long nv, const int* F, int* out_F, long long nf, int device,
+                             int num_sms, cudaStream_t s) {
+    const bool odd = ((uintptr_t)V | (uintptr_t)out_V | (uintptr_t)F | (uintptr_t)out_F) % 16 != 0;
+    if (odd || (nv && !own_memory(out_V, device)) || (nf && !own_memory(out_F, device))) {
         cudaError_t e = nv ? cudaMemcpyAsync(out_V, V, sizeof(float) * nv, cudaMemcpyDeviceToDevice, s) : cudaSuccess;
         if (e == cudaSuccess && nf) e = cudaMemcpyAsync(out_F, F, sizeof(int) * nf, cudaMemcpyDeviceToDevice, s);
         return e;

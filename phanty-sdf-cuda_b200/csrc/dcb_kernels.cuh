@@ -112,10 +112,11 @@ cudaError_t launch_vert_offsets(const BatchTable& B, const uint32_t* seg_start, 
 // face_off[b] = col_start[col_off[b]] (b < n), face_off[n] = total.
 cudaError_t launch_face_offsets(const BatchTable& B, const uint32_t* col_start, const unsigned long long* total,
                                 unsigned long long* face_off, cudaStream_t s);
+// Vertices (nv floats) and faces (nf ints) to the caller's device arrays: in one launch where the
+// arrays are aligned and on `device`, the mesh's own; else by the copy engine.
+cudaError_t launch_copy_mesh(const float* V, float* out_V, long long nv, const int* F, int* out_F, long long nf, int device,
+                             int num_sms, cudaStream_t s);
 // Global vertex ranks in the faces -> ranks within each face's grid (vpf ints per face).
-// Vertices (nv floats) and faces (nf ints) to the caller's device arrays in one launch.
-cudaError_t launch_copy_mesh(const float* V, float* out_V, long long nv, const int* F, int* out_F, long long nf, int num_sms,
-                             cudaStream_t s);
 cudaError_t launch_localize_faces(const unsigned long long* vert_off, const unsigned long long* face_off, int n,
                                   int* faces, int vpf, long long max_faces, int num_sms, cudaStream_t s);
 
