@@ -71,7 +71,7 @@ struct PostCounters {
     unsigned long long cursor;          // ring vertices reserved in the fill scratch
     unsigned long long nrings;          // ring records written
     unsigned int nlong;                 // vertices with long edge buckets
-    unsigned int ntoo_long;             // of them beyond what a block compares
+    unsigned int ntoo_long;             // of them beyond what a block sorts
     int linked[8];                      // round r of the face links changed something
     int fill_overflow;                  // the scratch or the record list was too small
     int pad3;
@@ -322,9 +322,11 @@ __global__ void k_edge_runs(EdgeRunParams P) {
 // ---- the same from buckets: edge uses grouped by the edge's smaller vertex (about four a vertex on
 // a mesh), so that a thread finds the runs among its vertex's few uses. A radix sort of the
 // uses by both vertices took six passes of five launches (512^3 CSG: 0.9 ms). No order of the runs
-// or in them reaches the output. Vertices with more than kBucketFew uses are taken by a block each;
-// beyond kBucketMany the sorted form above serves the whole mesh.
+// or in them reaches the output. Vertices with more than kBucketFew uses are taken by a block each,
+// which sorts them in shared memory; beyond kBucketMany (its 64 KB) the sorted form above serves the
+// whole mesh.
 constexpr unsigned int kBucketFew = 32, kBucketMany = 8192;
+constexpr int kLongThreads = 512, kLongBytes = kBucketMany * sizeof(unsigned long long);
 
 struct BucketParams {
     const int4* Fw;
@@ -387,11 +389,42 @@ __global__ void k_bucket_runs(BucketParams P, EdgeRunParams E) {
     }
 }
 
-__global__ void k_bucket_long(BucketParams P, EdgeRunParams E) {
+// A bitonic network orders the uses by larger vertex; a use's neighbours then tell whether its edge has
+// one, two or more. (Each use compared with all others, as a thread does for few, took 0.36 ms for a
+// fan of 1,000 uses, 1.0 for 2,000 and 14 for 8,000.)
+__global__ void __launch_bounds__(kLongThreads) k_bucket_long(BucketParams P, EdgeRunParams E) {
+    extern __shared__ unsigned long long s_use[];               // larger vertex << 32 | place in the bucket
     for (unsigned int w = blockIdx.x; w < P.C->nlong; w += gridDim.x) {
         const unsigned int u = P.longs[w], n = P.count[u], at = P.start[u];
         if (n > kBucketMany) continue;
-        for (unsigned int x = threadIdx.x; x < n; x += blockDim.x) bucket_use(P, E, P.use + at, P.pair + at, n, x);
+        unsigned int size = 2;
+        while (size < n) size *= 2;
+        __syncthreads();
+        for (unsigned int x = threadIdx.x; x < size; x += kLongThreads)
+            s_use[x] = x < n ? (unsigned long long)P.use[at + x].x << 32 | x : ~0ull;
+        for (unsigned int k = 2; k <= size; k *= 2)
+            for (unsigned int j = k / 2; j > 0; j /= 2) {
+                __syncthreads();
+                for (unsigned int t = threadIdx.x; t < size / 2; t += kLongThreads) {
+                    const unsigned int lo = 2 * t - (t & (j - 1));
+                    const unsigned long long a = s_use[lo], b = s_use[lo + j];
+                    if ((a > b) == ((lo & k) == 0)) { s_use[lo] = b; s_use[lo + j] = a; }
+                }
+            }
+        __syncthreads();
+        for (unsigned int x = threadIdx.x; x < n; x += kLongThreads) {
+            auto same = [&](unsigned int y) { return (s_use[y] >> 32) == (s_use[x] >> 32); };
+            const bool prev = x > 0 && same(x - 1), next = x + 1 < n && same(x + 1);
+            const bool many = prev ? next || (x > 1 && same(x - 2)) : next && x + 2 < n && same(x + 2);
+            const int use = (int)P.use[at + (unsigned int)s_use[x]].y;
+            int2 both = make_int2(-1, -1);
+            if (many ? E.close && E.remove : !prev && !next) push_boundary(E, use);
+            if (next && !prev && !many) {
+                both = make_int2(use >> 2, (int)(P.use[at + (unsigned int)s_use[x + 1]].y >> 2));
+                if (E.remove && both.x != both.y) atomicMin(&P.parent[max(both.x, both.y)], min(both.x, both.y));
+            }
+            P.pair[at + x] = both;
+        }
     }
 }
 
@@ -1183,7 +1216,8 @@ cudaError_t post_run(PostWork& W, PostRun& R, cudaStream_t s) {
         PP_TRY(exclusive_sum(W.scratch.p, W.scratch.bytes, bp.count, as<unsigned int>(W.u2), nvw, s));
         k_bucket_uses<true><<<grid_for(nfw, kThreads, sms), kThreads, 0, s>>>(bp);
         k_bucket_runs<<<grid_for(nvw, kThreads, sms), kThreads, 0, s>>>(bp, ep);
-        k_bucket_long<<<(unsigned)sms, kThreads, 0, s>>>(bp, ep);
+        PP_TRY(cudaFuncSetAttribute(k_bucket_long, cudaFuncAttributeMaxDynamicSharedMemorySize, kLongBytes));
+        k_bucket_long<<<(unsigned)sms * 2, kLongThreads, kLongBytes, s>>>(bp, ep);
         if (R.remove_floaters) {
             k_flatten<<<grid_for(nfw, kThreads, sms), kThreads, 0, s>>>(parent, nfw);
             for (int r = 0; r < kLinkRounds; ++r) {
@@ -1214,7 +1248,7 @@ cudaError_t post_run(PostWork& W, PostRun& R, cudaStream_t s) {
     e = read_counters(W, R, s);
     if (e != cudaSuccess) return e;
     if (host_counters(W).ntoo_long) {
-        // a vertex with more uses than a block compares: everything again from the sorted uses
+        // a vertex with more uses than a block sorts: everything again from the sorted uses
         PP_TRY(grow(W.val, sizeof(int) * ne));
         PP_TRY(grow(W.val2, sizeof(int) * ne));
         PP_TRY(grow(W.scratch, std::max(radix_sort_temp_bytes(ne, 8, true), select_temp_bytes(nfw))));
