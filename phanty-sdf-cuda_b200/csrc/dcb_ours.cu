@@ -1303,11 +1303,9 @@ size_t ours_workspace_bytes(long long nv, long long nq, long long npts, size_t* 
     b += al(sizeof(OursCell) * nv) + al(sizeof(double) * 3 * nv);            // cells, Vm
     b += al(sizeof(int4) * nq) + al(sizeof(double) * 3 * nq);               // quads, gsum
     b += 3 * al(sizeof(uint32_t) * npts) + al(sizeof(int) * npts);           // sel, band/rest, sel_cell
-    b += al(sizeof(unsigned long long) * npts) * 2 + al(sizeof(uint32_t) * npts);  // fill keys/values
+    b += al(sizeof(unsigned long long) * 2 * npts) + al(sizeof(uint32_t) * npts);  // fill keys/values; sphere centres, long searches
     b += 3 * al(sizeof(unsigned int) * (nv + 1)) + al(sizeof(uint32_t) * npts);    // count/start/fill, spheres
-    b += al(sizeof(float4) * npts);                                          // their centres
     b += 3 * al(sizeof(uint32_t) * (nv + 1));                                // cells by number of spheres
-    b += al(sizeof(uint32_t) * npts);                                        // points with long searches
     b += al(sizeof(uint32_t) * npts);                                        // selected points, sorted
     b += al(sizeof(int) * npts);                                             // last closest triangle per point
     b += al(sizeof(unsigned long long) * nt) + al(sizeof(BvhNode) * nt) + al(sizeof(int) * 2 * nt);
@@ -1333,16 +1331,19 @@ cudaError_t ours_run(OursRun& R, cudaStream_t s) {
     uint32_t* band = (uint32_t*)take(sizeof(uint32_t) * npts);
     uint32_t* rest = (uint32_t*)take(sizeof(uint32_t) * npts);
     P.sel_cell = (int*)take(sizeof(int) * npts);
-    unsigned long long* fk = (unsigned long long*)take(sizeof(unsigned long long) * npts);
-    unsigned long long* fk2 = (unsigned long long*)take(sizeof(unsigned long long) * npts);
+    // the keys and values of the selection are done with when the queries begin; the spheres'
+    // centres and the list of long searches then take their place
+    unsigned long long* fk = (unsigned long long*)take(sizeof(unsigned long long) * 2 * npts);
+    unsigned long long* fk2 = fk + npts;
     uint32_t* fv2 = (uint32_t*)take(sizeof(uint32_t) * npts);
+    P.cell_centres = (float4*)fk;
+    P.long_query = fv2;
+    static_assert(sizeof(float4) == 2 * sizeof(unsigned long long), "");
     P.cell_count = (unsigned int*)take(sizeof(unsigned int) * (nv + 1));
     P.cell_start = (unsigned int*)take(sizeof(unsigned int) * (nv + 1));
     P.cell_fill = (unsigned int*)take(sizeof(unsigned int) * (nv + 1));
     P.cell_spheres = (uint32_t*)take(sizeof(uint32_t) * npts);
-    P.cell_centres = (float4*)take(sizeof(float4) * npts);
     for (int q = 0; q < 3; ++q) P.team_list[q] = (uint32_t*)take(sizeof(uint32_t) * (nv + 1));
-    P.long_query = (uint32_t*)take(sizeof(uint32_t) * npts);
     P.mkeys_sorted = (unsigned long long*)take(sizeof(unsigned long long) * nt);
     P.tcode = (uint32_t*)take(sizeof(uint32_t) * nt);
     P.tidx = (uint32_t*)take(sizeof(uint32_t) * nt);
