@@ -1005,6 +1005,7 @@ struct SdfCounters {
     int err;
     int changed;
     unsigned long long total_entries;
+    unsigned long long scanned_entries;   // the same modulo 2^32
     unsigned long long exterior;
     unsigned int item_counts[2];
     unsigned int work_next;
@@ -1051,7 +1052,7 @@ int run_mesh_sdf(dcb_context* h, const float* d_verts, int64_t nv, const int32_t
     P.bin_count = as<uint32_t>(h->m_bin_count); P.bin_start = as<uint32_t>(h->m_bin_start);
     P.bin_fill = as<uint32_t>(h->m_bin_fill); P.axis_start = as<int>(h->m_axis_start);
     P.far = as<uint32_t>(h->m_far); P.ext = as<uint32_t>(h->m_ext); P.err = &dc->err;
-    P.item_counts = dc->item_counts; P.work_next = &dc->work_next;
+    P.item_counts = dc->item_counts; P.work_next = &dc->work_next; P.entries = &dc->total_entries;
 
     cudaEvent_t* ev = h->ev;
     DCB_TRY(h, cudaEventRecord(ev[0], s), "event");
@@ -1059,7 +1060,7 @@ int run_mesh_sdf(dcb_context* h, const float* d_verts, int64_t nv, const int32_t
     DCB_TRY(h, cudaMemsetAsync(P.bin_count, 0, sizeof(uint32_t) * P.nbins, s), "memset");
     DCB_TRY(h, cudaMemsetAsync(P.bin_fill, 0, sizeof(uint32_t) * P.nbins, s), "memset");
     DCB_TRY(h, launch_sdf_prep(P, h->num_sms, s), "launch triangle records");
-    DCB_TRY(h, launch_scan(P.bin_count, P.nbins, as<uint32_t>(h->m_partials), P.bin_start, &dc->total_entries, s),
+    DCB_TRY(h, launch_scan(P.bin_count, P.nbins, as<uint32_t>(h->m_partials), P.bin_start, &dc->scanned_entries, s),
             "launch bin scan");
     DCB_TRY(h, cudaMemcpyAsync(hc, dc, sizeof(SdfCounters), cudaMemcpyDeviceToHost, s), "read counters");
     DCB_TRY(h, cudaStreamSynchronize(s), "bins");

@@ -366,6 +366,7 @@ struct SdfParams {
     long long nv, nf;
     float* tris;                   // sdf_tri_record_bytes() per triangle
     uint32_t* bin_count;
+    unsigned long long* entries;   // sum of the counts
     uint32_t* bin_start;
     uint32_t* bin_fill;
     uint32_t* bin_scratch;         // bin entries as scattered

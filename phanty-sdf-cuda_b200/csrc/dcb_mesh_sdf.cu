@@ -147,6 +147,7 @@ __device__ __forceinline__ bool load_tri(const SdfParams& P, long long f, float3
 }
 
 __global__ void __launch_bounds__(256) k_tri_prep(SdfParams P) {
+    unsigned long long entries = 0;
     for (long long f = (long long)blockIdx.x * blockDim.x + threadIdx.x; f < P.nf; f += (long long)gridDim.x * blockDim.x) {
         float3 a, b, c;
         if (!load_tri(P, f, a, b, c)) continue;
@@ -172,11 +173,16 @@ __global__ void __launch_bounds__(256) k_tri_prep(SdfParams P) {
         t[4] = make_float4(c.z, n.x, n.y, n.z);
         t[kTriAngles] = make_float4(angle_at(sub(b, a), sub(c, a), a2), angle_at(sub(a, b), sub(c, b), a2),
                                     angle_at(sub(a, c), sub(b, c), a2), 0.f);
+        entries += (unsigned long long)(r[1] - r[0] + 1) * (unsigned)(r[3] - r[2] + 1) * (unsigned)(r[5] - r[4] + 1);
         for (int bz = r[4]; bz <= r[5]; ++bz)
             for (int by = r[2]; by <= r[3]; ++by)
                 for (int bx = r[0]; bx <= r[1]; ++bx)
                     atomicAdd(&P.bin_count[bx + (long long)P.gx * (by + (long long)P.gy * bz)], 1u);
     }
+    // their number in 64 bits (the bins' starts have 32: the host refuses more)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) entries += __shfl_xor_sync(0xffffffffu, entries, o);
+    if ((threadIdx.x & 31) == 0 && entries) atomicAdd(P.entries, entries);
 }
 
 __global__ void __launch_bounds__(256) k_tri_bins(SdfParams P) {
