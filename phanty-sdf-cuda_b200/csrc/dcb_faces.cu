@@ -24,7 +24,7 @@ namespace dcb {
 // Up to kScanOne counts: one block. More: the blocks' sums, then every block adds up the sums
 // before its own and places its counts (two launches; the sums are few and in L2). Beyond
 // kScanFew blocks that repeated addition would read more than the counts, so a block scans the
-// sums in between. A grid of 32^3 points has 961 and 2,883 counts to scan: 3.6 us each in one
+// sums in between. Places have 32 bits, the total 64: it tells the caller when they do not suffice. A grid of 32^3 points has 961 and 2,883 counts to scan: 3.6 us each in one
 // block, 5.8 and two gaps in three launches.
 
 constexpr int kScanThreads = 256;
@@ -106,13 +106,13 @@ k_scan_partials(const uint32_t* __restrict__ in, long long n, const unsigned lon
 __global__ void __launch_bounds__(kScanThreads)
 k_scan_single(uint32_t* partials, long long nb, unsigned long long* grand_total) {
     __shared__ uint32_t s_warp[kScanThreads / 32];
-    uint32_t carry = 0;
+    unsigned long long carry = 0;
     for (long long c0 = 0; c0 < nb; c0 += kScanThreads) {
         const long long idx = c0 + threadIdx.x;
         const uint32_t v = idx < nb ? partials[idx] : 0u;
         uint32_t total;
         const uint32_t ex = block_excl_scan(v, s_warp, total);
-        if (idx < nb) partials[idx] = carry + ex;
+        if (idx < nb) partials[idx] = (uint32_t)carry + ex;
         carry += total;
     }
     if (threadIdx.x == 0) *grand_total = carry;
@@ -128,12 +128,12 @@ k_scan_apply(const uint32_t* __restrict__ in, long long n, const unsigned long l
     __shared__ uint32_t s_warp[kScanThreads / 32];
     const long long base = (long long)blockIdx.x * kScanTile + (long long)threadIdx.x * kScanItems;
     uint32_t before = 0;
+    unsigned long long wide = 0;                       // this thread's part of the sums before
     if (SUMMED) {
         before = partials[blockIdx.x];
     } else {
-        uint32_t mine = 0;
-        for (unsigned q = threadIdx.x; q < blockIdx.x; q += kScanThreads) mine += partials[q];
-        block_excl_scan(mine, s_warp, before);
+        for (unsigned q = threadIdx.x; q < blockIdx.x; q += kScanThreads) wide += partials[q];
+        block_excl_scan((uint32_t)wide, s_warp, before);
     }
     uint32_t v[kScanItems], s = 0;
     load_counts(in, base, n, v);
@@ -145,7 +145,12 @@ k_scan_apply(const uint32_t* __restrict__ in, long long n, const unsigned long l
     for (int q = 0; q < kScanItems; ++q) { const uint32_t c = v[q]; v[q] = run; run += c; }
     store_counts(out, base, n, v);
     store_counts(copy, base, n, v);
-    if (!SUMMED && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *grand_total = before + total;
+    if (!SUMMED && blockIdx.x == gridDim.x - 1) {
+        uint32_t low, high;                            // a thread's part is eight sums at most: 35 bits
+        block_excl_scan((uint32_t)wide & 0xffffu, s_warp, low);
+        block_excl_scan((uint32_t)(wide >> 16), s_warp, high);
+        if (threadIdx.x == 0) *grand_total = ((unsigned long long)high << 16) + low + total;
+    }
 }
 
 __global__ void __launch_bounds__(kScanOneThreads)
@@ -153,7 +158,7 @@ k_scan_one(const uint32_t* __restrict__ in, long long n, const unsigned long lon
            uint32_t* __restrict__ copy, unsigned long long* grand_total) {
     n = scan_length(n, live);
     __shared__ uint32_t s_warp[kScanOneThreads / 32];
-    uint32_t carry = 0;
+    unsigned long long carry = 0;
     for (long long c0 = 0; c0 < n; c0 += kScanOneThreads * kScanOneItems) {
         const long long base = c0 + (long long)threadIdx.x * kScanOneItems;
         uint32_t v[kScanOneItems], s = 0;
@@ -161,7 +166,7 @@ k_scan_one(const uint32_t* __restrict__ in, long long n, const unsigned long lon
 #pragma unroll
         for (int q = 0; q < kScanOneItems; ++q) s += v[q];
         uint32_t total;
-        uint32_t run = block_excl_scan<kScanOneThreads>(s, s_warp, total) + carry;
+        uint32_t run = block_excl_scan<kScanOneThreads>(s, s_warp, total) + (uint32_t)carry;
 #pragma unroll
         for (int q = 0; q < kScanOneItems; ++q) { const uint32_t c = v[q]; v[q] = run; run += c; }
         store_counts(out, base, n, v);
