@@ -304,10 +304,12 @@ __global__ void k_ours_point_keys(OursParams P, const uint32_t* sel, long long n
 // its order does not matter. A histogram of the keys' first 12 bits gives the bin that the last
 // one lies in; keys below it are taken, those in it listed, and one block selects among them.
 // Instead of a 64-bit sort of all candidates: 0.41 ms of an outer iteration at 128^3 (two
-// million candidates), now 0.04. Sorted by Morton code afterwards
-// only beyond 8,192 points: below, the sort of the fill (0.12 ms) costs more than the nearness of
-// a warp's queries saves (at 128^3; with 100,000 points the queries take 0.2 ms longer unsorted).
-constexpr long long kFillUnsorted = 8192;
+// million candidates), now 0.04. Sorted by Morton code afterwards only beyond kFillUnsorted points:
+// below, the sort costs more than the nearness of a warp's queries saves. An outer iteration of
+// 128^3 with a fill of 8,000, 16,000, 32,000, 64,000, 128,000 points, sorted: 1.79, 2.08, 2.35, 3.15,
+// 4.41 ms; unsorted: 1.73, 1.96, 2.24, 3.07, 4.43. At 80^3 and 192^3 the lines cross between the same
+// two sizes.
+constexpr long long kFillUnsorted = 98304;
 constexpr int kFillBins = 4096, kFillThreads = 256, kFillDigit = 11;
 
 __device__ __forceinline__ unsigned long long fill_key(unsigned long long seed, int it, uint32_t point) {
