@@ -9,10 +9,10 @@ its own grid: weak scaling, no collective on the data path).
     python bench.py [--gpus N] [--steps K] [--warmup W] [--res 1024] [--impl reference]
 
 Under torchrun each rank runs on its LOCAL_RANK GPU; rank 0 prints one JSON line.
-``--impl reference`` times the CPU oracle (the FP64 restatement of the reference's
-CpuDualContouringBackend, which is single-threaded C++ in the reference and cannot be
-built here: it needs Eigen and libigl) with every host thread on a bounded sample of the
-same grid (8 z-slabs spread evenly over it), and reports the same metric.
+``--impl reference`` times the reference's own CPU backend (CpuDualContouringBackend::extract,
+compiled from its sources into oracle/_ref/ref_cpu_dc) on a bounded sample of the same grid, one
+process per host core, and reports the same metric; where that program was not built it prints
+that the reference is unavailable.
 """
 import argparse
 import json
@@ -312,70 +312,45 @@ def _sample_text(dims, ranges, cells, res):
 def run_reference(args, rank, world):
     """CPU reference arm: the reference's own CPU backend (CpuDualContouringBackend::extract,
     compiled from its sources into oracle/_ref/ref_cpu_dc) on a bounded sample of the same grid,
-    one process per host core; where that program was not built, the oracle port with all host
-    threads on evenly spread z-slabs."""
+    one process per host core."""
     import numpy as np
     from contouring_b200 import synth
     if rank != 0:
         return 0
+    if not os.path.exists(REF_CPU_DC):
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's own CPU backend (oracle/_ref/ref_cpu_dc) was "
+                          "not built: its sources are not here"}), flush=True)
+        return 0
     threads = os.cpu_count() or 1
     dims = (args.res,) * 3
-    if os.path.exists(REF_CPU_DC):
-        import tempfile
-        ncube = max(1, min(threads, 16))
-        origins = cube_origins(args.res, ncube)
-        spacing = origin = None
+    ncube = max(1, min(threads, 16))
+    origins = cube_origins(args.res, ncube)
+    spacing = origin = None
 
-        def cube(i0, j0, k0):
-            nonlocal spacing, origin
-            v, _, spacing, origin = synth.csg(args.res, seed=0, device="cpu", planes=(k0, k0 + REF_CUBE))
-            return v.numpy().reshape(REF_CUBE, args.res, args.res)[:, j0:j0 + REF_CUBE, i0:i0 + REF_CUBE].copy()
+    def cube(i0, j0, k0):
+        nonlocal spacing, origin
+        v, _, spacing, origin = synth.csg(args.res, seed=0, device="cpu", planes=(k0, k0 + REF_CUBE))
+        return v.numpy().reshape(REF_CUBE, args.res, args.res)[:, j0:j0 + REF_CUBE, i0:i0 + REF_CUBE].copy()
 
-        with tempfile.TemporaryDirectory() as td:
-            cubes = [cube(*o) for o in origins]
-            paths, cells = ref_cpu_cubes(lambda i0, j0, k0: cubes[origins.index((i0, j0, k0))], origins,
-                                         spacing, origin, td)
-            for _ in range(args.warmup):
-                ref_cpu_run(paths, td)
-            secs = [ref_cpu_run(paths, td) for _ in range(args.steps)]
-        dt = float(np.median(secs))
-        value = cells / dt / 1e6
-        sample = _ref_sample_text(ncube, args.res, cells)
-        line = {
-            "metric": "dc_extract_mcells_per_s", "value": round(value, 4), "unit": "Mcells/s",
-            "impl": "reference", "n_gpus": args.gpus, "steps": args.steps, "warmup": args.warmup,
-            "ms_per_step": round(1000 * dt, 3), "higher_is_better": True,
-            "scaling": "weak", "vs_baseline": None, "dtype": "f64", "data": "synthetic",
-            "config": {"workload": "csg%d_dense_dc" % args.res, "grid": list(dims), "sample": sample},
-            "cpu_baseline": {"value": round(value, 4), "unit": "Mcells/s", "cores": ncube,
-                             "kind": "reference", "sample": sample},
-            "e2e": {"value": round(value, 4), "unit": "Mcells/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
-        }
-        print(json.dumps(line), flush=True)
-        return 0
-    ranges = slab_ranges(args.res, args.ref_zslab)
-    slabs = []
-    for r in ranges:
-        v, _, spacing, origin = synth.csg(args.res, seed=0, device="cpu", planes=r)
-        slabs.append((r, v.numpy()))
-    for _ in range(args.warmup):
-        cpu_sample(slabs, dims, spacing, origin, threads)
-    rates, secs = [], []
-    for _ in range(args.steps):
-        rate, dt, cells = cpu_sample(slabs, dims, spacing, origin, threads)
-        rates.append(rate)
-        secs.append(dt)
-    value = float(np.median(rates))
-    sample = _sample_text(dims, ranges, cells, args.res)
+    with tempfile.TemporaryDirectory() as td:
+        cubes = [cube(*o) for o in origins]
+        paths, cells = ref_cpu_cubes(lambda i0, j0, k0: cubes[origins.index((i0, j0, k0))], origins,
+                                     spacing, origin, td)
+        for _ in range(args.warmup):
+            ref_cpu_run(paths, td)
+        secs = [ref_cpu_run(paths, td) for _ in range(args.steps)]
+    dt = float(np.median(secs))
+    value = cells / dt / 1e6
+    sample = _ref_sample_text(ncube, args.res, cells)
     line = {
-        "metric": "dc_extract_mcells_per_s", "value": round(value, 3), "unit": "Mcells/s",
+        "metric": "dc_extract_mcells_per_s", "value": round(value, 4), "unit": "Mcells/s",
         "impl": "reference", "n_gpus": args.gpus, "steps": args.steps, "warmup": args.warmup,
-        "ms_per_step": round(1000 * float(np.median(secs)), 3), "higher_is_better": True,
+        "ms_per_step": round(1000 * dt, 3), "higher_is_better": True,
         "scaling": "weak", "vs_baseline": None, "dtype": "f64", "data": "synthetic",
         "config": {"workload": "csg%d_dense_dc" % args.res, "grid": list(dims), "sample": sample},
-        "cpu_baseline": {"value": round(value, 3), "unit": "Mcells/s", "cores": threads,
-                         "kind": "port", "sample": sample},
-        "e2e": {"value": round(value, 3), "unit": "Mcells/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
+        "cpu_baseline": {"value": round(value, 4), "unit": "Mcells/s", "cores": ncube,
+                         "kind": "reference", "sample": sample},
+        "e2e": {"value": round(value, 4), "unit": "Mcells/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
     }
     print(json.dumps(line), flush=True)
     return 0
