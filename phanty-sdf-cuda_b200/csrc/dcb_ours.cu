@@ -1026,10 +1026,10 @@ __device__ void inner_solve(const OursParams& P, const double Acc[9], const doub
 // of 100 iterations, a chain each. An outer iteration of a 128^3 perturbed sphere takes 2.7 ms
 // (72^3, with cells of up to 1,600 spheres: 5.3; a 128^3 sphere 0.6). A team of 8 lanes per cell,
 // each lane solving, took 4.7 (6.8): half the instructions were the same solves again, and 10 of
-// 32 lanes were active (now 20). 28 slots because all cells of such grids are then in flight at
-// once (32: 2.8, 24 with five blocks an SM 2.8); 8 or 16 cells to a warp without block
-// synchronisations: 5.0 (a warp's chain is too long); four lanes a sphere: 3.0-3.4. The cells are
-// dealt by columns so that no block gets the large ones (taken in list order: 3.0).
+// 32 lanes were active (now 20). 28 slots as measured (32: 2.8; 24 with five blocks an SM: 2.8);
+// 8 or 16 cells to a warp without block synchronisations: 5.0 (a warp's chain is too long); four
+// lanes a sphere: 3.0-3.4. The cells are dealt by columns so that no block gets the large ones
+// (taken in list order: 3.0).
 constexpr int kInnerThreads = 128;
 constexpr int kSlots = 28;                 // a lane of the solving warp each
 constexpr unsigned int kRows = 512;

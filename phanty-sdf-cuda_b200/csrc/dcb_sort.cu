@@ -1,6 +1,7 @@
 // dcb_sort.cu — device-wide sort, scan and selection of the mesh post-pass (dcb_post.cu) and the
 // vertex refinement (dcb_ours.cu): a stable LSD radix sort over 8-bit digits (keys alone or
-// with 32-bit values), exclusive and inclusive sums, and flagged selection. Every primitive is a
+// with 32-bit values), exclusive and inclusive sums, and flagged selection. Sorts of up to kSortOne
+// (8,192) items are one block's bitonic network (k_sort_one); every other primitive is a
 // fixed sequence of launches with no waits between blocks: a per-tile count, a scan of the
 // counts, a per-tile placement. Inputs are left unmodified; the scratch space comes from the
 // caller (the *_temp_bytes functions give its size).

@@ -6,7 +6,7 @@
 //
 // Per cell: the Hermite samples (with the three neighbours' own samples of an averaged edge),
 // then A^T A, A^T b and the centroid summed in edge order (the CPU's std::map order), the
-// Jacobi eigen-decomposition and the truncated pseudo-inverse; a lane per (cell, crossing
+// Jacobi eigen-decomposition and the truncated pseudo-inverse; four lanes per (cell, crossing
 // edge) and a lane per solve when cells are few, a thread per cell when many.
 #include "dcb_f64.cuh"
 
