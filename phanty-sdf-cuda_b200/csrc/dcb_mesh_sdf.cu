@@ -45,13 +45,14 @@ namespace {
 
 constexpr float kFar = FLT_MAX;
 
-// Triangle record, 6 x 16 bytes.
+// Triangle record, 6 x 16 bytes. Behind the records: every triangle's unit normal (within them it would
+// take 2 to 4% of the band's time at 100^3: records of 112 or 128 bytes).
 struct Tri {
     float4 s;       // bounding sphere: centroid xyz, radius grown by a rounding allowance
     float a2;       // doubled area (0: skipped, as the reference skips area <= 1e-12)
     uint32_t r[3];  // bins it is listed in, per axis: first | last << 16 (kPackedBins axes and below)
     float v[9];     // vertices
-    float n[3];     // unit normal
+    float n[3];     // unit normal; 0 where it bounds no distance (a thin triangle's)
     float w[4];     // tie weights of its vertices: the angles there
 };
 constexpr int kTriF4 = 6;
@@ -170,9 +171,14 @@ __global__ void __launch_bounds__(256) k_tri_prep(SdfParams P) {
                            __uint_as_float((uint32_t)r[4] | (uint32_t)r[5] << 16));
         t[2] = make_float4(a.x, a.y, a.z, b.x);
         t[3] = make_float4(b.y, b.z, c.x, c.y);
-        t[4] = make_float4(c.z, n.x, n.y, n.z);
+        // The float normal is off by up to 3 sqrt(3) ulps (2^-24) of the longest edge's square over
+        // the doubled area, the edge being two radii at most: the triangle leaves the plane by that
+        // angle's part of R. Half of the allowance of `beyond` without its pm may go there.
+        const bool thin = !(1.25e-6f * R * R * R <= 1e-5f * a2 * (R + fabsf(cc.x) + fabsf(cc.y) + fabsf(cc.z)));
+        t[4] = thin ? make_float4(c.z, 0.f, 0.f, 0.f) : make_float4(c.z, n.x, n.y, n.z);
         t[kTriAngles] = make_float4(angle_at(sub(b, a), sub(c, a), a2), angle_at(sub(a, b), sub(c, b), a2),
                                     angle_at(sub(a, c), sub(b, c), a2), 0.f);
+        reinterpret_cast<float4*>(P.tris)[kTriF4 * (size_t)P.nf + f] = make_float4(n.x, n.y, n.z, 0.f);
         entries += (unsigned long long)(r[1] - r[0] + 1) * (unsigned)(r[3] - r[2] + 1) * (unsigned)(r[5] - r[4] + 1);
         for (int bz = r[4]; bz <= r[5]; ++bz)
             for (int by = r[2]; by <= r[3]; ++by)
@@ -331,7 +337,14 @@ __device__ __forceinline__ float reach_of(float best, float pm) {
 __device__ __forceinline__ float3 rec_v0(const float4* rec) { return f3(rec[2].x, rec[2].y, rec[2].z); }
 __device__ __forceinline__ float3 rec_v1(const float4* rec) { return f3(rec[2].w, rec[3].x, rec[3].y); }
 __device__ __forceinline__ float3 rec_v2(const float4* rec) { return f3(rec[3].z, rec[3].w, rec[4].x); }
+// The record's normal (0 for some); the triangle's.
 __device__ __forceinline__ float3 rec_normal(const float4* rec) { return f3(rec[4].y, rec[4].z, rec[4].w); }
+__device__ __forceinline__ float3 tri_normal(const SdfParams& P, const float4* rec, uint32_t f) {
+    const float3 n = rec_normal(rec);
+    if (n.x != 0.f || n.y != 0.f || n.z != 0.f) return n;
+    const float4 u = reinterpret_cast<const float4*>(P.tris)[kTriF4 * (size_t)P.nf + f];
+    return f3(u.x, u.y, u.z);
+}
 
 // The closest point of a record's triangle to p (xyz) and its squared distance (w). One copy for
 // all callers: inlined, the band kernel no longer fits the instruction cache (14 of 28 stall
@@ -351,7 +364,7 @@ __device__ __forceinline__ float sqrt_below(float x) {
 
 // Whether the triangle's float distance from p provably exceeds what `reach` was made from:
 // by its bounding sphere, then by its plane distance h and the lateral distance beyond the
-// sphere (d^2 >= h^2 + (l - R)^2).
+// sphere (d^2 >= h^2 + (l - R)^2; a normal of 0 leaves the sphere's bound).
 __device__ __forceinline__ bool beyond(const float4* rec, float3 p, float pm, float reach) {
     const float4 ts = rec[0];
     const float dx = p.x - ts.x, dy = p.y - ts.y, dz = p.z - ts.z;
@@ -517,7 +530,7 @@ __device__ __noinline__ float band_serial(const SdfParams& P, BandShared& S, flo
                 if (mine && (reach == kFar || !beyond(rec, pt, pm, reach))) {
                     const float4 r = closest(pt, rec);
                     const float3 cp = f3(r.x, r.y, r.z);
-                    if (visit(q, r.w, tie_weight(P, S.idx[c], rec, cp, veps), rec_normal(rec))) {
+                    if (visit(q, r.w, tie_weight(P, S.idx[c], rec, cp, veps), tri_normal(P, rec, S.idx[c]))) {
                         q.bp = cp;
                         reach = reach_of(r.w, pm);
                     }
@@ -549,7 +562,7 @@ __device__ __noinline__ float band_walk(const SdfParams& P, BandShared& S, bool 
         const float4 r = closest(p, rec);
         const uint32_t f = tie_triangle(S, single, e), mask = slot_mask(rec[1], bx, by, bz);
         const float w = tie_weight(P, f, rec, f3(r.x, r.y, r.z), veps);
-        const float3 n = rec_normal(rec);
+        const float3 n = tri_normal(P, rec, f);
         slots |= mask;
         int to = t;
         while (to > 0 && tie_triangle(S, single, S.tie_e[warp][to - 1][lane]) > f) {
@@ -899,7 +912,7 @@ __global__ void __launch_bounds__(kBandThreads, kBandCtasPerSm) k_band(SdfParams
             const float4 r = closest(pt, tie_record(P, S, single, S.tie_e[warp][first][lane]));
             q.bp = f3(r.x, r.y, r.z);
             // all tie with the first, and all normals on one side by 1e-3 of the distance: every
-            // sum of them lies on that side
+            // sum of them lies on that side (a normal of 0 is on neither)
             const float3 v = sub(pt, q.bp);
             const float vv = dot(v, v), clear = vv > 1e-30f ? 1e-3f * sqrtf(vv) : kFar;
             bool above = true, below = true;
@@ -1285,7 +1298,7 @@ unsigned grid_for(long long items, int per_block, int num_sms, int per_sm) {
 
 }  // namespace
 
-size_t sdf_tri_record_bytes() { return sizeof(Tri); }
+size_t sdf_tri_record_bytes() { return sizeof(Tri) + sizeof(float4); }
 
 // Bound of the band kernel's work items: the bins' 27-bin entry counts sum to at most 27 * entries.
 long long sdf_items_capacity(long long nbins, unsigned long long entries) {
