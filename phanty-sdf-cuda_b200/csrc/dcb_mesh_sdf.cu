@@ -52,7 +52,9 @@ struct Tri {
     float a2;       // doubled area (0: skipped, as the reference skips area <= 1e-12)
     uint32_t r[3];  // bins it is listed in, per axis: first | last << 16 (kPackedBins axes and below)
     float v[9];     // vertices
-    float n[3];     // unit normal; 0 where it bounds no distance (a thin triangle's)
+    float n[3];     // unit normal; 0 where it bounds no distance (a thin triangle's) or its weight may
+                    // leave a sum of normals without a side (a corner angle of 0, an area whose
+                    // square overflows)
     float w[4];     // tie weights of its vertices: the angles there
 };
 constexpr int kTriF4 = 6;
@@ -171,13 +173,15 @@ __global__ void __launch_bounds__(256) k_tri_prep(SdfParams P) {
                            __uint_as_float((uint32_t)r[4] | (uint32_t)r[5] << 16));
         t[2] = make_float4(a.x, a.y, a.z, b.x);
         t[3] = make_float4(b.y, b.z, c.x, c.y);
+        const float3 w = f3(angle_at(sub(b, a), sub(c, a), a2), angle_at(sub(a, b), sub(c, b), a2),
+                            angle_at(sub(a, c), sub(b, c), a2));
         // The float normal is off by up to 3 sqrt(3) ulps (2^-24) of the longest edge's square over
         // the doubled area, the edge being two radii at most: the triangle leaves the plane by that
         // angle's part of R. Half of the allowance of `beyond` without its pm may go there.
         const bool thin = !(1.25e-6f * R * R * R <= 1e-5f * a2 * (R + fabsf(cc.x) + fabsf(cc.y) + fabsf(cc.z)));
-        t[4] = thin ? make_float4(c.z, 0.f, 0.f, 0.f) : make_float4(c.z, n.x, n.y, n.z);
-        t[kTriAngles] = make_float4(angle_at(sub(b, a), sub(c, a), a2), angle_at(sub(a, b), sub(c, b), a2),
-                                    angle_at(sub(a, c), sub(b, c), a2), 0.f);
+        const bool plain = !thin && w.x > 0.f && w.y > 0.f && w.z > 0.f && a2 < 1e18f;
+        t[4] = plain ? make_float4(c.z, n.x, n.y, n.z) : make_float4(c.z, 0.f, 0.f, 0.f);
+        t[kTriAngles] = make_float4(w.x, w.y, w.z, 0.f);
         reinterpret_cast<float4*>(P.tris)[kTriF4 * (size_t)P.nf + f] = make_float4(n.x, n.y, n.z, 0.f);
         entries += (unsigned long long)(r[1] - r[0] + 1) * (unsigned)(r[3] - r[2] + 1) * (unsigned)(r[5] - r[4] + 1);
         for (int bz = r[4]; bz <= r[5]; ++bz)
@@ -912,7 +916,7 @@ __global__ void __launch_bounds__(kBandThreads, kBandCtasPerSm) k_band(SdfParams
             const float4 r = closest(pt, tie_record(P, S, single, S.tie_e[warp][first][lane]));
             q.bp = f3(r.x, r.y, r.z);
             // all tie with the first, and all normals on one side by 1e-3 of the distance: every
-            // sum of them lies on that side (a normal of 0 is on neither)
+            // sum of them with positive weights lies on that side (a normal of 0 is on neither)
             const float3 v = sub(pt, q.bp);
             const float vv = dot(v, v), clear = vv > 1e-30f ? 1e-3f * sqrtf(vv) : kFar;
             bool above = true, below = true;
