@@ -179,7 +179,8 @@ __global__ void __launch_bounds__(256) k_tri_prep(SdfParams P) {
         // the doubled area, the edge being two radii at most: the triangle leaves the plane by that
         // angle's part of R. Half of the allowance of `beyond` without its pm may go there.
         const bool thin = !(1.25e-6f * R * R * R <= 1e-5f * a2 * (R + fabsf(cc.x) + fabsf(cc.y) + fabsf(cc.z)));
-        const bool plain = !thin && w.x > 0.f && w.y > 0.f && w.z > 0.f && a2 < 1e18f;
+        // (kBandTies areas, each added by up to 27 bins, have a square below FLT_MAX)
+        const bool plain = !thin && w.x > 0.f && w.y > 0.f && w.z > 0.f && a2 < 5e16f;
         t[4] = plain ? make_float4(c.z, n.x, n.y, n.z) : make_float4(c.z, 0.f, 0.f, 0.f);
         t[kTriAngles] = make_float4(w.x, w.y, w.z, 0.f);
         reinterpret_cast<float4*>(P.tris)[kTriF4 * (size_t)P.nf + f] = make_float4(n.x, n.y, n.z, 0.f);
