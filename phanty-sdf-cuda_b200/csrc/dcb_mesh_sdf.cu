@@ -733,7 +733,8 @@ __global__ void __launch_bounds__(kBandThreads, kBandCtasPerSm) k_band(SdfParams
         if (packed) {
             // Only triangles whose float distances are good are asked: not slivers (a2 is 2.6 R^2
             // for an equilateral one) nor tiny ones (barycentrics lose (distance / side)^2 ulps);
-            // two radii of slack.
+            // two radii of slack. Nor beyond 1e9, where the barycentrics' products overflow (a side's
+            // and a distance's square: such distances come out too long).
             const float3 mid = f3(0.5f * (blo.x + bhi.x), 0.5f * (blo.y + bhi.y), 0.5f * (blo.z + bhi.z));
             const float small = 0.004f * reach_bin;
             float near = kFar;
@@ -751,10 +752,11 @@ __global__ void __launch_bounds__(kBandThreads, kBandCtasPerSm) k_band(SdfParams
             if (lane == 0) atomicMin(&S.reach, __float_as_uint(near));     // non-negative floats order as integers
             __syncthreads();
             near = __uint_as_float(S.reach);
-            if (near < 1e18f) {
+            if (near < 1e9f) {
                 const float3 hd = sub(bhi, mid);
                 const float ub = (near + sqrtf(dot(hd, hd))) * 1.0001f + 1e-5f * bpm;
-                reach_bin = fminf(reach_bin, reach_of(ub * ub * 1.001f + 2.f * kWindow * tie_tol(ub * ub), bpm));
+                const float bound = reach_of(ub * ub * 1.001f + 2.f * kWindow * tie_tol(ub * ub), bpm);
+                if (ub < 1e9f) reach_bin = fminf(reach_bin, bound);
             }
             stop = band_fill(P, S, 0, bx, by, bz, blo, bhi, reach_bin);
             single = stop >= L;
